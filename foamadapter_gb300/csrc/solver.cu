@@ -2400,6 +2400,8 @@ __global__ void __launch_bounds__(kPT, 1)
     }
 }
 
+#include "resident.cuh"
+
 // ---------------------------------------------------------------- graph glue
 cudaError_t add_kernel_deps(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraphNode_t* deps, size_t ndeps,
                             void* func, unsigned grid, unsigned block, void** args) {
@@ -2459,6 +2461,9 @@ struct SolverCache {
     cudaGraphExec_t gbg = nullptr;
     fvgb_solver_stats* h_stats = nullptr;  // pinned [ncases]
     GridBar* bar = nullptr;
+    ResMail* mail = nullptr;               // resident solves: partials and answers in flight
+    LLWord* zll = nullptr;                 // resident solves: published preconditioned residuals [n]
+    int res_fit = -1;                      // resident solves: every block's part fits on its SM (-1: not asked yet)
     float *pf2 = nullptr, *zf = nullptr;   // second direction buffer and z of the persistent mixed solve
     double* r0 = nullptr;                   // mixed: first FP64 residual, from the preparation kernel
     uint64_t converted_version = 0;        // fvgb_ls::version the FP32 matrix copy was formed from
@@ -3113,6 +3118,52 @@ int persistent_grid(SolverCache* c, bool mixed) {
     return g;
 }
 
+// Blocks of a resident solve that fit on the GPU at once (one per SM), 0: none.
+int resident_blocks() {
+    static thread_local int dev_of = -1, blocks = 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev != dev_of) {
+        int sms = 0, coop = 0, per_sm = 1;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+        for (const void* fn : {(const void*)k_pcg_resident<4>, (const void*)k_pcg_resident<8>}) {
+            int b = 0;
+            if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kT, kResSmem) != cudaSuccess)
+                b = 0;
+            per_sm = std::min(per_sm, b);
+        }
+        cudaGetLastError();
+        blocks = coop && per_sm > 0 ? std::min(sms, kResMaxBlocks) : 0;
+        dev_of = dev;
+    }
+    return blocks;
+}
+
+// Whether this system can be solved resident: at most one block per SM and every
+// block's matrix rows in its shared memory.  Asked once per system (one small
+// kernel and a read of its result); allocates what the solve keeps.
+bool resident_fits(SolverCache* c, cudaStream_t s) {
+    if (c->res_fit >= 0) return c->res_fit == 1;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    c->res_fit = 0;
+    if (c->nb > resident_blocks()) return false;
+    unsigned int need = ~0u, *d = nullptr;
+    if (calloc_dev(c, &d, 1) != cudaSuccess || settle_creation() != cudaSuccess) return false;
+    const MeshView m = c->ls->mesh->v;
+    if (rows_per_thread(c->n) == 8) k_res_need<8><<<c->nb, kT>>>(m, d);
+    else k_res_need<4><<<c->nb, kT>>>(m, d);
+    if (cudaMemcpy(&need, d, sizeof(need), cudaMemcpyDeviceToHost) != cudaSuccess || need > (unsigned)kResSmem)
+        return false;
+    if (calloc_dev(c, &c->mail, 1) != cudaSuccess || calloc_dev(c, &c->zll, (size_t)c->n) != cudaSuccess ||
+        settle_creation() != cudaSuccess)
+        return false;
+    c->res_fit = 1;
+    return true;
+}
+
 bool use_persistent(SolverCache* c, const fvgb_solver_cfg* cfg) {
     if (!c->whole || cfg->kernel_mode == 1 || cfg->kernel_mode == 3) return false;
     if (cfg->kernel_mode != 2 && c->n > (1 << 20)) return false;
@@ -3217,7 +3268,13 @@ fvgb_status launch(SolverCache* c, double* x, const fvgb_solver_cfg* cfg, fvgb_s
         const int pg = persistent_grid(c, mixed);
         const int grid = nvb < pg ? nvb : pg;
         FVGB_CUDA_TRY(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), s));
-        if (mixed) {
+        if (!mixed && resident_fits(c, s)) {
+            FVGB_CUDA_TRY(cudaMemsetAsync(c->mail, 0, sizeof(ResMail), s));
+            FVGB_CUDA_TRY(cudaMemsetAsync(c->zll, 0, sizeof(LLWord) * (size_t)c->n, s));
+            void* args[] = {&L, &m, &val, &b, &c->zll, &c->mail, &c->bar};
+            const void* fn = rows_per_thread(c->n) == 8 ? (const void*)k_pcg_resident<8> : (const void*)k_pcg_resident<4>;
+            FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, kResSmem, s));
+        } else if (mixed) {
             // k_ir_persistent(L, m, val, b, a32, ev, dinv, r0, rh, y, pbuf0, pbuf1, z, q, pa, pb, pc, gb, nvb)
             void* args[] = {&L,     &m,    &val,   &b,     &c->ah, &c->ev, &c->dinvf, &c->r0, &c->rh, &c->y,
                             &c->pf, &c->pf2, &c->zf, &c->qf, &c->pa, &c->pb, &c->pc,   &c->bar, &nvb};

@@ -1,0 +1,114 @@
+"""The resident single-case solves (one block per SM, kernel_mode 2) against the
+graph of kernels, bit for bit: iterates, counts and residual norms.
+
+Sizes at the edges of the kernel's layout: one row, a partial slice, one block
+more and less, the switch of rows per thread (2^15), the largest system with
+one block per SM and the first one beyond it (which takes the grid-barrier
+kernel).  Numberings: the box's own, and a random one in which almost every
+matrix slot reaches into another block (it fits the shared memory with 4 rows
+per thread and does not with 8).
+"""
+import numpy as np
+import pytest
+import torch
+
+from foamadapter_gb300 import abi, mesh, neon
+from foamadapter_gb300.mesh import DeviceMesh
+
+pytestmark = pytest.mark.gpu
+
+
+def renumber(hm, seed):
+    """The same mesh under a random cell numbering, faces back in upper-triangular order."""
+    perm = np.random.default_rng(seed).permutation(hm.n).astype(np.int32)
+    inv = np.argsort(perm)
+    o, n = perm[hm.own], perm[hm.nei]
+    flip = o > n
+    own, nei = np.where(flip, n, o).astype(np.int32), np.where(flip, o, n).astype(np.int32)
+    order = np.lexsort((nei, own))
+    hm.own, hm.nei = np.ascontiguousarray(own[order]), np.ascontiguousarray(nei[order])
+    hm.Sf = np.ascontiguousarray(np.where(flip[:, None], -hm.Sf, hm.Sf)[order])
+    hm.w = np.ascontiguousarray(np.where(flip, 1.0 - hm.w, hm.w)[order])
+    for k in ("Cf", "magSf", "delta"):
+        setattr(hm, k, np.ascontiguousarray(getattr(hm, k)[order]))
+    hm.V, hm.C = np.ascontiguousarray(hm.V[inv]), np.ascontiguousarray(hm.C[inv])
+    hm.bcells = np.ascontiguousarray(perm[hm.bcells])
+    return hm
+
+
+def system(dims, shuffled=False, two_d=False, dt=0.05):
+    hm = mesh.box(*dims, 1.0, 1.0, 1.0 / max(dims) if two_d else 1.0, jitter=0.1, seed=7, two_d=two_d)
+    if shuffled:
+        hm = renumber(hm, 3)
+    rng = np.random.default_rng(11)
+    dm = DeviceMesh(hm)
+    T = neon.VolumeField(dm, 300.0 + rng.standard_normal(hm.n),
+                         [("fixedValue", 400.0)] + [("zeroGradient", 0.0)] * (hm.npatch - 1))
+    g = neon.SurfaceField(dm, np.exp(0.5 * rng.standard_normal(hm.nif + hm.nbf)))
+    ls = neon.LinearSystem(dm)
+    ls.assemble([neon.ddt(T.internal.clone()), neon.laplacian(g, -1.0)], dt, T)
+    return hm, T, ls
+
+
+DIMS = [
+    ((1, 1, 1), False, False), ((7, 3, 1), False, False), ((11, 31, 3), False, False), ((32, 32, 1), False, True),
+    ((25, 41, 1), False, True), ((19, 23, 29), False, False), ((17, 17, 17), True, False),
+    ((47, 41, 17), False, False), ((32, 32, 32), False, False), ((36, 34, 31), True, False),
+    ((128, 128, 19), False, False), ((512, 608, 1), False, True), ((129, 128, 19), False, False),
+]
+
+
+@pytest.mark.parametrize("dims,shuffled,two_d", DIMS)
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED_IR])
+def test_resident_equals_graph(cuda, dims, shuffled, two_d, precision):
+    hm, T, ls = system(dims, shuffled, two_d)
+    kw = dict(rel_tol=1e-9, max_iter=400, precision=precision, inner_rel_tol=0.1)
+    out = []
+    for mode in (1, 2, 2):
+        x = T.internal.clone()
+        st = ls.solve(x, kernel_mode=mode, **kw)
+        out.append((x.cpu().numpy(), st.num_iter, st.num_outer, st.init_res_norm, st.final_res_norm, st.status))
+    for o in out[1:]:
+        assert o[1:] == out[0][1:]
+        np.testing.assert_array_equal(o[0], out[0][0])
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED_IR])
+def test_resident_stopping(cuda, precision):
+    """Iteration caps 0 and 3, an absolute tolerance met at the start, the ||b|| baseline
+    and a zero residual stop the resident solve where they stop the graph."""
+    hm, T, ls = system((19, 23, 29))
+    solved = T.internal.clone()
+    ls.solve(solved, rel_tol=1e-12, max_iter=2000)
+    for kw in (dict(rel_tol=1e-9, max_iter=0), dict(rel_tol=1e-9, max_iter=3), dict(rel_tol=0.0, abs_tol=1e30),
+               dict(rel_tol=1e-6, flags=abi.SOLVE_RHS_BASELINE), dict(rel_tol=1e-30, max_iter=60)):
+        for start in (T.internal, solved):
+            out = []
+            for mode in (1, 2):
+                x = start.clone()
+                st = ls.solve(x, kernel_mode=mode, precision=precision, max_outer=6, **kw)
+                out.append((x.cpu().numpy(), st.num_iter, st.num_outer, st.init_res_norm, st.final_res_norm,
+                            st.status))
+            assert out[0][1:] == out[1][1:], kw
+            np.testing.assert_array_equal(out[0][0], out[1][0])
+
+
+def test_resident_solves_on_two_streams(cuda):
+    """Two systems solved asynchronously on two streams give their own bits."""
+    systems = [system((19, 23, 29)), system((47, 41, 17))]
+    cfg = abi.SolverCfg(1e-9, 0.0, 400, abi.PREC_FP64, 0.1, 1000, 50, 2)
+    want = []
+    for _, T, ls in systems:
+        x = T.internal.clone()
+        ls.solve(x, rel_tol=1e-9, max_iter=400, kernel_mode=1)
+        want.append(x.cpu().numpy())
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        xs = [T.internal.clone() for _, T, _ in systems]
+        torch.cuda.synchronize()
+        for (_, _, ls), x, s in zip(systems, xs, streams):
+            abi.check(abi.lib().fvgb_solve_async(ls.handle, abi.ptr(x), cfg, None, s.cuda_stream))
+        torch.cuda.synchronize()
+        for x, w in zip(xs, want):
+            np.testing.assert_array_equal(x.cpu().numpy(), w)
