@@ -28,13 +28,16 @@
 #pragma once
 
 constexpr int kResMaxBlocks = 160;       // 5 partials per polling lane
-constexpr int kResSmem = 220 * 1024;     // dynamic shared memory of a resident block
+// Most dynamic shared memory of a resident block.  A launch asks only for what its
+// largest block needs: what is left stays L1, and a poll of 128 lines through an L1
+// of a few KB takes 2,700 clocks instead of 1,400.
+constexpr int kResSmem = 220 * 1024;
 
 struct alignas(16) LLWord {  // one published value
     unsigned long long w0, w1;  // epoch << 32 | low half, epoch << 32 | high half
 };
 struct alignas(128) LLLine {
-    LLWord w;
+    LLWord w;  // an FP64 partial; an FP32 one takes w.w0 alone
 };
 struct ResMail {
     LLLine part[2][3][kResMaxBlocks];  // [epoch parity][dot product][block]
@@ -55,6 +58,19 @@ __device__ __forceinline__ bool ll_load(const LLWord* p, unsigned epoch, double*
     return (unsigned)(a >> 32) == epoch && (unsigned)(b >> 32) == epoch;
 }
 
+// a float travels as one word
+__device__ __forceinline__ void ll_store(unsigned long long* p, float v, unsigned epoch) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p),
+                 "l"(((unsigned long long)epoch << 32) | __float_as_uint(v))
+                 : "memory");
+}
+__device__ __forceinline__ bool ll_load(const unsigned long long* p, unsigned epoch, float* v) {
+    unsigned long long a;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
+    *v = __uint_as_float((unsigned)a);
+    return (unsigned)(a >> 32) == epoch;
+}
+
 // Bound of every wait: true when it has run out, here or in another block.
 __device__ __forceinline__ bool res_give_up(GridBar* gb, unsigned spins) {
     if ((spins & 63u) != 63u) return false;
@@ -72,9 +88,13 @@ __device__ __forceinline__ double plus_zero(double v) {
     return __longlong_as_double((u << 1) == 0 ? 0ll : (long long)u);
 }
 
+__device__ __forceinline__ bool ll_get(const LLLine* p, unsigned epoch, double* v) { return ll_load(&p->w, epoch, v); }
+__device__ __forceinline__ bool ll_get(const LLLine* p, unsigned epoch, float* v) { return ll_load(&p->w.w0, epoch, v); }
+
 // One warp: the final tree over every block's partial, in all lanes.
 // With at most 256 blocks a tree thread holds one partial, so lane l adds
 // partials l, l+32, ... and the butterfly finishes, exactly final_tree.
+template <class V = double>
 __device__ __forceinline__ bool res_collect(GridBar* gb, const LLLine* part, unsigned epoch, int nblk, double* out) {
     constexpr int NS = kResMaxBlocks / 32;
     const int lane = threadIdx.x & 31;
@@ -85,13 +105,14 @@ __device__ __forceinline__ bool res_collect(GridBar* gb, const LLLine* part, uns
         v[s] = 0.0;
         have[s] = lane + 32 * s >= nblk;
     }
+#pragma unroll 1
     for (unsigned spins = 0;; ++spins) {
         bool all = true;
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-            double t;
-            if (!have[s] && ll_load(&part[lane + 32 * s].w, epoch, &t)) {
-                v[s] = plus_zero(t);
+            V t;
+            if (!have[s] && ll_get(&part[lane + 32 * s], epoch, &t)) {
+                v[s] = plus_zero((double)t);
                 have[s] = true;
             }
             all = all && have[s];
@@ -113,9 +134,10 @@ __device__ __forceinline__ bool res_collect(GridBar* gb, const LLLine* part, uns
 }
 
 // One warp: the block's partial from its 256 thread partials (block_tree)
-__device__ __forceinline__ double res_block_tree(const double* sm) {
+template <class V>
+__device__ __forceinline__ V res_block_tree(const V* sm) {
     const int lane = threadIdx.x & 31;
-    double s = sm[lane];
+    V s = sm[lane];
 #pragma unroll
     for (int k = 1; k < kT / 32; ++k) s = s + sm[lane + 32 * k];
 #pragma unroll
@@ -123,18 +145,23 @@ __device__ __forceinline__ double res_block_tree(const double* sm) {
     return s;
 }
 
-// The block's part of the system in shared memory.
+// The block's part of the system in shared memory (V: double, or float for the
+// FP32 inner solve).
+template <class V>
 struct ResMatrix {
-    double* sp;            // [rows + nh] own directions, then the halo's
-    double* sval;          // [len]
-    double* zh;            // [nh] the halo's z, fetched while a reduction is under way (null: no room)
+    V* sp;                 // [rows + nh] own directions, then the halo's
+    V* sval;               // [len]
+    V* zh;                 // [nh] the halo's z, fetched while a reduction is under way (null: no room)
     int* hcol;             // [nh] column of every halo entry
     unsigned short* scol;  // [len] index into sp
     int nh, pos0;
 };
 
-__host__ __device__ inline size_t res_bytes(int rows, int len, int nh, bool zh) {
-    return 8 * (size_t)(rows + nh) + 8 * (size_t)len + (zh ? 8 * (size_t)nh : 0) + 4 * (size_t)nh + 2 * (size_t)len;
+// bytes of that part: value size v, with or without the staged z (with FP32 values
+// it starts with one FP64 residual per row)
+__host__ __device__ inline size_t res_bytes(int v, int rows, int len, int nh, bool zh) {
+    return (v == 4 ? 8 * (size_t)rows : 0) + (size_t)v * ((size_t)rows + nh + len + (zh ? nh : 0)) + 4 * (size_t)nh +
+           2 * (size_t)len;
 }
 
 // Slots and halo entries of block row0's rows (all threads; counter: shared).
@@ -146,9 +173,11 @@ __device__ __forceinline__ void res_count(const MeshView& m, int row0, int* coun
     *len = __ldg(&m.m_ptr[s1]) - __ldg(&m.m_ptr[s0]);
     if (threadIdx.x == 0) *counter = 0;
     __syncthreads();
+#pragma unroll 1
     for (int s = s0 + wid; s < s1; s += kT / 32) {
         const int b0 = __ldg(&m.m_ptr[s]), w = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5, i = s * 32 + lane;
         int c = 0;
+#pragma unroll 1
         for (int k = 0; k < w; ++k)
             c += (unsigned)(slot_col(m, b0 + k * 32 + lane, i) - row0) >= (unsigned)ROWS;
         c = __reduce_add_sync(0xffffffffu, c);
@@ -159,38 +188,44 @@ __device__ __forceinline__ void res_count(const MeshView& m, int row0, int* coun
     __syncthreads();
 }
 
-// Whether every block's part fits in shared memory: the largest need, in bytes.
+// The largest block's need in bytes: need[0] with FP64 values, need[1] with FP32,
+// need[2] and need[3] the same with the halo's z staged.
 template <int R>
 __global__ void __launch_bounds__(kT) k_res_need(MeshView m, unsigned int* need) {
     __shared__ int counter;
     int len, nh;
     res_count<R>(m, (int)blockIdx.x * (kT * R), &counter, &len, &nh);
-    if (threadIdx.x == 0) {
-        const size_t b = kT * R + nh > 65536 ? ~(size_t)0 : res_bytes(kT * R, len, nh, false);
-        atomicMax(need, b > 0xffffffffull ? 0xffffffffu : (unsigned)b);
+    if (threadIdx.x < 4) {
+        const size_t b = kT * R + nh > 65536 ? ~(size_t)0
+                                             : res_bytes(threadIdx.x & 1 ? 4 : 8, kT * R, len, nh, threadIdx.x >= 2);
+        atomicMax(&need[threadIdx.x], b > 0xffffffffull ? 0xffffffffu : (unsigned)b);
     }
 }
 
-template <int R>
-__device__ __forceinline__ ResMatrix res_load(const MeshView& m, const double* __restrict__ val, unsigned char* dyn,
-                                              int row0, int* counter) {
+// Lays the block's part out and fills the columns; the values are the caller's.
+template <int R, class V>
+__device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned char* dyn, int row0, int* counter) {
     constexpr int ROWS = kT * R;
     const int T = threadIdx.x, lane = T & 31, wid = T >> 5;
     const int s0 = row0 >> 5, s1 = min((m.n + 31) >> 5, s0 + ROWS / 32);
-    ResMatrix M;
+    ResMatrix<V> M;
     int len;
     res_count<R>(m, row0, counter, &len, &M.nh);
     M.pos0 = __ldg(&m.m_ptr[s0]);
-    const bool zh = res_bytes(ROWS, len, M.nh, true) <= (size_t)kResSmem;
-    M.sp = (double*)dyn;
+    unsigned int have;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(have));
+    const bool zh = res_bytes((int)sizeof(V), ROWS, len, M.nh, true) <= (size_t)have;
+    M.sp = (V*)(dyn + (sizeof(V) == 4 ? 8 * ROWS : 0));
     M.sval = M.sp + ROWS + M.nh;
     M.zh = zh ? M.sval + len : nullptr;
     M.hcol = (int*)(M.sval + len + (zh ? M.nh : 0));
     M.scol = (unsigned short*)(M.hcol + M.nh);
     if (T == 0) *counter = 0;
     __syncthreads();
+#pragma unroll 1
     for (int s = s0 + wid; s < s1; s += kT / 32) {
         const int b0 = __ldg(&m.m_ptr[s]), w = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5, i = s * 32 + lane;
+#pragma unroll 1
         for (int k = 0; k < w; ++k) {
             const int pos = b0 + k * 32 + lane;
             const int c = slot_col(m, pos, i), d = c - row0;
@@ -209,23 +244,24 @@ __device__ __forceinline__ ResMatrix res_load(const MeshView& m, const double* _
                 idx = ROWS + h;
             }
             M.scol[pos - M.pos0] = (unsigned short)idx;
-            M.sval[pos - M.pos0] = __ldg(&val[pos]);
         }
     }
     __syncthreads();
     return M;
 }
 
-// The halo's z of `epoch` into dst, by threads T0 <= T < kT; four loads in flight each.
-__device__ __forceinline__ bool res_halo(GridBar* gb, const ResMatrix& M, const LLWord* z, unsigned epoch, int T0,
-                                         double* dst) {
+// The halo's z of `epoch` into M.zh, by threads T0 <= T < kT; four loads in flight each.
+template <class V, class W>
+__device__ __forceinline__ bool res_halo(GridBar* gb, const ResMatrix<V>& M, const W* z, unsigned epoch, int T0) {
+#pragma unroll 1
     for (int h0 = (int)threadIdx.x - T0; h0 < M.nh; h0 += 4 * (kT - T0)) {
         bool have[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) have[u] = h0 + u * (kT - T0) >= M.nh;
+#pragma unroll 1
         for (unsigned spins = 0;; ++spins) {
             bool all = true;
-            double v[4];
+            V v[4];
             bool ok[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -235,7 +271,7 @@ __device__ __forceinline__ bool res_halo(GridBar* gb, const ResMatrix& M, const 
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 if (ok[u]) {
-                    dst[h0 + u * (kT - T0)] = v[u];
+                    M.zh[h0 + u * (kT - T0)] = v[u];
                     have[u] = true;
                 }
                 all = all && have[u];
@@ -246,6 +282,86 @@ __device__ __forceinline__ bool res_halo(GridBar* gb, const ResMatrix& M, const 
     }
     return true;
 }
+
+__device__ __forceinline__ double res_fma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float res_fma(float a, float b, float c) { return fmaf(a, b, c); }
+
+// The halo's new direction, z (restart) or z + beta p, in M.sp (all threads).
+template <class V, class W>
+__device__ __forceinline__ bool res_halo_dir(GridBar* gb, const ResMatrix<V>& M, const W* z, unsigned epoch,
+                                             bool restart, V beta) {
+    bool good = true;
+    const int nown = (int)(M.sval - M.sp) - M.nh;
+#pragma unroll 1
+    for (int h = threadIdx.x; h < M.nh; h += kT) {
+        V v;
+        if (M.zh) {
+            v = M.zh[h];
+        } else {  // no room to stage it
+            unsigned spins = 0;
+#pragma unroll 1
+            while (!ll_load(z + M.hcol[h], epoch, &v))
+                if (res_give_up(gb, spins++)) {
+                    good = false;
+                    break;
+                }
+        }
+        V* p = M.sp + nown + h;
+        *p = restart ? v : res_fma(beta, *p, v);
+    }
+    return good;
+}
+
+// The matrix rows of one thread: slot bases (in the block's arrays) and widths of
+// its R slices, one per j.
+template <int R>
+struct ResRows {
+    int base[R], w[R], kmin, kmax;
+    __device__ __forceinline__ ResRows(const MeshView& m, int first_row, int pos0) {
+        kmin = INT_MAX;
+        kmax = 0;
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int s = (first_row >> 5) + j;
+            base[j] = w[j] = 0;
+            if (s * 32 < m.n) {
+                const int b0 = __ldg(&m.m_ptr[s]);
+                base[j] = b0 - pos0 + (threadIdx.x & 31);
+                w[j] = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5;
+            }
+            kmin = min(kmin, w[j]);
+            kmax = max(kmax, w[j]);
+        }
+    }
+    // q[j] = sum over the row's slots of value * f(own[j], x[column]): fma chains from
+    // +0 in slot order, the R rows interleaved.  A branch per row would serialise the
+    // dependent shared-memory loads, so the slots all R rows have go without one.
+    template <class V, class F>
+    __device__ __forceinline__ void product(const ResMatrix<V>& M, V* q, F f, const V* own) const {
+#pragma unroll
+        for (int j = 0; j < R; ++j) q[j] = (V)0;
+#pragma unroll 1
+        for (int k = 0; k < kmin; ++k) {
+            int c[R];
+            V a[R], x[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j) c[j] = M.scol[base[j] + 32 * k];
+#pragma unroll
+            for (int j = 0; j < R; ++j) a[j] = M.sval[base[j] + 32 * k];
+#pragma unroll
+            for (int j = 0; j < R; ++j) x[j] = M.sp[c[j]];
+#pragma unroll
+            for (int j = 0; j < R; ++j) q[j] = res_fma(a[j], f(own[j], x[j]), q[j]);
+        }
+#pragma unroll 1
+        for (int k = kmin; k < kmax; ++k) {
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+                if (k < w[j])
+                    q[j] = res_fma(M.sval[base[j] + 32 * k], f(own[j], M.sp[M.scol[base[j] + 32 * k]]), q[j]);
+        }
+    }
+};
 
 struct ResShared {
     double value, res0, res;
@@ -272,26 +388,40 @@ __global__ void __launch_bounds__(kT, 1)
     const SolverParams prm = L.bs->prm;
     double* x = prm.x;
     if (T == 0) sh.bad = 0;
-    const ResMatrix M = res_load<R>(m, val, dyn, row0, &sh.counter);
+    const ResMatrix<double> M = res_load<R, double>(m, dyn, row0, &sh.counter);
+    // cold code in rolled loops: the kernel's iteration has to stay in the
+    // instruction cache (unrolled over the rows it was 97 KB)
+#pragma unroll 1
+    for (int j = 0; j < R; ++j) {
+        const int l = loc0 + 32 * j, i = row0 + l;
+        M.sp[l] = i < n ? __ldg(&b[i]) - spmv_row_cg(m, val, x, i) : 0.0;
+    }
     double xr[R], rv[R], pr[R], di[R], zr[R];
-    int base[R], w[R];
-    int wmax = 0;
+    ResRows<R> W(m, row0 + wid * (32 * R), M.pos0);
+#pragma unroll 1
+    for (int k = 0; k < W.kmax; ++k) {
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            if (k < W.w[j]) M.sval[W.base[j] + 32 * k] = __ldg(&val[M.pos0 + W.base[j] + 32 * k]);
+    }
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-        const int i = row0 + loc0 + 32 * j, s = (row0 >> 5) + wid * R + j;
-        base[j] = w[j] = 0;
-        if (s * 32 < n) {
-            const int b0 = __ldg(&m.m_ptr[s]);
-            base[j] = b0 - M.pos0 + lane;
-            w[j] = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5;
-        }
-        wmax = max(wmax, w[j]);
-        xr[j] = rv[j] = pr[j] = di[j] = 0.0;
+        rv[j] = M.sp[loc0 + 32 * j];
+        xr[j] = pr[j] = di[j] = 0.0;
+        const int i = row0 + loc0 + 32 * j;
         if (i < n) {
             xr[j] = x[i];
-            di[j] = 1.0 / __ldg(&val[__ldg(&m.diag_pos[i])]);
-            rv[j] = __ldg(&b[i]) - spmv_row_cg(m, val, x, i);
+            di[j] = __ldg(&val[__ldg(&m.diag_pos[i])]);
         }
+    }
+#pragma unroll 1
+    for (int j = 0; j < R; ++j) {  // 1 / diagonal, one division's code
+        double d = 1.0;
+#pragma unroll
+        for (int u = 0; u < R; ++u) d = u == j ? di[u] : d;
+        d = 1.0 / d;
+#pragma unroll
+        for (int u = 0; u < R; ++u) di[u] = u == j && row0 + loc0 + 32 * u < n ? d : di[u];
     }
     unsigned epoch = 0;
     double rz = 0.0, tol = 0.0, res0 = 0.0, res = 0.0;  // warp 0: rz; warp 1: the others
@@ -370,27 +500,13 @@ __global__ void __launch_bounds__(kT, 1)
             }
             if (!good && lane == 0) sh.bad = 1;
         } else if (M.zh) {
-            if (!res_halo(gb, M, z, epoch, 64, M.zh)) sh.bad = 1;
+            if (!res_halo(gb, M, z, epoch, 64)) sh.bad = 1;
         }
         __syncthreads();
         if (sh.code || sh.bad) break;
         // p = z + beta p: the halo's copies, then the own rows
         const double beta = sh.value;
-        if (!M.zh) {  // no room to stage it
-            for (int h = T; h < M.nh; h += kT) {
-                double v;
-                unsigned spins = 0;
-                while (!ll_load(z + M.hcol[h], epoch, &v))
-                    if (res_give_up(gb, spins++)) {
-                        sh.bad = 1;
-                        break;
-                    }
-                M.sp[ROWS + h] = first ? v : fma(beta, M.sp[ROWS + h], v);
-            }
-        } else {
-            for (int h = T; h < M.nh; h += kT)
-                M.sp[ROWS + h] = first ? M.zh[h] : fma(beta, M.sp[ROWS + h], M.zh[h]);
-        }
+        if (!res_halo_dir(gb, M, z, epoch, first, beta)) sh.bad = 1;
 #pragma unroll
         for (int j = 0; j < R; ++j) {
             pr[j] = first ? zr[j] : fma(beta, pr[j], zr[j]);
@@ -399,13 +515,7 @@ __global__ void __launch_bounds__(kT, 1)
         __syncthreads();
         // q = A p: fma chains in slot order, R rows interleaved; p.q
         double q[R];
-#pragma unroll
-        for (int j = 0; j < R; ++j) q[j] = 0.0;
-        for (int k = 0; k < wmax; ++k) {
-#pragma unroll
-            for (int j = 0; j < R; ++j)
-                if (k < w[j]) q[j] = fma(M.sval[base[j] + 32 * k], M.sp[M.scol[base[j] + 32 * k]], q[j]);
-        }
+        W.product(M, q, [](double, double xk) { return xk; }, pr);
         double apq = 0.0;
 #pragma unroll
         for (int j = 0; j < R; ++j)
@@ -444,5 +554,350 @@ __global__ void __launch_bounds__(kT, 1)
         cs->res = res;
         cs->iter = iter;
         cs->status = sh.bad ? FVGB_ERR_CUDA : (sh.code == 2 ? FVGB_ERR_BREAKDOWN : status);
+    }
+}
+
+struct IrResShared {
+    double v[3];       // collected sums of a residual
+    double nsig, isig;
+    float fa, fbeta;
+    int restart, done, inner, brk, bad, counter;
+    unsigned int flags;
+};
+
+// Mixed-precision solve of one case on its blocks: the algorithm, arithmetic and
+// decisions of k_ir_persistent with the layout of k_pcg_resident.  The FP32 matrix
+// copy, the vectors of the inner CG and x are resident; a refinement step writes x
+// for the other blocks behind a fence and reads the FP64 matrix through L2.  An
+// inner iteration is two hops (2 x 1.4 us with 128 blocks on both dies), two final
+// trees and divisions in FP64 (2 x 0.7 us) and 1.5 us of FP32 work on shared
+// memory.  512 x 512 cavity step: 128 -> 71 ms against k_ir_persistent.
+template <int R>
+__global__ void __launch_bounds__(kT, 1)
+    k_ir_resident(Layout L, MeshView m, const double* __restrict__ val, const double* __restrict__ b, float* a32,
+                  float* ev, float* dinv, unsigned long long* z, ResMail* mail, GridBar* gb) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ double sma[kT], smb[kT];
+    __shared__ float smf[kT];
+    __shared__ IrResShared sh;
+    constexpr int ROWS = kT * R;
+    const int n = m.n, T = threadIdx.x, lane = T & 31, wid = T >> 5, nblk = (int)gridDim.x, blk = (int)blockIdx.x;
+    const int row0 = blk * ROWS;
+    const int loc0 = wid * (32 * R) + lane;  // this thread's rows: loc0 + 32 j
+    const SolverParams prm = L.bs->prm;
+    double* x = prm.x;
+    if (T == 0) {
+        sh.bad = 0;
+        sh.flags = 0u;
+    }
+    double* stage = (double*)dyn;  // [rows] FP64 residuals
+    const ResMatrix<float> M = res_load<R, float>(m, dyn, row0, &sh.counter);
+    // prepare: dinv, a32, ev (formed, or those of the unchanged matrix), sign flags, |D^-1/2 (b - A x0)|
+    unsigned int f = 0u;
+    double asr = 0.0;
+    ResRows<R> W(m, row0 + wid * (32 * R), M.pos0);
+#pragma unroll 1
+    for (int j = 0; j < R; ++j) {
+        const int i = row0 + loc0 + 32 * j, s = i >> 5;
+        if (s * 32 >= n) continue;
+        const int b0 = __ldg(&m.m_ptr[s]), wj = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5;
+        float* sv = M.sval + (b0 - M.pos0);
+        if (i >= n) {
+#pragma unroll 1
+            for (int k = 0; k < wj; ++k) sv[lane + 32 * k] = 0.0f;
+            continue;
+        }
+        const double d = __ldg(&val[__ldg(&m.diag_pos[i])]);
+        f |= d > 0.0 ? 1u : (d < 0.0 ? 2u : 4u);
+        float dj;
+        if (prm.convert) {
+            dj = (float)(1.0 / d);
+            dinv[i] = dj;
+            const double sg = d < 0.0 ? -1.0 : 1.0;
+            double e = 0.0;
+#pragma unroll 1
+            for (int k = 0; k < wj; ++k) {
+                const int pos = b0 + lane + 32 * k;
+                const int code = __ldg(&m.m_code[pos]);
+                float a = 0.0f;
+                if (code != FVGB_PAD) {
+                    const double av = __ldg(&val[pos]);
+                    e = e + av;
+                    if (code != -1) a = (float)(sg * av);
+                }
+                a32[pos] = a;
+                sv[lane + 32 * k] = a;
+            }
+            ev[i] = (float)(sg * e);
+        } else {
+            dj = dinv[i];
+#pragma unroll 1
+            for (int k = 0; k < wj; ++k) sv[lane + 32 * k] = a32[b0 + lane + 32 * k];
+        }
+        const double r = __ldg(&b[i]) - spmv_row_cg(m, val, x, i);
+        stage[loc0 + 32 * j] = r;
+        asr = fma(r * (double)fabsf(dj), r, asr);
+    }
+    double xr[R];
+    float yv[R], rh[R], pr[R], zr[R], di[R], ei[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        const int i = row0 + loc0 + 32 * j;
+        xr[j] = i < n ? x[i] : 0.0;
+        di[j] = i < n ? dinv[i] : 0.0f;
+        ei[j] = i < n ? ev[i] : 0.0f;
+        yv[j] = rh[j] = pr[j] = zr[j] = 0.0f;
+    }
+    if (f) atomicOr(&sh.flags, f);
+    sma[T] = asr;
+    unsigned epoch = 1;
+    // refinement state: warp 0
+    double sres = 0.0, sig = 1.0, isig = 1.0, res0 = 0.0, res = 0.0, tol = 0.0, rho = 0.0, rho_prev = 0.0, itol = 0.0;
+    int total = 0, outer = 0, inner_it = 0, status = FVGB_OK;
+    unsigned int flags = 0u;
+    __syncthreads();
+    if (wid < 2) {
+        // the sign flags of all blocks travel as an exact sum of 1, 2^10 and 2^20 per block
+        double v;
+        if (wid == 0) {
+            v = res_block_tree(sma);
+        } else {
+            const unsigned int g = sh.flags;
+            v = (double)((g & 1u) | ((g & 2u) << 9) | ((g & 4u) << 18));
+        }
+        if (lane == 0) ll_store(&mail->part[epoch & 1u][wid][blk].w, v, epoch);
+        double t;
+        const bool good = res_collect(gb, mail->part[epoch & 1u][wid], epoch, nblk, &t);
+        if (lane == 0) {
+            sh.v[wid] = t;
+            if (!good) sh.bad = 1;
+        }
+    }
+    __syncthreads();
+    bool done = sh.bad != 0, first = true;
+    if (wid == 0) {
+        sres = sqrt(sh.v[0]);
+        const unsigned int g = (unsigned)sh.v[1];
+        flags = ((g & 1023u) ? 1u : 0u) | ((g >> 10) & 1023u ? 2u : 0u) | ((g >> 20) ? 4u : 0u);
+    }
+    while (!done) {
+        if (!first) {
+            // x += y / sig, published behind a fence
+            const double is = sh.isig;
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                const int i = row0 + loc0 + 32 * j;
+                xr[j] = fma((double)yv[j], is, xr[j]);
+                if (i < n) x[i] = xr[j];
+            }
+            ++epoch;
+            __syncthreads();
+            if (wid == 0) {
+                if (lane == 0) {
+                    __threadfence();
+                    ll_store(&mail->part[epoch & 1u][0][blk].w, 0.0, epoch);
+                }
+                double t;
+                const bool good = res_collect(gb, mail->part[epoch & 1u][0], epoch, nblk, &t);
+                __threadfence();
+                if (!good && lane == 0) sh.bad = 1;
+            }
+        }
+        double nsig = 1.0, nisig = 1.0;
+        if (wid == 0) {
+            residual_scale(sres, &nsig, &nisig);
+            if (lane == 0) sh.nsig = nsig;
+        }
+        __syncthreads();
+        if (sh.bad) break;
+        // residual: r = b - A x (FP64), rh = sign*(float)(sig r), y = 0, z = |dinv| rh
+        const double ns = sh.nsig;
+        ++epoch;
+        if (!first) {
+#pragma unroll 1
+            for (int j = 0; j < R; ++j) {
+                const int i = row0 + loc0 + 32 * j;
+                if (i < n) stage[loc0 + 32 * j] = __ldg(&b[i]) - spmv_row_cg(m, val, x, i);
+            }
+        }
+        double arr = 0.0;
+        asr = 0.0;
+        float arho = 0.0f;
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int i = row0 + loc0 + 32 * j;
+            if (i >= n) continue;
+            const double r = stage[loc0 + 32 * j];
+            float t = (float)(r * ns);
+            if (di[j] < 0.0f) t = -t;
+            rh[j] = t;
+            yv[j] = 0.0f;
+            zr[j] = fabsf(di[j]) * t;
+            ll_store(z + i, zr[j], epoch);
+            arr = fma(r, r, arr);
+            asr = fma(r * (double)fabsf(di[j]), r, asr);
+            arho = fmaf(t, zr[j], arho);
+        }
+        sma[T] = arr;
+        smb[T] = asr;
+        smf[T] = arho;
+        __syncthreads();
+        if (wid < 3) {
+            LLLine* part = mail->part[epoch & 1u][wid];
+            const double v = wid == 0 ? res_block_tree(sma) : (wid == 1 ? res_block_tree(smb) : (double)res_block_tree(smf));
+            if (lane == 0) ll_store(&part[blk].w, v, epoch);
+            double t;
+            const bool good = res_collect(gb, part, epoch, nblk, &t);
+            if (lane == 0) {
+                sh.v[wid] = t;
+                if (!good) sh.bad = 1;
+            }
+        } else if (M.zh) {
+            if (!res_halo(gb, M, z, epoch, 96)) sh.bad = 1;
+        }
+        __syncthreads();
+        if (sh.bad) break;
+        if (wid == 0) {
+            const double rr = sh.v[0], sr2 = sh.v[1], nrho = sh.v[2];
+            bool d = false;
+            res = sqrt(rr);
+            if (!first) outer += 1;
+            if (first) {
+                res0 = res;
+                tol = prm.rel_tol * tol_base(&L.cases[0], res);
+                if (prm.abs_tol > tol) tol = prm.abs_tol;
+                if ((flags & 4u) || flags == 3u) {
+                    status = FVGB_ERR_UNSUPPORTED;
+                    d = true;
+                }
+            }
+            if (!d) {
+                if (!isfinite(res)) {
+                    status = FVGB_ERR_BREAKDOWN;
+                    d = true;
+                } else if (!(res > tol) || res == 0.0) {
+                    d = true;
+                } else if (outer >= prm.max_outer || total >= prm.max_iter) {
+                    status = FVGB_ERR_NOT_CONVERGED;
+                    d = true;
+                }
+            }
+            const double g = nsig * isig;
+            const double rho_rec = rho * g * g;
+            const bool restart = first || inner_it == 0 || nrho > 4.0 * rho_rec;
+            const float frel = restart ? -1.0f : (float)((nrho / rho_prev) * (sig * nisig));
+            sig = nsig;
+            isig = nisig;
+            sres = sqrt(sr2);
+            rho = nrho;
+            const double dr = prm.inner_rel_tol * prm.inner_rel_tol;
+            const double dt = (tol / res) * (tol / res);
+            itol = rho * (dr > dt ? dr : dt);
+            inner_it = 0;
+            if (lane == 0) {
+                sh.inner = !d && rho > itol && prm.inner_max_iter > 0 && total < prm.max_iter;
+                sh.done = d;
+                sh.isig = isig;
+                sh.restart = frel < 0.0f;
+                sh.fbeta = frel;
+            }
+        }
+        __syncthreads();
+        first = false;
+        done = sh.done;
+        if (done) break;
+        while (sh.inner) {
+            // p = z + beta p: the halo's copies, then the own rows
+            const bool restart = sh.restart;
+            const float fb = sh.fbeta;
+            if (!res_halo_dir(gb, M, z, epoch, restart, fb)) sh.bad = 1;
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                pr[j] = restart ? zr[j] : fmaf(fb, pr[j], zr[j]);
+                M.sp[loc0 + 32 * j] = pr[j];
+            }
+            __syncthreads();
+            // q = A p in the difference form, R rows interleaved; p.q
+            float q[R];
+            W.product(M, q, [](float xi, float xk) { return xk - xi; }, pr);
+            float acc = 0.0f;
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                q[j] = fmaf(ei[j], pr[j], q[j]);
+                if (row0 + loc0 + 32 * j < n) acc = fmaf(pr[j], q[j], acc);
+            }
+            smf[T] = acc;
+            ++epoch;
+            __syncthreads();
+            if (wid == 0) {
+                LLLine* part = mail->part[epoch & 1u][2];
+                const float v = res_block_tree(smf);
+                if (lane == 0) ll_store(&part[blk].w.w0, v, epoch);
+                double pq;
+                const bool good = res_collect<float>(gb, part, epoch, nblk, &pq);
+                const double alpha = rho / pq;
+                const bool brk = pq == 0.0 || !isfinite(alpha);
+                if (brk && inner_it == 0) status = FVGB_ERR_BREAKDOWN;
+                if (lane == 0) {
+                    sh.fa = (float)alpha;
+                    sh.brk = brk;
+                    if (brk) sh.inner = 0;
+                    if (brk && inner_it == 0) sh.done = 1;
+                    if (!good) sh.bad = 1;
+                }
+            }
+            __syncthreads();
+            if (sh.brk || sh.bad) break;
+            const float fa = sh.fa;
+            // y += alpha p, rh -= alpha q, z = |dinv| rh, rh.z
+            ++epoch;
+            acc = 0.0f;
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                const int i = row0 + loc0 + 32 * j;
+                yv[j] = fmaf(fa, pr[j], yv[j]);
+                rh[j] = fmaf(-fa, q[j], rh[j]);
+                zr[j] = fabsf(di[j]) * rh[j];
+                if (i < n) {
+                    ll_store(z + i, zr[j], epoch);
+                    acc = fmaf(rh[j], zr[j], acc);
+                }
+            }
+            smf[T] = acc;
+            __syncthreads();
+            if (wid == 0) {
+                LLLine* part = mail->part[epoch & 1u][2];
+                const float v = res_block_tree(smf);
+                if (lane == 0) ll_store(&part[blk].w.w0, v, epoch);
+                double rhon;
+                const bool good = res_collect<float>(gb, part, epoch, nblk, &rhon);
+                const float fbeta = (float)(rhon / rho);
+                rho_prev = rho;
+                rho = rhon;
+                inner_it += 1;
+                total += 1;
+                if (lane == 0) {
+                    sh.inner = rhon > itol && inner_it < prm.inner_max_iter && total < prm.max_iter;
+                    sh.restart = 0;
+                    sh.fbeta = fbeta;
+                    if (!good) sh.bad = 1;
+                }
+            } else if (M.zh) {
+                if (!res_halo(gb, M, z, epoch, 32)) sh.bad = 1;
+            }
+            __syncthreads();
+            if (sh.bad) break;
+        }
+        if (sh.bad) break;
+        done = sh.done;
+    }
+    if (blk == 0 && T == 0) {
+        CaseState* cs = &L.cases[0];
+        cs->res0 = res0;
+        cs->res = res;
+        cs->iter = 0;
+        cs->total = total;
+        cs->outer = outer;
+        cs->status = sh.bad ? FVGB_ERR_CUDA : status;
     }
 }

@@ -2463,7 +2463,8 @@ struct SolverCache {
     GridBar* bar = nullptr;
     ResMail* mail = nullptr;               // resident solves: partials and answers in flight
     LLWord* zll = nullptr;                 // resident solves: published preconditioned residuals [n]
-    int res_fit = -1;                      // resident solves: every block's part fits on its SM (-1: not asked yet)
+    unsigned long long* zll32 = nullptr;   // the same of the mixed solve
+    unsigned int res_need[4] = {~0u, ~0u, ~0u, ~0u};  // resident solves: shared memory of the largest block (k_res_need)
     float *pf2 = nullptr, *zf = nullptr;   // second direction buffer and z of the persistent mixed solve
     double* r0 = nullptr;                   // mixed: first FP64 residual, from the preparation kernel
     uint64_t converted_version = 0;        // fvgb_ls::version the FP32 matrix copy was formed from
@@ -3127,7 +3128,8 @@ int resident_blocks() {
         int sms = 0, coop = 0, per_sm = 1;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        for (const void* fn : {(const void*)k_pcg_resident<4>, (const void*)k_pcg_resident<8>}) {
+        for (const void* fn : {(const void*)k_pcg_resident<4>, (const void*)k_pcg_resident<8>,
+                               (const void*)k_ir_resident<4>, (const void*)k_ir_resident<8>}) {
             int b = 0;
             if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem) != cudaSuccess ||
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kT, kResSmem) != cudaSuccess)
@@ -3144,24 +3146,28 @@ int resident_blocks() {
 // Whether this system can be solved resident: at most one block per SM and every
 // block's matrix rows in its shared memory.  Asked once per system (one small
 // kernel and a read of its result); allocates what the solve keeps.
-bool resident_fits(SolverCache* c, cudaStream_t s) {
-    if (c->res_fit >= 0) return c->res_fit == 1;
+bool resident_fits(SolverCache* c, bool mixed, cudaStream_t s) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
-    c->res_fit = 0;
     if (c->nb > resident_blocks()) return false;
-    unsigned int need = ~0u, *d = nullptr;
-    if (calloc_dev(c, &d, 1) != cudaSuccess || settle_creation() != cudaSuccess) return false;
-    const MeshView m = c->ls->mesh->v;
-    if (rows_per_thread(c->n) == 8) k_res_need<8><<<c->nb, kT>>>(m, d);
-    else k_res_need<4><<<c->nb, kT>>>(m, d);
-    if (cudaMemcpy(&need, d, sizeof(need), cudaMemcpyDeviceToHost) != cudaSuccess || need > (unsigned)kResSmem)
-        return false;
-    if (calloc_dev(c, &c->mail, 1) != cudaSuccess || calloc_dev(c, &c->zll, (size_t)c->n) != cudaSuccess ||
-        settle_creation() != cudaSuccess)
-        return false;
-    c->res_fit = 1;
-    return true;
+    if (!c->mail || !(mixed ? (void*)c->zll32 : (void*)c->zll))
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    if (!c->mail) {
+        unsigned int* d = nullptr;
+        ResMail* mail = nullptr;
+        if (calloc_dev(c, &d, 4) != cudaSuccess || calloc_dev(c, &mail, 1) != cudaSuccess ||
+            settle_creation() != cudaSuccess)
+            return false;
+        const MeshView m = c->ls->mesh->v;
+        if (rows_per_thread(c->n) == 8) k_res_need<8><<<c->nb, kT>>>(m, d);
+        else k_res_need<4><<<c->nb, kT>>>(m, d);
+        if (cudaMemcpy(c->res_need, d, sizeof(c->res_need), cudaMemcpyDeviceToHost) != cudaSuccess) return false;
+        c->mail = mail;
+    }
+    if (c->res_need[mixed ? 1 : 0] > (unsigned)kResSmem) return false;
+    cudaError_t e = cudaSuccess;
+    if (mixed && !c->zll32) e = calloc_dev(c, &c->zll32, (size_t)c->n);
+    if (!mixed && !c->zll) e = calloc_dev(c, &c->zll, (size_t)c->n);
+    return e == cudaSuccess;
 }
 
 bool use_persistent(SolverCache* c, const fvgb_solver_cfg* cfg) {
@@ -3268,21 +3274,31 @@ fvgb_status launch(SolverCache* c, double* x, const fvgb_solver_cfg* cfg, fvgb_s
         const int pg = persistent_grid(c, mixed);
         const int grid = nvb < pg ? nvb : pg;
         FVGB_CUDA_TRY(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), s));
-        if (!mixed && resident_fits(c, s)) {
+        const bool r8 = rows_per_thread(c->n) == 8;
+        if (resident_fits(c, mixed, s)) {
             FVGB_CUDA_TRY(cudaMemsetAsync(c->mail, 0, sizeof(ResMail), s));
-            FVGB_CUDA_TRY(cudaMemsetAsync(c->zll, 0, sizeof(LLWord) * (size_t)c->n, s));
-            void* args[] = {&L, &m, &val, &b, &c->zll, &c->mail, &c->bar};
-            const void* fn = rows_per_thread(c->n) == 8 ? (const void*)k_pcg_resident<8> : (const void*)k_pcg_resident<4>;
-            FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, kResSmem, s));
+            const unsigned int* need = c->res_need + (mixed ? 1 : 0);
+            const size_t smem = need[2] <= (unsigned)kResSmem ? need[2] : need[0];
+            if (mixed) {
+                FVGB_CUDA_TRY(cudaMemsetAsync(c->zll32, 0, sizeof(*c->zll32) * (size_t)c->n, s));
+                void* args[] = {&L, &m, &val, &b, &c->ah, &c->ev, &c->dinvf, &c->zll32, &c->mail, &c->bar};
+                const void* fn = r8 ? (const void*)k_ir_resident<8> : (const void*)k_ir_resident<4>;
+                FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s));
+            } else {
+                FVGB_CUDA_TRY(cudaMemsetAsync(c->zll, 0, sizeof(LLWord) * (size_t)c->n, s));
+                void* args[] = {&L, &m, &val, &b, &c->zll, &c->mail, &c->bar};
+                const void* fn = r8 ? (const void*)k_pcg_resident<8> : (const void*)k_pcg_resident<4>;
+                FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s));
+            }
         } else if (mixed) {
             // k_ir_persistent(L, m, val, b, a32, ev, dinv, r0, rh, y, pbuf0, pbuf1, z, q, pa, pb, pc, gb, nvb)
             void* args[] = {&L,     &m,    &val,   &b,     &c->ah, &c->ev, &c->dinvf, &c->r0, &c->rh, &c->y,
                             &c->pf, &c->pf2, &c->zf, &c->qf, &c->pa, &c->pb, &c->pc,   &c->bar, &nvb};
-            const void* fn = rows_per_thread(c->n) == 8 ? (const void*)k_ir_persistent<8> : (const void*)k_ir_persistent<4>;
+            const void* fn = r8 ? (const void*)k_ir_persistent<8> : (const void*)k_ir_persistent<4>;
             FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPT), args, 0, s));
         } else {
             void* args[] = {&L, &m, &val, &b, &c->dinv, &c->r, &c->p, &c->q, &c->z, &c->pa, &c->pb, &c->bar, &nvb};
-            const void* fn = rows_per_thread(c->n) == 8 ? (const void*)k_pcg_persistent<8> : (const void*)k_pcg_persistent<4>;
+            const void* fn = r8 ? (const void*)k_pcg_persistent<8> : (const void*)k_pcg_persistent<4>;
             FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPT), args, 0, s));
         }
         k_finish<<<grid_for(c->ncases, 128), 128, 0, s>>>(c->L);
