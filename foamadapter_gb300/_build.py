@@ -40,7 +40,7 @@ CU_UNITS = {
     "ilu.cu": ["-fmad=false"],
 }
 CPP_UNITS = ["common.cpp", "meshgen.cpp", "foamio.cpp", "foamdict.cpp", "tunecache.cpp"]
-HEADERS = [INCLUDE / "fvgb.h", CSRC / "internal.cuh", CSRC / "resident.cuh",
+HEADERS = [INCLUDE / "fvgb.h", CSRC / "internal.cuh", CSRC / "resident.cuh", CSRC / "ll.cuh",
            CSRC / "fvgb_host_common.h", CSRC / "json_min.h", CSRC / "tunecache.h"]
 
 

@@ -441,6 +441,7 @@ extern "C" fvgb_status fvgb_mesh_create_boxes(const fvgb_box_spec* specs, int32_
     m->nslices = nslices;
     m->m_len = (int64_t)N * kMW;
     m->g_len = (int64_t)N * kGW;
+    m->g_width = kGW;
     MeshView& v = m->v;
     v.n = (int32_t)N;
     v.nif = (int32_t)NIF;

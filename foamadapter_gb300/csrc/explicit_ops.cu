@@ -14,6 +14,7 @@
 #include <string>
 
 #include "internal.cuh"
+#include "ll.cuh"
 #include "tunecache.h"
 
 namespace {
@@ -270,6 +271,191 @@ __global__ void __launch_bounds__(kThreads)
         else if (t == FVGB_BC_FIXED_GRADIENT) v = tn + (gq ? __ldg(&gq[b]) : __ldg(&ref[b]) / __ldg(&m.bdelta[b]));
         Tnew_b[b] = v;
     }
+}
+
+// nsteps of the fused step in one launch: a thread keeps its cell, the cell's fluxes
+// and where each face's upwind value comes from (the cell itself or another cell of
+// the block in shared memory, or a slot of its own: a boundary value, or a cell of
+// another block received with its step beside it, ll.cuh).  Per step a block waits
+// only for the cells next to its own, in both directions whatever the flow's (so
+// blocks stay within a step of each other and three step buffers suffice: a cell
+// seen at step k means its block is done reading step k - 2).  What bounds a step
+// is one round trip to L2 (~600 clocks, behind the publishing store's ~500) and a
+// cell's chain of 10 DFMAs (64 clocks each with one warp per scheduler).  64 x 64
+// cells: 1.3 us a step against 6.2 for a launch per step; 280 x 280: 2.9 against 14.
+template <int MAXT, int E>
+__global__ void __launch_bounds__(MAXT)
+    k_advect_steps(MeshView m, PatchTable pt, const double* __restrict__ flux, double* T, double* T_b, double dt,
+                   const double* __restrict__ ref, int nsteps, LLWord* ll, GridBar* gb) {
+    // [2][bs] cells of this block by step parity, [E][bs] slots, [E][bs] boundary constants, [E][bs] cells (int)
+    extern __shared__ double sm[];
+    const int bs = (int)blockDim.x, t = (int)threadIdx.x, c = blockIdx.x * bs + t, first = blockIdx.x * bs;
+    double* slot = sm + 2 * bs;
+    double* bq = slot + E * bs;
+    int* scell = (int*)(bq + E * bs);
+    double F[E], Tc = 0.0, iv = 0.0;
+    int src[E];  // index into sm; cells of the block (bit in `local`) add the step parity's offset
+    unsigned plus = 0u, remote = 0u, bnd = 0u, local = 0u, grad = 0u, fixed = 0u;
+    int cnt = 0;
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        F[j] = 0.0;
+        src[j] = t;
+    }
+    if (c < m.n) {
+        Entries e;
+        load_entries(m, c, e);
+        Tc = __ldcg(&T[c]);
+        iv = __ldg(&m.invV[c]);
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const int cd = e.code[j];
+            if (cd == FVGB_PAD) continue;
+            cnt = j + 1;
+            F[j] = __ldg(&flux[entry_face(cd)]);
+            const bool own = cd >= 0;
+            if (own) plus |= 1u << j;  // boundary faces are the cell's own too
+            const int o = e.other[j], d = o - first, mine = 2 * bs + j * bs + t;
+            if (cd >= m.nif) {
+                bnd |= 1u << j;
+                src[j] = mine;
+                sm[mine] = __ldcg(&T_b[o]);
+                scell[j * bs + t] = o;
+                const int ty = pt.type[__ldg(&m.bpatch[o])];
+                if (ty == FVGB_BC_FIXED_VALUE) {
+                    fixed |= 1u << j;
+                    bq[j * bs + t] = __ldg(&ref[o]);
+                } else if (ty == FVGB_BC_FIXED_GRADIENT) {
+                    grad |= 1u << j;
+                    bq[j * bs + t] = __ldg(&ref[o]) / __ldg(&m.bdelta[o]);
+                }
+                continue;
+            }
+            const bool away = (unsigned)d >= (unsigned)bs;
+            if (away) {
+                remote |= 1u << j;
+                scell[j * bs + t] = o;
+            }
+            if (nonneg(F[j]) != own) src[j] = away ? mine : d;  // the value across, else the cell's own
+            if (src[j] < bs) local |= 1u << j;
+        }
+    }
+    sm[t] = Tc;
+    bool bad = false;
+    const bool full = __all_sync(0xffffffffu, cnt == E);
+    LLWord *from = ll, *to = ll + m.n, *spare = ll + 2 * (size_t)m.n;  // step k - 1's cells, step k's, the next's
+    __syncthreads();
+    for (int k = 1; k <= nsteps; ++k) {
+        const int par = ((k - 1) & 1) * bs;
+        // Cells of other blocks: the first poll goes out at once, and the boundary
+        // values of the step before are formed during its round trip (~600 clocks).
+        unsigned long long a[E], b[E];
+        unsigned left = k > 1 ? remote : 0u;
+#pragma unroll
+        for (int j = 0; j < E; ++j)
+            if (left >> j & 1u) ll_issue(from + scell[j * bs + t], &a[j], &b[j]);
+        if (k == 1) {
+            for (int j = 0; j < E; ++j)
+                if (remote >> j & 1u) slot[j * bs + t] = __ldcg(&T[scell[j * bs + t]]);
+        } else if (grad | fixed) {
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                if (grad >> j & 1u) slot[j * bs + t] = Tc + bq[j * bs + t];
+                if (fixed >> j & 1u) slot[j * bs + t] = bq[j * bs + t];
+            }
+        }
+#pragma unroll 1
+        for (unsigned spins = 0; left; ++spins) {
+#pragma unroll
+            for (int j = 0; j < E; ++j)
+                if ((left >> j & 1u) && ll_take(a[j], b[j], (unsigned)(k - 1), &slot[j * bs + t])) left &= ~(1u << j);
+            if (left && ll_give_up(gb, spins)) {
+                bad = true;
+                break;
+            }
+#pragma unroll
+            for (int j = 0; j < E; ++j)
+                if (left >> j & 1u) ll_issue(from + scell[j * bs + t], &a[j], &b[j]);
+        }
+        LLWord* seen = from;  // from now on `from` is step k's buffer
+        from = to;
+        to = spare;
+        spare = seen;
+        double p[E], s;
+#pragma unroll
+        for (int j = 0; j < E; ++j) p[j] = sm[src[j] + (local >> j & 1u ? par : 0)];
+#pragma unroll
+        for (int j = 0; j < E; ++j) p[j] = fmul(m, F[j], p[j]);
+        s = cnt > 0 ? facc0(plus & 1u, p[0]) : 0.0;
+        if (full) {
+#pragma unroll
+            for (int j = 1; j < E; ++j) s = facc(m, s, plus >> j & 1u, p[j]);
+        } else {
+#pragma unroll
+            for (int j = 1; j < E; ++j) {
+                const double a = facc(m, s, plus >> j & 1u, p[j]);
+                s = j < cnt ? a : s;
+            }
+        }
+        const double dv = facc0(true, fmul(m, s, iv));  // +0 + s/V
+        Tc = fsub(m, Tc, fmul(m, dt, dv));
+        if (remote) ll_store(from + c, Tc, (unsigned)k);
+        sm[(k & 1) * bs + t] = Tc;
+        if (__syncthreads_or(bad)) {
+            bad = true;
+            break;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        if (grad >> j & 1u) slot[j * bs + t] = Tc + bq[j * bs + t];
+        if (fixed >> j & 1u) slot[j * bs + t] = bq[j * bs + t];
+    }
+    if (c < m.n) {
+        // a wait that ran out (seconds) leaves no number that could pass for a result
+        const double nan = __longlong_as_double(0x7ff8000000000000LL);
+        T[c] = bad ? nan : Tc;
+        for (int j = 0; j < cnt; ++j)
+            if (bnd >> j & 1u) T_b[scell[j * bs + t]] = bad ? nan : slot[j * bs + t];
+    }
+}
+
+struct AdvectPlan {
+    const void* fn = nullptr;  // null: the steps run one launch each
+    int threads = 0;
+    size_t smem = 0;
+};
+
+// One block per SM, from one warp per scheduler (128 threads) up, so that a step's
+// DFMA chain shares its scheduler with as few warps as the mesh allows; faces per
+// cell 4 (one-cell-thick meshes), 6 or 8.  None for wider cells, for more cells than
+// one 1024-thread block per SM holds, or for fewer than 4 steps (a block that is
+// done must not overtake a neighbour's first step: at least 3).
+inline AdvectPlan advect_plan(const fvgb_mesh* m, int nsteps) {
+    AdvectPlan p;
+    int dev = 0, sms = 0, coop = 0;
+    if (nsteps < 4 || m->g_width > kG || cudaGetDevice(&dev) != cudaSuccess) return p;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    const int64_t per_sm = ((int64_t)m->v.n + sms - 1) / sms;
+    const int bs = (int)std::max<int64_t>(128, (per_sm + 127) / 128 * 128);
+    if (!coop || per_sm > 1024) return p;
+    const int E = m->g_width <= 4 ? 0 : (m->g_width <= 6 ? 1 : 2), r = bs <= 256 ? 0 : (bs <= 512 ? 1 : 2);
+    static const void* const fns[3][3] = {
+        {(const void*)k_advect_steps<256, 4>, (const void*)k_advect_steps<256, 6>, (const void*)k_advect_steps<256, 8>},
+        {(const void*)k_advect_steps<512, 4>, (const void*)k_advect_steps<512, 6>, (const void*)k_advect_steps<512, 8>},
+        {(const void*)k_advect_steps<1024, 4>, (const void*)k_advect_steps<1024, 6>,
+         (const void*)k_advect_steps<1024, 8>}};
+    const void* fn = fns[r][E];
+    const int width = 4 + 2 * E;
+    p.smem = (size_t)bs * (8 * (2 + 2 * width) + 4 * width);
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess) {
+        cudaGetLastError();
+        return p;
+    }
+    p.fn = fn;
+    p.threads = bs;
+    return p;
 }
 
 // meshes up to this size advance with the one-pass step kernel (k_advect_euler,
@@ -1074,13 +1260,29 @@ extern "C" fvgb_status fvgb_advect_euler_steps(const fvgb_mesh* m, const double*
     FVGB_CHECK_ARG(bc->ref || !patch_table_needs_ref(pt), "fvgb_advect_euler_steps: ref is null");
     if (nsteps == 0) return FVGB_OK;
     cudaStream_t s = (cudaStream_t)stream;
+    const AdvectPlan plan = advect_plan(m, nsteps);
+    // GridBar, then the step buffers of the cells that cross blocks
+    const size_t ex_bytes = 128 + sizeof(LLWord) * 3 * (size_t)m->v.n;
+    char* ex = plan.fn ? (char*)face_buffer(ex_bytes / sizeof(double), s) : nullptr;
+    if (ex) {
+        MeshView v = m->v;
+        const double* ref = bc->ref;
+        GridBar* gb = (GridBar*)ex;
+        LLWord* ll = (LLWord*)(ex + 128);
+        cudaError_t e = cudaMemsetAsync(ex, 0, ex_bytes, s);
+        void* args[] = {&v, &pt, &flux, &T, &T_b, &dt, &ref, &nsteps, &ll, &gb};
+        if (e == cudaSuccess)
+            e = cudaLaunchCooperativeKernel(plan.fn, dim3(grid_for(v.n, plan.threads)), dim3(plan.threads), args,
+                                            plan.smem, s);
+        cudaFreeAsync(ex, s);
+        if (e != cudaSuccess) return cuda_fail(e, "fvgb_advect_euler_steps");
+        return FVGB_OK;
+    }
     // the fixed-gradient boundary quotients ref/delta do not change between
     // steps: formed once for the whole call
-    double* gq = nullptr;
-    if (m->v.nbf > 0 && cudaMallocAsync(&gq, sizeof(double) * (size_t)m->v.nbf, s) == cudaSuccess)
-        k_bc_gradq<<<grid_for(m->v.nbf, kThreads), kThreads, 0, s>>>(m->v, pt, bc->ref, gq);
-    else
-        cudaGetLastError();  // without the buffer each step forms its quotients itself
+    // (without the buffer each step forms its quotients itself)
+    double* gq = m->v.nbf > 0 ? face_buffer((size_t)m->v.nbf, s) : nullptr;
+    if (gq) k_bc_gradq<<<grid_for(m->v.nbf, kThreads), kThreads, 0, s>>>(m->v, pt, bc->ref, gq);
     fvgb_status st = FVGB_OK;
     if (m->v.n <= kStepsMaxCells) {
         for (int k = 0; k < nsteps; ++k) {

@@ -239,6 +239,7 @@ extern "C" fvgb_status fvgb_mesh_create(const fvgb_mesh_desc* d, fvgb_mesh** out
     }
     SellPack gs = sell_shape(go, n);
     m->g_len = gs.len;
+    for (size_t k = 0; k + 1 < gs.ptr.size(); ++k) m->g_width = std::max(m->g_width, (gs.ptr[k + 1] - gs.ptr[k]) / kSlice);
     std::vector<int32_t> sg_code(gs.len, FVGB_PAD), sg_other(gs.len, 0);
     for (int32_t c = 0; c < n; ++c)
         for (int32_t k = 0; k < go[c + 1] - go[c]; ++k) {

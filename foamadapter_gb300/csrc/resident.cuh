@@ -10,10 +10,7 @@
 // rows first, then one entry per slot that reaches into another block (a halo
 // entry).  Only the halo and the dot products cross blocks.
 //
-// Everything that crosses blocks carries its epoch beside the data: a value
-// travels as two 8-byte words, each half the value and the 32-bit epoch, so a
-// reader polls the data itself and no fence, counter or second read is needed
-// (a fence behind the vector stores costs 930 clocks here, one such hop 570).
+// Everything that crosses blocks carries its epoch beside the data (ll.cuh).
 //  * Halo: an owner publishes the preconditioned residual z of its rows; a
 //    reader keeps its own copy of the halo's direction and forms the new one,
 //    p = z + beta p, with the owner's arithmetic.
@@ -33,9 +30,6 @@ constexpr int kResMaxBlocks = 160;       // 5 partials per polling lane
 // of a few KB takes 2,700 clocks instead of 1,400.
 constexpr int kResSmem = 220 * 1024;
 
-struct alignas(16) LLWord {  // one published value
-    unsigned long long w0, w1;  // epoch << 32 | low half, epoch << 32 | high half
-};
 struct alignas(128) LLLine {
     LLWord w;  // an FP64 partial; an FP32 one takes w.w0 alone
 };
@@ -44,43 +38,6 @@ struct ResMail {
 };
 // Two parities suffice: a block publishes epoch e after it has every block's
 // partial of e - 1, and a block publishes that after it is done with epoch e - 2.
-
-__device__ __forceinline__ void ll_store(LLWord* p, double v, unsigned epoch) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(v), e = (unsigned long long)epoch << 32;
-    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(e | (u & 0xffffffffull)),
-                 "l"(e | (u >> 32))
-                 : "memory");
-}
-__device__ __forceinline__ bool ll_load(const LLWord* p, unsigned epoch, double* v) {
-    unsigned long long a, b;
-    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-    *v = __longlong_as_double((long long)((b << 32) | (a & 0xffffffffull)));
-    return (unsigned)(a >> 32) == epoch && (unsigned)(b >> 32) == epoch;
-}
-
-// a float travels as one word
-__device__ __forceinline__ void ll_store(unsigned long long* p, float v, unsigned epoch) {
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p),
-                 "l"(((unsigned long long)epoch << 32) | __float_as_uint(v))
-                 : "memory");
-}
-__device__ __forceinline__ bool ll_load(const unsigned long long* p, unsigned epoch, float* v) {
-    unsigned long long a;
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
-    *v = __uint_as_float((unsigned)a);
-    return (unsigned)(a >> 32) == epoch;
-}
-
-// Bound of every wait: true when it has run out, here or in another block.
-__device__ __forceinline__ bool res_give_up(GridBar* gb, unsigned spins) {
-    if ((spins & 63u) != 63u) return false;
-    int ab;
-    asm volatile("ld.relaxed.gpu.s32 %0, [%1];" : "=r"(ab) : "l"(&gb->abort) : "memory");
-    if (ab) return true;
-    if (spins < (1u << 23)) return false;  // seconds
-    atomicExch(&gb->abort, 1);
-    return true;
-}
 
 // v, or +0 for a zero of either sign: the sum 0.0 + v
 __device__ __forceinline__ double plus_zero(double v) {
@@ -118,7 +75,7 @@ __device__ __forceinline__ bool res_collect(GridBar* gb, const LLLine* part, uns
             all = all && have[s];
         }
         if (__all_sync(0xffffffffu, all)) break;
-        if (__any_sync(0xffffffffu, res_give_up(gb, spins))) {
+        if (__any_sync(0xffffffffu, ll_give_up(gb, spins))) {
             good = false;
             break;
         }
@@ -277,7 +234,7 @@ __device__ __forceinline__ bool res_halo(GridBar* gb, const ResMatrix<V>& M, con
                 all = all && have[u];
             }
             if (all) break;
-            if (res_give_up(gb, spins)) return false;
+            if (ll_give_up(gb, spins)) return false;
         }
     }
     return true;
@@ -301,7 +258,7 @@ __device__ __forceinline__ bool res_halo_dir(GridBar* gb, const ResMatrix<V>& M,
             unsigned spins = 0;
 #pragma unroll 1
             while (!ll_load(z + M.hcol[h], epoch, &v))
-                if (res_give_up(gb, spins++)) {
+                if (ll_give_up(gb, spins++)) {
                     good = false;
                     break;
                 }

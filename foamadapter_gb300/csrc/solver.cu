@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "ll.cuh"
 #include "tunecache.h"
 
 #include <algorithm>
@@ -1716,11 +1717,6 @@ cudaError_t launch_variant(const void* fn, unsigned grid, cudaStream_t s, A... a
 // barrier and the solve reports FVGB_ERR_CUDA.
 constexpr int kPT = 1024;
 static_assert((kT * 4) % kPT == 0, "a virtual block is a whole number of rows per thread");
-
-struct GridBar {
-    unsigned long long count;  // arrivals since the launch (never reset inside it)
-    int abort, pad;
-};
 
 // Barrier number `epoch` (1, 2, ...) of a grid of `nblocks` blocks.
 __device__ __forceinline__ bool grid_sync(GridBar* g, unsigned long long target) {
