@@ -440,6 +440,7 @@ extern "C" fvgb_status fvgb_mesh_create_boxes(const fvgb_box_spec* specs, int32_
     m->nnz = (int32_t)(N + 2 * NIF);
     m->nslices = nslices;
     m->m_len = (int64_t)N * kMW;
+    m->m_width = kMW;
     m->g_len = (int64_t)N * kGW;
     m->g_width = kGW;
     MeshView& v = m->v;

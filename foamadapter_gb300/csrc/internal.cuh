@@ -128,6 +128,7 @@ struct fvgb_mesh {
     int32_t nnz = 0;
     int32_t nslices = 0;
     int64_t m_len = 0, g_len = 0;
+    int32_t m_width = 0;         // most slots of any slice of the matrix
     int32_t g_width = 0;         // most faces of any cell's slice in the gather lists
     int32_t* csr_pos = nullptr;  // [nnz] slot of CSR entry j
     std::vector<int32_t> h_patch_offs;

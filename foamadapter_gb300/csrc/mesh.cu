@@ -173,6 +173,7 @@ extern "C" fvgb_status fvgb_mesh_create(const fvgb_mesh_desc* d, fvgb_mesh** out
     SellPack ms = sell_shape(ro, n);
     m->nslices = (int32_t)ms.ptr.size() - 1;
     m->m_len = ms.len;
+    for (size_t k = 0; k + 1 < ms.ptr.size(); ++k) m->m_width = std::max(m->m_width, (ms.ptr[k + 1] - ms.ptr[k]) / kSlice);
     std::vector<int32_t> s_col(ms.len), s_code(ms.len, FVGB_PAD), csr_pos(nnz), diag_pos(n),
         own_pos(nif), nei_pos(nif);
     for (int64_t i = 0; i < ms.len; ++i) s_col[i] = 0;

@@ -121,22 +121,21 @@ __host__ __device__ inline size_t res_bytes(int v, int rows, int len, int nh, bo
            2 * (size_t)len;
 }
 
-// Slots and halo entries of block row0's rows (all threads; counter: shared).
-template <int R>
-__device__ __forceinline__ void res_count(const MeshView& m, int row0, int* counter, int* len, int* nh) {
-    constexpr int ROWS = kT * R;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int s0 = row0 >> 5, s1 = min((m.n + 31) >> 5, s0 + ROWS / 32);
+// Slots and halo entries of the block's rows [row0, row0 + rows) (all threads;
+// counter: shared).
+__device__ __forceinline__ void res_count(const MeshView& m, int row0, int rows, int* counter, int* len, int* nh) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
+    const int ns = (m.n + 31) >> 5, s0 = min(ns, row0 >> 5), s1 = min(ns, s0 + rows / 32);
     *len = __ldg(&m.m_ptr[s1]) - __ldg(&m.m_ptr[s0]);
     if (threadIdx.x == 0) *counter = 0;
     __syncthreads();
 #pragma unroll 1
-    for (int s = s0 + wid; s < s1; s += kT / 32) {
+    for (int s = s0 + wid; s < s1; s += nw) {
         const int b0 = __ldg(&m.m_ptr[s]), w = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5, i = s * 32 + lane;
         int c = 0;
 #pragma unroll 1
         for (int k = 0; k < w; ++k)
-            c += (unsigned)(slot_col(m, b0 + k * 32 + lane, i) - row0) >= (unsigned)ROWS;
+            c += (unsigned)(slot_col(m, b0 + k * 32 + lane, i) - row0) >= (unsigned)rows;
         c = __reduce_add_sync(0xffffffffu, c);
         if (lane == 0 && c) atomicAdd(counter, c);
     }
@@ -151,7 +150,7 @@ template <int R>
 __global__ void __launch_bounds__(kT) k_res_need(MeshView m, unsigned int* need) {
     __shared__ int counter;
     int len, nh;
-    res_count<R>(m, (int)blockIdx.x * (kT * R), &counter, &len, &nh);
+    res_count(m, (int)blockIdx.x * (kT * R), kT * R, &counter, &len, &nh);
     if (threadIdx.x < 4) {
         const size_t b = kT * R + nh > 65536 ? ~(size_t)0
                                              : res_bytes(threadIdx.x & 1 ? 4 : 8, kT * R, len, nh, threadIdx.x >= 2);
@@ -160,33 +159,33 @@ __global__ void __launch_bounds__(kT) k_res_need(MeshView m, unsigned int* need)
 }
 
 // Lays the block's part out and fills the columns; the values are the caller's.
-template <int R, class V>
-__device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned char* dyn, int row0, int* counter) {
-    constexpr int ROWS = kT * R;
-    const int T = threadIdx.x, lane = T & 31, wid = T >> 5;
-    const int s0 = row0 >> 5, s1 = min((m.n + 31) >> 5, s0 + ROWS / 32);
+template <class V>
+__device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned char* dyn, int row0, int rows,
+                                                 int* counter) {
+    const int T = threadIdx.x, lane = T & 31, wid = T >> 5, nw = (int)blockDim.x >> 5;
+    const int ns = (m.n + 31) >> 5, s0 = min(ns, row0 >> 5), s1 = min(ns, s0 + rows / 32);
     ResMatrix<V> M;
     int len;
-    res_count<R>(m, row0, counter, &len, &M.nh);
+    res_count(m, row0, rows, counter, &len, &M.nh);
     M.pos0 = __ldg(&m.m_ptr[s0]);
     unsigned int have;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(have));
-    const bool zh = res_bytes((int)sizeof(V), ROWS, len, M.nh, true) <= (size_t)have;
-    M.sp = (V*)(dyn + (sizeof(V) == 4 ? 8 * ROWS : 0));
-    M.sval = M.sp + ROWS + M.nh;
+    const bool zh = res_bytes((int)sizeof(V), rows, len, M.nh, true) <= (size_t)have;
+    M.sp = (V*)(dyn + (sizeof(V) == 4 ? 8 * rows : 0));
+    M.sval = M.sp + rows + M.nh;
     M.zh = zh ? M.sval + len : nullptr;
     M.hcol = (int*)(M.sval + len + (zh ? M.nh : 0));
     M.scol = (unsigned short*)(M.hcol + M.nh);
     if (T == 0) *counter = 0;
     __syncthreads();
 #pragma unroll 1
-    for (int s = s0 + wid; s < s1; s += kT / 32) {
+    for (int s = s0 + wid; s < s1; s += nw) {
         const int b0 = __ldg(&m.m_ptr[s]), w = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5, i = s * 32 + lane;
 #pragma unroll 1
         for (int k = 0; k < w; ++k) {
             const int pos = b0 + k * 32 + lane;
             const int c = slot_col(m, pos, i), d = c - row0;
-            const bool halo = (unsigned)d >= (unsigned)ROWS;
+            const bool halo = (unsigned)d >= (unsigned)rows;
             const unsigned ball = __ballot_sync(0xffffffffu, halo);
             int base = 0;
             if (ball) {
@@ -198,7 +197,7 @@ __device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned cha
             if (halo) {
                 const int h = base + __popc(ball & ((1u << lane) - 1));
                 M.hcol[h] = c;
-                idx = ROWS + h;
+                idx = rows + h;
             }
             M.scol[pos - M.pos0] = (unsigned short)idx;
         }
@@ -345,7 +344,7 @@ __global__ void __launch_bounds__(kT, 1)
     const SolverParams prm = L.bs->prm;
     double* x = prm.x;
     if (T == 0) sh.bad = 0;
-    const ResMatrix<double> M = res_load<R, double>(m, dyn, row0, &sh.counter);
+    const ResMatrix<double> M = res_load<double>(m, dyn, row0, ROWS, &sh.counter);
     // cold code in rolled loops: the kernel's iteration has to stay in the
     // instruction cache (unrolled over the rows it was 97 KB)
 #pragma unroll 1
@@ -548,7 +547,7 @@ __global__ void __launch_bounds__(kT, 1)
         sh.flags = 0u;
     }
     double* stage = (double*)dyn;  // [rows] FP64 residuals
-    const ResMatrix<float> M = res_load<R, float>(m, dyn, row0, &sh.counter);
+    const ResMatrix<float> M = res_load<float>(m, dyn, row0, ROWS, &sh.counter);
     // prepare: dinv, a32, ev (formed, or those of the unchanged matrix), sign flags, |D^-1/2 (b - A x0)|
     unsigned int f = 0u;
     double asr = 0.0;
@@ -857,4 +856,323 @@ __global__ void __launch_bounds__(kT, 1)
         cs->outer = outer;
         cs->status = sh.bad ? FVGB_ERR_CUDA : status;
     }
+}
+
+// ---------------------------------------------------------- one cluster (small systems)
+// FP64 CG of at most kClMaxUnits tree warps (4-row tree) in ONE thread-block cluster:
+// the reduction tree's warps ("units", 128 consecutive rows) are spread over its
+// blocks, a thread holding one row, so the rows of a virtual block share out over up
+// to 8 SMs' FP64 pipes.  Everything that crosses blocks is a word with its epoch
+// (ll.cuh) in distributed shared memory: a unit sends its 32 lane partials to the
+// block that forms its virtual block's tree, that block sends the result to all, and
+// the halo's z is polled where its owner keeps it.  What bounds an iteration is its
+// ~55 dependent FP64 instructions (64 clocks each) in the chains, trees and
+// divisions, then four hops of 700 clocks.  40 x 40 cavity pressure (1,600 rows, 13
+// of 16 blocks): 4.4 us an iteration against 7.5 for k_pcg_resident's two blocks.
+// Measured slower: every unit's partials to every block (one hop less, but a
+// warp's 16 stores of 512 bytes take 450 clocks; 4.9 us with the trees in every
+// block), cluster barriers in place of the words (5.2), partials read by the trees
+// across the cluster (5.1).
+constexpr int kClRows = 128;     // rows of a unit: 32 lanes x 4 rows
+constexpr int kClMaxUnits = 32;  // two per block of a 16-block cluster
+constexpr int kClMaxVb = kClMaxUnits / 8;
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// address of this block's shared object p in block `rank`
+__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cl_store(unsigned at, double v, unsigned epoch) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v), e = (unsigned long long)epoch << 32;
+    asm volatile("st.relaxed.cluster.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(at), "l"(e | (u & 0xffffffffull)),
+                 "l"(e | (u >> 32))
+                 : "memory");
+}
+__device__ __forceinline__ bool cl_load(unsigned at, unsigned epoch, double* v) {
+    unsigned long long a, b;
+    asm volatile("ld.relaxed.cluster.shared::cluster.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(at) : "memory");
+    return ll_take(a, b, epoch, v);
+}
+// the same of this block's own words (through the cluster's window each poll would
+// take the network's latency)
+__device__ __forceinline__ bool cl_load_own(unsigned at, unsigned epoch, double* v) {
+    unsigned long long a, b;
+    asm volatile("ld.relaxed.cluster.shared::cta.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(at) : "memory");
+    return ll_take(a, b, epoch, v);
+}
+constexpr unsigned kClSpins = 1u << 23;  // bound of every wait: seconds
+
+struct ClShared {
+    LLWord part[2][2][8][32];            // [epoch parity][dot product][unit of the virtual block formed here][lane]
+    LLWord val[2][2][kClMaxVb];          // [epoch parity][dot product][virtual block]
+    LLWord z[2 * kClRows];               // this block's z, polled by the others
+    double a[2 * kClRows], b[2 * kClRows];  // staged operands of the dot products
+    double value;
+    int code, bad, counter;
+};
+
+// One warp: lane partials of the block's unit u as the tree thread sums them, sent to
+// `at` (the slot of lane 0).
+__device__ __forceinline__ void cl_chain(unsigned at, unsigned epoch, const double* a, const double* b, int u,
+                                         int row0, int n) {
+    const int lane = threadIdx.x & 31;
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int l = u * kClRows + 32 * j + lane;
+        if (row0 + l < n) acc = fma(a[l], b[l], acc);
+    }
+    cl_store(at + 16u * lane, acc, epoch);
+}
+
+// One warp: a virtual block's partial from its k1 units' lanes as they arrive at
+// `part` (block_tree), sent to `val`, lane r's address in block r.
+__device__ __forceinline__ bool cl_tree(unsigned part, unsigned epoch, int k1, unsigned val, int ncta) {
+    const int lane = threadIdx.x & 31;
+    const unsigned at = part + 16u * lane;
+    double t[8];
+    bool good = true;
+#pragma unroll 1
+    for (unsigned spins = 0;; ++spins) {
+        bool all = true;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) all = (cl_load_own(at + 512u * k, epoch, &t[k]) || k >= k1) && all;
+        if (__all_sync(0xffffffffu, all)) break;
+        if (spins > kClSpins) {
+            good = false;
+            break;
+        }
+    }
+    double s = t[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+        if (k >= k1) break;
+        s = s + t[k];
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, off);
+    if (lane < ncta) cl_store(val, s, epoch);
+    return good;
+}
+
+// One warp: final_tree over the virtual blocks' partials as they arrive (the
+// butterfly's other terms are +0).
+__device__ __forceinline__ bool cl_final(const LLWord* val, unsigned epoch, int nvb, double* out) {
+    const unsigned at = (unsigned)__cvta_generic_to_shared(val);
+    double v[kClMaxVb];
+    bool good = true;
+#pragma unroll 1
+    for (unsigned spins = 0;; ++spins) {
+        bool all = true;
+#pragma unroll
+        for (int k = 0; k < kClMaxVb; ++k) all = (cl_load_own(at + 16u * k, epoch, &v[k]) || k >= nvb) && all;
+        if (__all_sync(0xffffffffu, all)) break;
+        if (spins > kClSpins) {
+            good = false;
+            break;
+        }
+    }
+    static_assert(kClMaxVb == 4, "two butterfly steps");
+#pragma unroll
+    for (int k = 0; k < kClMaxVb; ++k) v[k] = k < nvb ? plus_zero(v[k]) : 0.0;
+    if (nvb > 2) {
+        v[0] = v[0] + v[2];
+        v[1] = v[1] + v[3];
+    }
+    *out = nvb > 1 ? v[0] + v[1] : v[0];
+    return good;
+}
+
+__global__ void __launch_bounds__(2 * kClRows, 1)
+    k_pcg_cluster(Layout L, MeshView m, const double* __restrict__ val, const double* __restrict__ b, int units) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ ClShared sh;
+    const int n = m.n, T = threadIdx.x, lane = T & 31, wid = T >> 5, nw = (int)blockDim.x >> 5;
+    const int rows = (int)blockDim.x, lg = rows == kClRows ? 7 : 8;  // one unit per block, or two
+    const int rank = (int)blockIdx.x, ncta = (int)gridDim.x;
+    const int row0 = rank * rows, i = row0 + T, nvb = (units + 7) / 8;
+    const SolverParams prm = L.bs->prm;
+    double* x = prm.x;
+    for (int k = T; k < (int)(offsetof(ClShared, a) / sizeof(LLWord)); k += rows) ((LLWord*)&sh)[k] = LLWord{0ull, 0ull};
+    if (T == 0) sh.code = sh.bad = 0;
+    const ResMatrix<double> M = res_load<double>(m, dyn, row0, rows, &sh.counter);
+    // this thread's row, its slots (at most 8) in registers
+    double xr = 0.0, rv = 0.0, pr = 0.0, di = 0.0, v8[8];
+    int c8[8], w = 0, b0 = 0;
+    if ((i & ~31) < n) {
+        b0 = __ldg(&m.m_ptr[i >> 5]);
+        w = (__ldg(&m.m_ptr[(i >> 5) + 1]) - b0) >> 5;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        v8[k] = k < w ? __ldg(&val[b0 + lane + 32 * k]) : 0.0;
+        c8[k] = k < w ? M.scol[b0 - M.pos0 + lane + 32 * k] : 0;
+    }
+    if (i < n) {
+        xr = x[i];
+        di = 1.0 / __ldg(&val[__ldg(&m.diag_pos[i])]);
+        rv = __ldg(&b[i]) - spmv_row_cg(m, val, x, i);
+    }
+    // where this thread's first halo entry lives
+    unsigned hat = 0u;
+    if (T < M.nh) hat = cluster_addr(&sh.z[M.hcol[T] & (rows - 1)], M.hcol[T] >> lg);
+    double rz = 0.0, tol = 0.0, res0 = 0.0, res = 0.0, alpha = 0.0;  // warp 0: rz; the last warp: the residual's
+    int iter = 0, status = FVGB_OK;
+    // chain warps: a unit's two dot products on warps of different schedulers; the tree
+    // of dot product d of virtual block v is formed by warp 2 of block d * nvb + v (or
+    // that modulo the cluster's size: at most 8 trees, and never two on one warp when
+    // the cluster has as many blocks)
+    const int cu = wid >> 2, first_w = 4 * cu + (cu & 1) * 2;  // of the unit this warp belongs to
+    const int unit = rank * (rows / kClRows) + cu;
+    const int chain = unit < units ? wid - first_w : -1;  // the dot product this warp's chain forms (0, 1), if any
+    int tree2 = -1, tree1 = -1;                           // the trees this warp forms: dot * nvb + virtual block
+    for (int q = rank, k = 2; q < 2 * nvb; q += ncta, ++k)
+        if (wid == k % nw) {
+            tree2 = q;
+            if (q < nvb) tree1 = q;
+        }
+    const int tdot = tree2 >= nvb, tv = tree2 - tdot * nvb, tk = min(units - 8 * tv, 8);
+    // addresses with epoch parity 0; parity 1 is one array further
+    constexpr unsigned kPartPar = sizeof(LLWord) * 2 * 8 * 32, kValPar = sizeof(LLWord) * 2 * kClMaxVb;
+    unsigned to2 = 0u, to1 = 0u, tval = 0u;
+    if (chain == 0 || chain == 1)
+        to2 = cluster_addr(sh.part[0][chain][unit & 7], (chain * nvb + (unit >> 3)) % ncta);
+    if (chain == 0) to1 = to2;
+    if (tree2 >= 0 && lane < ncta) tval = cluster_addr(&sh.val[0][tdot][tv], lane);
+    const unsigned tpart = (unsigned)__cvta_generic_to_shared(sh.part[0][tdot]);
+    bool first = true;
+    unsigned epoch = 0;
+    cluster_arrive();  // every block has cleared its words
+    cluster_wait();
+    for (;;) {
+        // z = dinv r, r.z, r.r
+        ++epoch;
+        const unsigned par = epoch & 1u;
+        const double z = __fma_rn(di, rv, m.k_nzero);
+        sh.a[T] = z;
+        sh.b[T] = rv;
+        cl_store((unsigned)__cvta_generic_to_shared(&sh.z[T]), z, epoch);
+        __syncthreads();
+        if (chain == 0 || chain == 1) cl_chain(to2 + par * kPartPar, epoch, sh.b, chain ? sh.b : sh.a, cu, row0, n);
+        if (!first) xr = fma(alpha, pr, xr);  // off the reduction's path
+        bool good = true;
+        if (tree2 >= 0) good = cl_tree(tpart + par * kPartPar, epoch, tk, tval + par * kValPar, ncta);
+        double rr = 0.0;
+        if (wid == 0) {
+            double t;
+            good = cl_final(sh.val[par][0], epoch, nvb, &t) && good;
+            const double beta = t / rz;
+            rz = t;
+            if (lane == 0) sh.value = beta;
+        } else if (wid == nw - 1) {
+            good = cl_final(sh.val[par][1], epoch, nvb, &rr) && good;
+        }
+        // the halo's z
+        double hz = 0.0;
+        if (T < M.nh) {
+            unsigned spins = 0;
+            while (!cl_load(hat, epoch, &hz))
+                if (++spins > kClSpins) {
+                    good = false;
+                    break;
+                }
+        }
+        if (!good) sh.bad = 1;
+        __syncthreads();
+        // p = z + beta p: the halo's copies and the own row
+        const double beta = sh.value;
+        if (T < M.nh) M.sp[rows + T] = first ? hz : fma(beta, M.sp[rows + T], hz);
+#pragma unroll 1
+        for (int h = T + rows; h < M.nh; h += rows) {
+            const unsigned at = cluster_addr(&sh.z[M.hcol[h] & (rows - 1)], M.hcol[h] >> lg);
+            unsigned spins = 0;
+            while (!cl_load(at, epoch, &hz))
+                if (++spins > kClSpins) {
+                    sh.bad = 1;
+                    break;
+                }
+            M.sp[rows + h] = first ? hz : fma(beta, M.sp[rows + h], hz);
+        }
+        pr = first ? z : fma(beta, pr, z);
+        M.sp[T] = pr;
+        __syncthreads();
+        // q = A p, p.q
+        double q = 0.0, x8[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x8[k] = M.sp[c8[k]];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k >= w) break;  // w is the warp's
+            q = fma(v8[k], x8[k], q);
+        }
+        sh.b[T] = q;
+        ++epoch;
+        const unsigned par1 = epoch & 1u;
+        __syncthreads();
+        if (chain == 0) cl_chain(to1 + par1 * kPartPar, epoch, M.sp, sh.b, cu, row0, n);
+        if (tree1 >= 0 && !cl_tree(tpart + par1 * kPartPar, epoch, tk, tval + par1 * kValPar, ncta)) sh.bad = 1;
+        // the stopping test of the residual, while the partials are under way: x is
+        // already the iterate it belongs to, and nothing of this product is used
+        // when it ends the solve
+        if (wid == nw - 1) {
+            res = sqrt(rr);
+            int d = 0;
+            if (first) {
+                res0 = res;
+                tol = prm.rel_tol * tol_base(&L.cases[0], res);
+                if (prm.abs_tol > tol) tol = prm.abs_tol;
+                d = !(res > tol) || res == 0.0;
+                if (!isfinite(res)) {
+                    d = 1;
+                    status = FVGB_ERR_BREAKDOWN;
+                } else if (!d && prm.max_iter <= 0) {
+                    d = 1;
+                    status = FVGB_ERR_NOT_CONVERGED;
+                }
+            } else {
+                ++iter;
+                if (!isfinite(res)) {
+                    status = FVGB_ERR_BREAKDOWN;
+                    d = 1;
+                } else if (!(res > tol)) {
+                    d = 1;
+                } else if (iter >= prm.max_iter) {
+                    status = FVGB_ERR_NOT_CONVERGED;
+                    d = 1;
+                }
+            }
+            if (d && lane == 0) sh.code = 1;
+        }
+        int brk = 0;
+        if (wid == 0) {
+            double pq;
+            if (!cl_final(sh.val[par1][0], epoch, nvb, &pq)) sh.bad = 1;
+            const double a = rz / pq;
+            const long long ua = __double_as_longlong(a), up = __double_as_longlong(pq);
+            brk = (up << 1) == 0 || (ua & 0x7ff0000000000000ll) == 0x7ff0000000000000ll;
+            if (lane == 0) sh.value = a;
+        }
+        brk = __syncthreads_or(brk);
+        if (sh.code || sh.bad) break;
+        if (brk) {
+            status = FVGB_ERR_BREAKDOWN;
+            break;
+        }
+        alpha = sh.value;
+        rv = fma(-alpha, q, rv);
+        first = false;
+    }
+    if (i < n) x[i] = xr;
+    if (rank == 0 && wid == nw - 1 && lane == 0) {
+        CaseState* cs = &L.cases[0];
+        cs->res0 = res0;
+        cs->res = res;
+        cs->iter = iter;
+        cs->status = sh.bad ? FVGB_ERR_CUDA : status;
+    }
+    cluster_arrive();  // no block leaves while another may read its shared memory
+    cluster_wait();
 }

@@ -3139,6 +3139,58 @@ int resident_blocks() {
     return blocks;
 }
 
+// The one-cluster solve of a system of `units` tree warps: the cluster's size (0:
+// does not fit the device), the threads of a block, its shared memory.
+struct ClusterPlan {
+    int ctas = 0, threads = 0, units = 0;
+    size_t smem = 0;
+};
+
+// Rows of up to 8 slots, all of them halo; wider rows take the grid-wide resident solve.
+size_t cluster_smem(int U) {
+    return res_bytes(8, U * kClRows, U * kClRows * 8, U * kClRows * 8, false);
+}
+
+ClusterPlan cluster_plan(const SolverCache* c) {
+    ClusterPlan p;
+    const int units = (c->n + kClRows - 1) / kClRows;
+    if (units > kClMaxUnits || rows_per_thread(c->n) != 4 || c->ls->mesh->m_width > 8) return p;
+    const int U = units > 16 ? 2 : 1;
+    int ctas = 1;
+    while (ctas * U < units) ctas *= 2;
+    p.smem = cluster_smem(U);
+    p.threads = U * kClRows;
+    p.units = units;
+    static thread_local int dev_of = -1, most = 0;  // the largest cluster the device runs
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return p;
+    if (dev != dev_of) {
+        most = 0;
+        if (cudaFuncSetAttribute(k_pcg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaFuncSetAttribute(k_pcg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)cluster_smem(2)) == cudaSuccess) {
+            for (int k = 16; k >= 1 && !most; k /= 2) {
+                cudaLaunchConfig_t lc{};
+                cudaLaunchAttribute at{};
+                at.id = cudaLaunchAttributeClusterDimension;
+                at.val.clusterDim.x = (unsigned)k;
+                at.val.clusterDim.y = at.val.clusterDim.z = 1;
+                lc.gridDim = dim3((unsigned)k);
+                lc.blockDim = dim3(2 * kClRows);
+                lc.dynamicSmemBytes = cluster_smem(2);
+                lc.attrs = &at;
+                lc.numAttrs = 1;
+                int nc = 0;
+                if (cudaOccupancyMaxActiveClusters(&nc, k_pcg_cluster, &lc) == cudaSuccess && nc > 0) most = k;
+            }
+        }
+        cudaGetLastError();
+        dev_of = dev;
+    }
+    if (ctas <= most) p.ctas = ctas;
+    return p;
+}
+
 // Whether this system can be solved resident: at most one block per SM and every
 // block's matrix rows in its shared memory.  Asked once per system (one small
 // kernel and a read of its result); allocates what the solve keeps.
@@ -3267,6 +3319,24 @@ fvgb_status launch(SolverCache* c, double* x, const fvgb_solver_cfg* cfg, fvgb_s
         const double* b = c->ls->rhs;
         int nvb = c->nb;
         const bool mixed = cfg->precision == FVGB_PREC_MIXED_IR;
+        const ClusterPlan cl = mixed ? ClusterPlan{} : cluster_plan(c);
+        if (cl.ctas) {
+            cudaLaunchConfig_t lc{};
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = (unsigned)cl.ctas;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            lc.gridDim = dim3((unsigned)cl.ctas);
+            lc.blockDim = dim3((unsigned)cl.threads);
+            lc.dynamicSmemBytes = cl.smem;
+            lc.stream = s;
+            lc.attrs = &at;
+            lc.numAttrs = 1;
+            FVGB_CUDA_TRY(cudaLaunchKernelEx(&lc, k_pcg_cluster, L, m, val, b, cl.units));
+            k_finish<<<grid_for(c->ncases, 128), 128, 0, s>>>(c->L);
+            FVGB_LAUNCH_CHECK("fvgb_solve: finish");
+            return FVGB_OK;
+        }
         const int pg = persistent_grid(c, mixed);
         const int grid = nvb < pg ? nvb : pg;
         FVGB_CUDA_TRY(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), s));

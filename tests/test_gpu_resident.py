@@ -51,6 +51,8 @@ def system(dims, shuffled=False, two_d=False, dt=0.05):
 
 
 DIMS = [
+    ((5, 5, 5), False, False), ((16, 8, 1), False, True), ((127, 1, 1), False, False), ((129, 1, 1), False, False),
+    ((16, 16, 8), False, False), ((13, 13, 13), True, False), ((64, 64, 1), False, True), ((17, 241, 1), False, True),
     ((1, 1, 1), False, False), ((7, 3, 1), False, False), ((11, 31, 3), False, False), ((32, 32, 1), False, True),
     ((25, 41, 1), False, True), ((19, 23, 29), False, False), ((17, 17, 17), True, False),
     ((47, 41, 17), False, False), ((32, 32, 32), False, False), ((36, 34, 31), True, False),
