@@ -38,9 +38,9 @@
 // r (k_init, k_update), a coarse level's by the restriction that produces its
 // right-hand side; the residual is one gather per slot (k_resid); level 0
 // adds the coarse correction (k_prolong) before its second sweep (k_post),
-// coarser levels form it inside the sweep (k_post_fused); the coarsest level
-// runs in one block (k_tail, which can take more levels: kTailRows).  Coarse
-// levels are sliced ELL like the system matrix.
+// coarser levels form it inside the sweep (k_post_fused); the small levels and the
+// coarsest one's dense solve run in one cluster (k_tail).  Coarse levels are sliced
+// ELL like the system matrix.
 //
 // A solve is one CUDA graph (init, a device-side while loop over the CG
 // iteration with the V-cycle inside, or over the multigrid iteration, bounded
@@ -67,7 +67,9 @@ constexpr int kMaxLevels = 25;
 constexpr double kOmega = 0.9;
 constexpr int kPgmRounds = 15;
 constexpr double kPgmLeftRatio = 0.05;
-constexpr int kTailRows = 0;  // levels this small run in the single-block tail (0: the coarsest only)
+constexpr int kTailThreads = 1024;
+constexpr int kFusedPostRows = 1 << 19;  // level 0's coarse correction inside its last sweep up to here
+constexpr int kTailSmem = 200 * 1024;  // the levels whose parts fit this together run in the tail
 
 struct HostCsr {
     int n = 0;
@@ -289,6 +291,8 @@ struct Level {
     double *val = nullptr, *dinv = nullptr;
     int* agg = nullptr;                    // [n], when a coarser level follows
     int *mptr = nullptr, *mem = nullptr;   // members of the next level's rows
+    int* blk = nullptr;                    // first coarse row of every block of k_resid_restrict (null: an aggregate exceeds a block)
+    int nblk = 0;
     int *gptr = nullptr, *gsrc = nullptr;  // sums forming the next level's values
     int* gdst = nullptr;                   // the next level's slot of each sum
     int nnz_next = 0;
@@ -319,6 +323,7 @@ template <> float* Level::rs<float>() const { return rf; }
 
 template <class T>
 struct TailLevelT;
+struct TailPart;
 
 }  // namespace
 
@@ -330,7 +335,15 @@ struct AmgCache {
     double* ainv = nullptr;  // [nc*nc] inverse of the coarsest matrix
     double *r = nullptr, *p = nullptr, *q = nullptr, *z = nullptr, *part = nullptr;
     AmgState* st = nullptr;
-    int tail_from = 1;             // first level run by the single-block tail
+    int cluster = 1;               // blocks of the tail's cluster
+    size_t tail_smem = 0;          // shared memory of the largest of them
+    TailPart* tail_parts = nullptr;  // [cluster][levels of the tail]
+    struct TailIdx {
+        int per = 0;
+        int *col = nullptr, *acol = nullptr, *agg = nullptr, *mem = nullptr, *mptr = nullptr;
+    };
+    std::vector<TailIdx> tail_idx;  // encoded columns of the tail's levels
+    int tail_from = 1;             // first level run by the tail
     TailLevelT<double>* tail = nullptr;    // device descriptors of levels tail_from..L-1
     cudaGraphExec_t graph = nullptr;
     // the FP32 V-cycle of mixed-precision solves
@@ -361,34 +374,55 @@ cudaError_t upload(AmgCache* c, T** p, const std::vector<T>& h) {
 }
 
 // ------------------------------------------------------------ row access
-// Row i of a sliced-ELL matrix with values of type V: f(column, value) for
-// every slot, the column and value loads of the first slots issued before the
-// caller's gathers.
+__device__ __forceinline__ double fmaT(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fmaT(float a, float b, float c) { return fmaf(a, b, c); }
+
+// Row i of a sliced-ELL matrix with values of type V: sum(i, get) = the fma chain
+// over its slots, in slot order from +0, of value * get(column).  Up to 8 slots at a
+// time: their column, value and gathered loads are under way together (index array
+// chosen once per row), the fmas then run only over the row's own slots (a row's width
+// is its slice's, so the branch is the warp's; predicated fmas would all be issued).
+template <class V, class G>
+__device__ __forceinline__ V chain8(int m, const int* col, const V* a, V s, G get) {
+    V x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = k < m ? get(col[k]) : V(0);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (k >= m) break;
+        s = fmaT(a[k], x[k], s);
+    }
+    return s;
+}
+
 template <class V>
 struct EllRowsT {  // level 0: the system's sliced-ELL matrix (or its FP32 copy)
     MeshView m;
     const V* val;
-    template <class F>
-    __device__ __forceinline__ void each(int i, F f) const {
+    template <class G>
+    __device__ __forceinline__ V sum(int i, G get) const {
         const int slice = i >> 5;
         const int b0 = __ldg(&m.m_ptr[slice]);
         const int base = b0 + (i & 31);
         const int w = (__ldg(&m.m_ptr[slice + 1]) - b0) >> 5;
-        int col[8];
-        V a[8];
+        V s = V(0);
+#pragma unroll 1
+        for (int k0 = 0; k0 < w; k0 += 8) {
+            const int at = base + 32 * k0, left = w - k0;
+            int col[8];
+            V a[8];
+            if (m.m_off) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            col[k] = i;
-            a[k] = V(0);
-            if (k < w) {
-                col[k] = slot_col(m, base + k * 32, i);
-                a[k] = __ldg(&val[base + k * 32]);
+                for (int k = 0; k < 8; ++k) col[k] = k < left ? i + (int)__ldg(&m.m_off[at + k * 32]) : i;
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) col[k] = k < left ? __ldg(&m.m_col[at + k * 32]) : i;
             }
-        }
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < w) f(col[k], a[k]);
-        for (int k = 8; k < w; ++k) f(slot_col(m, base + k * 32, i), __ldg(&val[base + k * 32]));
+            for (int k = 0; k < 8; ++k) a[k] = k < left ? __ldg(&val[at + k * 32]) : V(0);
+            s = chain8(left, col, a, s, get);
+        }
+        return s;
     }
 };
 
@@ -397,48 +431,51 @@ struct SellRowsT {  // levels >= 1
     const int* ptr;
     const int* col;
     const V* val;
-    template <class F>
-    __device__ __forceinline__ void each(int i, F f) const {
+    template <class G>
+    __device__ __forceinline__ V sum(int i, G get) const {
         const int slice = i >> 5;
         const int b0 = __ldg(&ptr[slice]);
         const int base = b0 + (i & 31);
         const int w = (__ldg(&ptr[slice + 1]) - b0) >> 5;
-        constexpr int P = 16;  // coarse rows hold up to ~20 entries
-        int c[P];
-        V a[P];
+        V s = V(0);
+#pragma unroll 1
+        for (int k0 = 0; k0 < w; k0 += 8) {
+            const int at = base + 32 * k0, left = w - k0;
+            int c[8];
+            V a[8];
 #pragma unroll
-        for (int k = 0; k < P; ++k) {
-            c[k] = i;
-            a[k] = V(0);
-            if (k < w) {
-                c[k] = __ldg(&col[base + k * 32]);
-                a[k] = __ldg(&val[base + k * 32]);
-            }
+            for (int k = 0; k < 8; ++k) c[k] = k < left ? __ldg(&col[at + k * 32]) : i;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) a[k] = k < left ? __ldg(&val[at + k * 32]) : V(0);
+            s = chain8(left, c, a, s, get);
         }
-#pragma unroll
-        for (int k = 0; k < P; ++k)
-            if (k < w) f(c[k], a[k]);
-        for (int k = P; k < w; ++k) f(__ldg(&col[base + k * 32]), __ldg(&val[base + k * 32]));
+        return s;
     }
 };
 
 using EllRows = EllRowsT<double>;
 using SellRows = SellRowsT<double>;
 
-__device__ __forceinline__ double fmaT(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float fmaT(float a, float b, float c) { return fmaf(a, b, c); }
-
 // ------------------------------------------------------------ reductions
+// (sm[t] += sm[t + s] for s = 128, 64, ..., 1.)  The seven serial additions of the end
+// run in one warp, a different one from block to block: a DADD occupies its scheduler
+// for 64 clocks, and the blocks of an SM end together.
 __device__ __forceinline__ double block_sum(double v, double* sm) {
-    sm[threadIdx.x] = v;
+    __shared__ double out;
+    const int t = threadIdx.x, lane = t & 31;
+    sm[t] = v;
     __syncthreads();
-    for (int s = kT / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) sm[threadIdx.x] += sm[threadIdx.x + s];
-        __syncthreads();
+    if ((t >> 5) == (int)(blockIdx.x & 7)) {
+        double q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = sm[lane + 32 * k] + sm[lane + 32 * k + 128];
+        double r = (q[0] + q[2]) + (q[1] + q[3]);
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) r += __shfl_down_sync(0xffffffffu, r, s);
+        if (lane == 0) out = r;
     }
-    const double r = sm[0];
     __syncthreads();
-    return r;
+    return out;
 }
 
 // Block partial into part[blockIdx.x]; true in the last block to arrive, which
@@ -460,7 +497,10 @@ __device__ __forceinline__ bool arrive(AmgState* st, double* part, double partia
     return true;
 }
 
-__device__ __forceinline__ volatile const int32_t& done_flag(const AmgState* st) { return st->done; }
+// The solve's end, set by an earlier kernel (or by the last block of this one, when
+// every block has read it): a plain load, one request per SM.  A volatile one goes to
+// L2 from every warp, 8,192 times to one address with 1,024 blocks: 2.2 us a kernel.
+__device__ __forceinline__ int done_flag(const AmgState* st) { return st->done; }
 
 // ------------------------------------------------------------ numeric setup
 __global__ void __launch_bounds__(kT) k_dinv_ell(MeshView m, const double* __restrict__ val, double* __restrict__ dinv) {
@@ -489,7 +529,10 @@ __global__ void __launch_bounds__(kT) k_dense(int n, SellRows rows, double* __re
     const int i = blockIdx.x;
     for (int j = threadIdx.x; j < n; j += kT) a[(size_t)i * n + j] = 0.0;
     __syncthreads();
-    if (threadIdx.x == 0) rows.each(i, [&](int j, double v) { a[(size_t)i * n + j] += v; });
+    if (threadIdx.x == 0) {
+        const int b0 = __ldg(&rows.ptr[i >> 5]), b1 = __ldg(&rows.ptr[(i >> 5) + 1]);
+        for (int pos = b0 + (i & 31); pos < b1; pos += 32) a[(size_t)i * n + __ldg(&rows.col[pos])] += __ldg(&rows.val[pos]);
+    }
 }
 
 // In-place Gauss-Jordan inverse of an n x n SPD matrix, one block of 1024 threads.
@@ -507,10 +550,67 @@ __global__ void __launch_bounds__(1024) k_gauss_jordan(int n, double* __restrict
             const int i = t / n, j = t - i * n;
             if (i == k) continue;
             const double akj = a[(size_t)k * n + j];
-            a[(size_t)i * n + j] = (j == k ? 0.0 : a[(size_t)i * n + j]) - f[i] * akj;
+            a[(size_t)i * n + j] = fma(-f[i], akj, j == k ? 0.0 : a[(size_t)i * n + j]);
         }
         __syncthreads();
     }
+}
+
+// Every thread of the cluster has its stores so far seen by every other (cluster scope).
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The same inverse, the rows dealt over one cluster's blocks (row i to block i mod C)
+// and held in their shared memory: one block's FP64 pipe needs 16 clocks per warp-wide
+// update, 2.4 ms for 221 rows (n^3 / 2 clocks); 16 of them and one cluster barrier per
+// step bring the 221-row inverse from 3.7 ms to 0.4.  Same operations on every entry
+// in the same order, so the same bits.
+constexpr int kGjThreads = 512;
+__host__ __device__ inline size_t gj_smem(int n, int C) { return 8 * ((size_t)((n + C - 1) / C) * (n + 1) + 2 * (size_t)n); }
+
+__global__ void __launch_bounds__(kGjThreads) k_gauss_jordan_cluster(int n, double* __restrict__ a) {
+    extern __shared__ double sm[];  // [R][n] own rows, [2][n] scaled pivot rows, [R] column k
+    const int C = (int)gridDim.x, rank = (int)blockIdx.x, R = (n + C - 1) / C, own = (n - rank + C - 1) / C;
+    const int tx = threadIdx.x & 255, ty = threadIdx.x >> 8;
+    double* prow = sm + (size_t)R * n;
+    double* f = prow + 2 * (size_t)n;
+    for (int l = ty; l < own; l += kGjThreads / 256)
+        for (int j = tx; j < n; j += 256) sm[(size_t)l * n + j] = a[(size_t)(l * C + rank) * n + j];
+    cluster_barrier();  // also: every block runs before its shared memory is written
+    for (int k = 0; k < n; ++k) {
+        double* cur = prow + (k & 1) * (size_t)n;
+        if (rank == k % C) {
+            double* row = sm + (size_t)(k / C) * n;
+            const double piv = row[k];
+            __syncthreads();
+            const double ip = 1.0 / piv;
+            for (int j = threadIdx.x; j < n; j += kGjThreads) {
+                const double v = (j == k ? 1.0 : row[j]) * ip;
+                row[j] = v;
+                const unsigned at = (unsigned)__cvta_generic_to_shared(&cur[j]);
+                for (int q = 0; q < C; ++q) {
+                    unsigned ra;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(at), "r"(q));
+                    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(v) : "memory");
+                }
+            }
+        }
+        for (int l = threadIdx.x; l < own; l += kGjThreads) f[l] = sm[(size_t)l * n + k];
+        cluster_barrier();
+        for (int l = ty; l < own; l += kGjThreads / 256) {
+            if (l * C + rank == k) continue;
+            const double fl = f[l];
+            for (int j = tx; j < n; j += 256) {
+                double* e = sm + (size_t)l * n + j;
+                *e = fma(-fl, cur[j], j == k ? 0.0 : *e);
+            }
+        }
+        __syncthreads();
+    }
+    for (int l = ty; l < own; l += kGjThreads / 256)
+        for (int j = tx; j < n; j += 256) a[(size_t)(l * C + rank) * n + j] = sm[(size_t)l * n + j];
+    cluster_barrier();  // no block leaves while another may write its shared memory
 }
 
 // ------------------------------------------------------------ V-cycle
@@ -533,8 +633,7 @@ __global__ void __launch_bounds__(kT)
     if (done_flag(st)) return;
     const int i = blockIdx.x * kT + threadIdx.x;
     if (i >= n) return;
-    T s = T(0);
-    rows.each(i, [&](int j, T a) { s = fmaT(a, __ldg(&x[j]), s); });
+    const T s = rows.sum(i, [&](int j) { return __ldg(&x[j]); });
     r[i] = __ldg(&b[i]) - s;
 }
 
@@ -553,66 +652,245 @@ __global__ void __launch_bounds__(kT)
     xc[c] = T(kOmega) * __ldg(&dinv_c[c]) * s;
 }
 
-// The small levels t..L-1 of a V-cycle in one block of 1024 threads: their
-// kernels would each be a few blocks that wait on latency, so one block runs
-// the same steps with barriers between them.  Level t's b and x (its
-// pre-smoothing sweep) come from the restriction above it; its xo is the
-// correction handed back up.
+// Both in one kernel: a block takes whole aggregates of at most kT rows together
+// (coarse rows [blk[b], blk[b+1])), a thread per fine row in the aggregates' order; the
+// coarse rows then sum their members' residuals from shared memory, in the same order
+// as k_restrict.  One launch and the residual's way through memory less.
+template <class R, class T>
+__global__ void __launch_bounds__(kT)
+    k_resid_restrict(const AmgState* st, R rows, const int* __restrict__ blk, const T* __restrict__ b,
+                     const T* __restrict__ x, const int* __restrict__ mptr, const int* __restrict__ mem,
+                     const T* __restrict__ dinv_c, T* __restrict__ bc, T* __restrict__ xc) {
+    __shared__ T sm[kT];
+    const int done = done_flag(st);
+    const int c0 = __ldg(&blk[blockIdx.x]), c1 = __ldg(&blk[blockIdx.x + 1]);
+    const int m0 = __ldg(&mptr[c0]), m1 = __ldg(&mptr[c1]), t = threadIdx.x;
+    if (done) return;
+    if (m0 + t < m1) {
+        const int i = __ldg(&mem[m0 + t]);
+        const T s = rows.sum(i, [&](int j) { return __ldg(&x[j]); });
+        sm[t] = __ldg(&b[i]) - s;
+    }
+    __syncthreads();
+    const int c = c0 + t;
+    if (c >= c1) return;
+    const int k1 = __ldg(&mptr[c + 1]) - m0;
+    T s = T(0);
+    for (int k = __ldg(&mptr[c]) - m0; k < k1; ++k) s += sm[k];
+    bc[c] = s;
+    xc[c] = T(kOmega) * __ldg(&dinv_c[c]) * s;
+}
+
+// The small levels t..L-1 of a V-cycle in one thread-block cluster: each step (a
+// residual, a restriction, a sweep) as a kernel of its own costs a launch and a chain
+// of waits on L2 (slice, slots, gathered vector, coarse correction) for almost no
+// work: 6.6 us apiece in the solve's graph.  Here a block owns a range of slices of
+// every level, copies their slots, columns, aggregates and members to shared memory
+// at once, and keeps its part of the levels' vectors there; a gather reads the owner's
+// shared memory.  A step is then one such read, a row's chain of fmas and a cluster
+// barrier.  (With the vectors in global memory a step took 4,000-9,000 clocks, the
+// tail of the 512 x 512 cavity's hierarchy 42 us.)  Level t's b and x (its
+// pre-smoothing sweep) come from the restriction above it; its xo is handed back up.
 template <class T>
 struct TailLevelT {
-    int n;
-    SellRowsT<T> A;
+    int n, per;        // rows; slices per block
+    const T* val;      // [slots]
+    const int* col;    // [slots] owner << 16 | row in the owner's part, of the column
+    const int* acol;   // [slots] the same of the column's aggregate (in the level below)
+    const int* ptr;    // [slices + 1]
+    const int* agg;    // [n] the same of the row's aggregate
+    const int* mem;    // the same of the members of this level's rows (in the level above; levels > t)
+    const int* mptr;   // [n + 1]
     const T* dinv;
-    const int* agg;   // to level l+1
-    const int* mptr;  // members of level l+1's rows
-    const int* mem;
-    T *b, *x, *xo, *r;
+    T *b, *x, *xo;     // level t: global
 };
+// A block's part of one level: its slices, slots and members, and where they lie in
+// shared memory.
+struct TailPart {
+    int s0, s1, pos0, mem0, len, nmem;
+    int o_val, o_col, o_acol, o_ptr, o_mem, o_mptr;  // bytes; of element pos0, s0, mem0, 32 s0
+    int o_x, o_b, o_r, o_xo;                         // vectors, the same offsets in every block
+    int o_inv, o_rhs;  // coarsest level: its rows of the inverse (-1: read in place), the whole right-hand side
+};
+constexpr int kTailRowsMax = 65535;  // rows of a block's part: 16 bits of an encoded column
+inline size_t tail_round(size_t b) { return (b + 15) / 16 * 16; }
+
+// 16-byte pieces of [first, first + bytes) rounded outwards, to shared memory at dst
+// (the piece that holds `first`'s 16-byte line); every thread of the block.
+__device__ __forceinline__ void tail_copy(unsigned char* dst, const void* first, size_t bytes) {
+    const size_t a = (size_t)first & ~(size_t)15, n = ((size_t)first + bytes - a + 15) >> 4;
+    for (size_t k = threadIdx.x; k < n; k += kTailThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst + 16 * k)),
+                     "l"(a + 16 * k)
+                     : "memory");
+}
+// element e of a vector kept at `base` in its owner's shared memory
+template <class T>
+__device__ __forceinline__ T tail_get(const T* base, int e, int rank) {
+    const int q = e >> 16;
+    if (q == rank) return base[e & 0xffff];
+    unsigned ra;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"((unsigned)__cvta_generic_to_shared(base + (e & 0xffff))), "r"(q));
+    T v;
+    if constexpr (sizeof(T) == 8) asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(ra) : "memory");
+    else asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
+    return v;
+}
 
 template <class T>
-__global__ void __launch_bounds__(1024)
-    k_tail(const AmgState* st, const TailLevelT<T>* __restrict__ lv, int nl, const T* __restrict__ ainv) {
-    if (done_flag(st)) return;
-    const int Tt = threadIdx.x, NT = blockDim.x;
+__global__ void __launch_bounds__(kTailThreads)
+    k_tail(const AmgState* st, const TailLevelT<T>* __restrict__ lv, const TailPart* __restrict__ parts, int nl,
+           const T* __restrict__ ainv) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ TailPart part[kMaxLevels];
+    __shared__ TailLevelT<T> lev[kMaxLevels];
+    const int done = done_flag(st);  // the same in every block: only other kernels write it
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = kTailThreads / 32, rank = (int)blockIdx.x;
+    for (int k = t; k < (int)(nl * sizeof(TailPart) / 4); k += kTailThreads)
+        ((int*)part)[k] = __ldg((const int*)(parts + (size_t)rank * nl) + k);
+    for (int k = t; k < (int)(nl * sizeof(TailLevelT<T>) / 4); k += kTailThreads)
+        ((int*)lev)[k] = __ldg((const int*)lv + k);
+    __syncthreads();
+    if (done) return;
+    for (int l = 0; l < nl; ++l) {
+        const TailLevelT<T>& F = lev[l];
+        const TailPart& P = part[l];
+        const int rows = min(F.n, P.s1 * 32) - P.s0 * 32;
+        if (rows <= 0) continue;
+        if (l + 1 < nl) {
+            tail_copy(dyn + (P.o_val & ~15), F.val + P.pos0, sizeof(T) * (size_t)P.len);
+            tail_copy(dyn + (P.o_col & ~15), F.col + P.pos0, 4 * (size_t)P.len);
+            tail_copy(dyn + (P.o_acol & ~15), F.acol + P.pos0, 4 * (size_t)P.len);
+            tail_copy(dyn + (P.o_ptr & ~15), F.ptr + P.s0, 4 * (size_t)(P.s1 - P.s0 + 1));
+        } else if (P.o_inv >= 0) {
+            tail_copy(dyn + P.o_inv, ainv + (size_t)P.s0 * 32 * F.n, sizeof(T) * (size_t)rows * F.n);
+        }
+        if (l > 0) {
+            tail_copy(dyn + (P.o_mem & ~15), F.mem + P.mem0, 4 * (size_t)P.nmem);
+            tail_copy(dyn + (P.o_mptr & ~15), F.mptr + P.s0 * 32, 4 * (size_t)(rows + 1));
+        }
+    }
+    {
+        const TailLevelT<T>& F = lev[0];
+        const TailPart& P = part[0];
+        for (int q = t; q < (P.s1 - P.s0) * 32; q += kTailThreads) {
+            const int i = min(F.n - 1, P.s0 * 32 + q);
+            ((T*)(dyn + P.o_x))[q] = __ldcg(&F.x[i]);
+            ((T*)(dyn + P.o_b))[q] = __ldcg(&F.b[i]);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    cluster_barrier();
+    constexpr int G = 8;  // gathers under way per thread
     for (int l = 0; l + 1 < nl; ++l) {  // down
-        const TailLevelT<T>& F = lv[l];
-        const TailLevelT<T>& C = lv[l + 1];
-        for (int i = Tt; i < F.n; i += NT) {
-            T s = T(0);
-            F.A.each(i, [&](int j, T a) { s = fmaT(a, F.x[j], s); });
-            F.r[i] = F.b[i] - s;
+        {
+            const TailPart P = part[l];
+            const int n = lev[l].n;
+            const T *val = (const T*)(dyn + P.o_val), *x = (const T*)(dyn + P.o_x), *b = (const T*)(dyn + P.o_b);
+            T* r = (T*)(dyn + P.o_r);
+            const int *col = (const int*)(dyn + P.o_col), *ptr = (const int*)(dyn + P.o_ptr);
+            for (int sl = wid; sl < P.s1 - P.s0; sl += nw) {
+                const int q = sl * 32 + lane, base = ptr[sl] - P.pos0 + lane, w = (ptr[sl + 1] - ptr[sl]) >> 5;
+                if (P.s0 * 32 + q >= n) continue;
+                T s = T(0);
+                for (int k0 = 0; k0 < w; k0 += G) {
+                    T v[G];
+#pragma unroll
+                    for (int k = 0; k < G; ++k) v[k] = tail_get(x, col[base + 32 * min(k0 + k, w - 1)], rank);
+#pragma unroll
+                    for (int k = 0; k < G; ++k) {
+                        if (k0 + k >= w) break;
+                        s = fmaT(val[base + 32 * (k0 + k)], v[k], s);
+                    }
+                }
+                r[q] = b[q] - s;
+            }
         }
-        __syncthreads();
-        for (int c = Tt; c < C.n; c += NT) {
-            T s = T(0);
-            for (int k = F.mptr[c]; k < F.mptr[c + 1]; ++k) s += F.r[F.mem[k]];
-            C.b[c] = s;
-            C.x[c] = T(kOmega) * C.dinv[c] * s;
+        cluster_barrier();
+        {
+            const TailPart P = part[l + 1];
+            const TailLevelT<T>& K = lev[l + 1];
+            const T* r = (const T*)(dyn + part[l].o_r);
+            T *kb = (T*)(dyn + P.o_b), *kx = (T*)(dyn + P.o_x);
+            const int *mem = (const int*)(dyn + P.o_mem), *mptr = (const int*)(dyn + P.o_mptr);
+            for (int q = t; q < (P.s1 - P.s0) * 32; q += kTailThreads) {
+                if (P.s0 * 32 + q >= K.n) continue;
+                const T dc = __ldg(&K.dinv[P.s0 * 32 + q]);
+                const int m1 = mptr[q + 1] - P.mem0;
+                T s = T(0);
+                for (int k0 = mptr[q] - P.mem0; k0 < m1; k0 += G) {
+                    T v[G];
+#pragma unroll
+                    for (int k = 0; k < G; ++k) v[k] = tail_get(r, mem[min(k0 + k, m1 - 1)], rank);
+#pragma unroll
+                    for (int k = 0; k < G; ++k) {
+                        if (k0 + k >= m1) break;
+                        s += v[k];
+                    }
+                }
+                kb[q] = s;
+                kx[q] = T(kOmega) * dc * s;
+            }
         }
-        __syncthreads();
+        cluster_barrier();
     }
     {  // coarsest: xo = A^-1 b, a warp per row
-        const TailLevelT<T>& B = lv[nl - 1];
-        const int lane = Tt & 31;
-        for (int row = Tt >> 5; row < B.n; row += NT >> 5) {
+        const TailPart P = part[nl - 1];
+        const int n = lev[nl - 1].n, per = lev[nl - 1].per * 32;
+        T *xo = (T*)(dyn + P.o_xo), *rhs = (T*)(dyn + P.o_rhs);
+        if (P.s1 > P.s0) {  // the whole right-hand side once
+            for (int q = 0; q * per < n; ++q)
+                for (int k = t; k < min(per, n - q * per); k += kTailThreads)
+                    rhs[q * per + k] = tail_get((const T*)(dyn + P.o_b), q << 16 | k, rank);
+            __syncthreads();
+        }
+        for (int row = P.s0 * 32 + wid; row < min(n, P.s1 * 32); row += nw) {
+            const T* inv = P.o_inv >= 0 ? (const T*)(dyn + P.o_inv) + (size_t)(row - P.s0 * 32) * n : ainv + (size_t)row * n;
             T s = T(0);
-            for (int j = lane; j < B.n; j += 32) s = fmaT(__ldg(&ainv[(size_t)row * B.n + j]), B.b[j], s);
+#pragma unroll 4
+            for (int j = lane; j < n; j += 32) s = fmaT(inv[j], rhs[j], s);
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) B.xo[row] = s;
+            if (lane == 0) xo[row - P.s0 * 32] = s;
         }
-        __syncthreads();
+        cluster_barrier();
     }
-    for (int l = nl - 2; l >= 0; --l) {  // up
-        const TailLevelT<T>& F = lv[l];
-        const TailLevelT<T>& C = lv[l + 1];
-        for (int i = Tt; i < F.n; i += NT) F.r[i] = F.x[i] + C.xo[F.agg[i]];
-        __syncthreads();
-        for (int i = Tt; i < F.n; i += NT) {
+    for (int l = nl - 2; l >= 0; --l) {  // up: y = x + P xc formed inside the sweep
+        const TailLevelT<T>& F = lev[l];
+        const TailPart P = part[l];
+        const T *val = (const T*)(dyn + P.o_val), *x = (const T*)(dyn + P.o_x), *b = (const T*)(dyn + P.o_b);
+        const T* xc = (const T*)(dyn + part[l + 1].o_xo);
+        T* xo = (T*)(dyn + P.o_xo);
+        const int *col = (const int*)(dyn + P.o_col), *acol = (const int*)(dyn + P.o_acol), *ptr = (const int*)(dyn + P.o_ptr);
+        for (int sl = wid; sl < P.s1 - P.s0; sl += nw) {
+            const int q = sl * 32 + lane, i = P.s0 * 32 + q, base = ptr[sl] - P.pos0 + lane, w = (ptr[sl + 1] - ptr[sl]) >> 5;
+            if (i >= F.n) continue;
+            const T di = __ldg(&F.dinv[i]);
+            const T yi = x[q] + tail_get(xc, __ldg(&F.agg[i]), rank);
             T s = T(0);
-            F.A.each(i, [&](int j, T a) { s = fmaT(a, F.r[j], s); });
-            F.xo[i] = fmaT(T(kOmega) * F.dinv[i], F.b[i] - s, F.r[i]);
+            for (int k0 = 0; k0 < w; k0 += G) {
+                T v[G], u[G];
+#pragma unroll
+                for (int k = 0; k < G; ++k) {
+                    const int at = base + 32 * min(k0 + k, w - 1);
+                    u[k] = tail_get(xc, acol[at], rank);
+                    v[k] = tail_get(x, col[at], rank);
+                }
+#pragma unroll
+                for (int k = 0; k < G; ++k) {
+                    if (k0 + k >= w) break;
+                    s = fmaT(val[base + 32 * (k0 + k)], v[k] + u[k], s);
+                }
+            }
+            const T out = fmaT(T(kOmega) * di, b[q] - s, yi);
+            xo[q] = out;
+            if (l == 0) F.xo[i] = out;
         }
-        __syncthreads();
+        cluster_barrier();  // (the last: no block leaves while another may read its shared memory)
+    }
+    if (nl == 1) {  // the coarsest level alone
+        const TailPart P = part[0];
+        for (int q = t; q < (P.s1 - P.s0) * 32; q += kTailThreads)
+            if (P.s0 * 32 + q < lev[0].n) lev[0].xo[P.s0 * 32 + q] = ((const T*)(dyn + P.o_xo))[q];
     }
 }
 
@@ -636,8 +914,7 @@ __global__ void __launch_bounds__(kT)
     const int i = blockIdx.x * kT + threadIdx.x;
     if (i >= n) return;
     const T yi = __ldg(&x[i]) + __ldg(&xc[__ldg(&agg[i])]);
-    T s = T(0);
-    rows.each(i, [&](int j, T a) { s = fmaT(a, __ldg(&x[j]) + __ldg(&xc[__ldg(&agg[j])]), s); });
+    const T s = rows.sum(i, [&](int j) { return __ldg(&x[j]) + __ldg(&xc[__ldg(&agg[j])]); });
     out[i] = fmaT(T(kOmega) * __ldg(&dinv[i]), __ldg(&b[i]) - s, yi);
 }
 
@@ -650,8 +927,7 @@ __global__ void __launch_bounds__(kT)
     if (done_flag(st)) return;
     const int i = blockIdx.x * kT + threadIdx.x;
     if (i >= n) return;
-    T s = T(0);
-    rows.each(i, [&](int j, T a) { s = fmaT(a, __ldg(&y[j]), s); });
+    const T s = rows.sum(i, [&](int j) { return __ldg(&y[j]); });
     const T v = fmaT(T(kOmega) * __ldg(&dinv[i]), __ldg(&b[i]) - s, __ldg(&y[i]));
     if constexpr (std::is_same<T, float>::value && std::is_same<TO, double>::value)
         out[i] = (double)v * st->vinv;
@@ -737,8 +1013,7 @@ __global__ void __launch_bounds__(kT)
     const double* x = st->x;
     double ri = 0.0;
     if (i < n) {
-        double s = 0.0;
-        A.each(i, [&](int j, double a) { s = fma(a, x[j], s); });
+        const double s = A.sum(i, [&](int j) { return x[j]; });
         ri = __ldg(&b[i]) - s;
         r[i] = ri;
         first_sweep(i, ri, dinv0, x0, d0f, b0f, x0f, 1.0);
@@ -789,8 +1064,7 @@ __global__ void __launch_bounds__(kT)
     const int i = blockIdx.x * kT + threadIdx.x;
     double v = 0.0;
     if (i < n) {
-        double s = 0.0;
-        A.each(i, [&](int j, double a) { s = fma(a, __ldg(&p[j]), s); });
+        const double s = A.sum(i, [&](int j) { return __ldg(&p[j]); });
         q[i] = s;
         v = __ldg(&p[i]) * s;
     }
@@ -814,7 +1088,7 @@ __global__ void __launch_bounds__(kT)
     if (done_flag(st)) return;
     const int i = blockIdx.x * kT + threadIdx.x;
     const double alpha = st->alpha;
-    const double sigma = sigma_scale(st->res);  // the previous residual norm (rewritten by the last block below)
+    const double sigma = b0f ? sigma_scale(st->res) : 1.0;  // the previous residual norm (rewritten by the last block below)
     double* x = st->x;
     double v = 0.0;
     if (i < n) {
@@ -842,30 +1116,58 @@ __global__ void __launch_bounds__(kT)
     }
 }
 
-// beta = r.z / rz_old
-__global__ void __launch_bounds__(kT)
-    k_rz(AmgState* st, int n, const double* __restrict__ r, const double* __restrict__ z, double* part) {
-    __shared__ double sm[kT];
-    if (done_flag(st)) return;
-    const int i = blockIdx.x * kT + threadIdx.x;
-    const double v = i < n ? __ldg(&r[i]) * __ldg(&z[i]) : 0.0;
-    double tot;
-    if (arrive(st, part, block_sum(v, sm), sm, &tot) && threadIdx.x == 0) {
-        st->beta = tot / st->rz;
-        st->rz = tot;
-        if (!isfinite(st->beta)) {
-            st->status = FVGB_ERR_BREAKDOWN;
-            st->done = 1;
-        }
-    }
-}
-
 // p = z + beta p
 __global__ void __launch_bounds__(kT)
     k_dir(const AmgState* st, int n, const double* __restrict__ z, double* __restrict__ p) {
     if (done_flag(st)) return;
     const int i = blockIdx.x * kT + threadIdx.x;
     if (i < n) p[i] = fma(st->beta, p[i], __ldg(&z[i]));
+}
+
+// Level 0's last sweep of the V-cycle inside the CG, z = y + w D^-1 (b - A y), with the
+// CG's next step: beta = r.z / rz_old (k_rz, the same blocks and sums) and the loop's
+// condition.  FUSED: y = x + P xc formed inside the sweep (as k_post_fused: systems
+// whose working set stays in L2 gain the launch, larger ones lose the extra traffic).
+template <class R, class T, bool FUSED>
+__global__ void __launch_bounds__(kT)
+    k_post_rz(AmgState* st, R rows, int n, const T* __restrict__ dinv, const T* __restrict__ b, const T* __restrict__ y,
+              const T* __restrict__ xc, const int* __restrict__ agg, double* __restrict__ z,
+              const double* __restrict__ r, double* part, cudaGraphConditionalHandle h) {
+    __shared__ double sm[kT];
+    const int done = done_flag(st);
+    const int i = blockIdx.x * kT + threadIdx.x;
+    if (done) {
+        if (i == 0) cudaGraphSetConditional(h, 0u);
+        return;
+    }
+    double v = 0.0;
+    if (i < n) {
+        T s = T(0);
+        T yi = __ldg(&y[i]);
+        if (FUSED) {
+            yi = yi + __ldg(&xc[__ldg(&agg[i])]);
+            s = rows.sum(i, [&](int j) { return __ldg(&y[j]) + __ldg(&xc[__ldg(&agg[j])]); });
+        } else {
+            s = rows.sum(i, [&](int j) { return __ldg(&y[j]); });
+        }
+        const T o = fmaT(T(kOmega) * __ldg(&dinv[i]), __ldg(&b[i]) - s, yi);
+        double zi;
+        if constexpr (std::is_same<T, float>::value) zi = (double)o * st->vinv;
+        else zi = o;
+        z[i] = zi;
+        v = __ldg(&r[i]) * zi;
+    }
+    double tot;
+    if (arrive(st, part, block_sum(v, sm), sm, &tot) && threadIdx.x == 0) {
+        const double beta = tot / st->rz;
+        st->beta = beta;
+        st->rz = tot;
+        if (!isfinite(beta)) {
+            st->status = FVGB_ERR_BREAKDOWN;
+            st->done = 1;
+        }
+        cudaGraphSetConditional(h, st->done ? 0u : 1u);
+    }
 }
 
 // ------------------------------------------------------------ standalone multigrid
@@ -890,12 +1192,11 @@ __global__ void __launch_bounds__(kT)
     __shared__ double sm[kT];
     if (done_flag(st)) return;
     const int i = blockIdx.x * kT + threadIdx.x;
-    const double sigma = sigma_scale(st->res);  // the previous residual norm (rewritten by the last block below)
+    const double sigma = b0f ? sigma_scale(st->res) : 1.0;  // the previous residual norm (rewritten by the last block below)
     const double* x = st->x;
     double ri = 0.0;
     if (i < n) {
-        double s = 0.0;
-        A.each(i, [&](int j, double a) { s = fma(a, x[j], s); });
+        const double s = A.sum(i, [&](int j) { return x[j]; });
         ri = __ldg(&b[i]) - s;
         r[i] = ri;
         first_sweep(i, ri, dinv0, x0, d0f, b0f, x0f, sigma);
@@ -934,6 +1235,158 @@ __global__ void k_stats(AmgState* st) {
 }
 
 // ------------------------------------------------------------ host side
+template <class T>
+std::vector<TailLevelT<T>> tail_levels(const AmgCache* c) {
+    std::vector<TailLevelT<T>> tl;
+    for (int l = c->tail_from; l < (int)c->lv.size(); ++l) {
+        const Level& V = c->lv[l];
+        const auto& E = c->tail_idx[l - c->tail_from];
+        tl.push_back(TailLevelT<T>{V.n, E.per, V.vals<T>(), E.col, E.acol, V.sptr, E.agg, E.mem, E.mptr, V.dinvs<T>(),
+                                   V.bs<T>(), V.xs<T>(), V.xos<T>()});
+    }
+    return tl;
+}
+
+cudaLaunchAttribute cluster_attr(int C) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    return at;
+}
+
+// The largest cluster (16, 8, ... blocks) the device runs k_tail and
+// k_gauss_jordan_cluster with.
+constexpr size_t kGjMaxSmem = 200 * 1024;
+int cluster_size() {
+    const void* fns[3] = {(const void*)k_tail<double>, (const void*)k_tail<float>, (const void*)k_gauss_jordan_cluster};
+    int best = 16;
+    for (const void* fn : fns) {
+        const bool gj = fn == (const void*)k_gauss_jordan_cluster;
+        const size_t smem = gj ? kGjMaxSmem : (size_t)kTailSmem;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) best = std::min(best, 8);
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) best = 1;
+        for (; best > 1; best /= 2) {
+            cudaLaunchConfig_t lc{};
+            cudaLaunchAttribute at = cluster_attr(best);
+            lc.gridDim = dim3((unsigned)best);
+            lc.blockDim = dim3(gj ? kGjThreads : kTailThreads);
+            lc.dynamicSmemBytes = smem;
+            lc.attrs = &at;
+            lc.numAttrs = 1;
+            int nc = 0;
+            if (cudaOccupancyMaxActiveClusters(&nc, fn, &lc) == cudaSuccess && nc > 0) break;
+        }
+    }
+    cudaGetLastError();
+    return best;
+}
+
+// Picks the levels of the one-cluster tail (from the coarsest up, as long as every
+// block's part fits its shared memory with FP64 values), lays the parts out and
+// uploads the encoded columns.
+fvgb_status tail_setup(AmgCache* c, const std::vector<std::vector<int>>& h_sptr, const std::vector<std::vector<int>>& h_scol,
+                       const std::vector<std::vector<int>>& h_agg, const std::vector<std::vector<int>>& h_mptr,
+                       const std::vector<std::vector<int>>& h_mem) {
+    const int L = (int)c->lv.size(), C = c->cluster = cluster_size();
+    std::vector<int> per(L), ns(L);
+    for (int l = 0; l < L; ++l) {
+        ns[l] = (c->lv[l].n + 31) / 32;
+        per[l] = (ns[l] + C - 1) / C;
+    }
+    auto s0 = [&](int l, int r) { return std::min(ns[l], r * per[l]); };
+    bool inv_in_smem = true;
+    // layout of levels t.. for every block; the vectors first, at the same offsets
+    auto layout = [&](int t, std::vector<TailPart>& parts) {
+        parts.assign((size_t)C * (L - t), TailPart{});
+        size_t most = 0, o = 0;
+        for (int l = t; l < L; ++l)
+            for (int TailPart::*f : {&TailPart::o_x, &TailPart::o_b, &TailPart::o_r, &TailPart::o_xo}) {
+                for (int r = 0; r < C; ++r) parts[(size_t)r * (L - t) + l - t].*f = (int)o;
+                o += tail_round(8 * 32 * (size_t)per[l]);
+            }
+        for (int r = 0; r < C; ++r) {
+            size_t q = o;
+            // an array's copy starts at the 16-byte line of its first element
+            auto put = [&](size_t first, size_t count, size_t size) {
+                const size_t shift = first * size % 16, at = q + shift;
+                q += tail_round(shift + count * size);
+                return (int)at;
+            };
+            for (int l = t; l < L; ++l) {
+                TailPart& P = parts[(size_t)r * (L - t) + l - t];
+                P.s0 = s0(l, r);
+                P.s1 = s0(l, r + 1);
+                const int rows = std::max(0, std::min(c->lv[l].n, P.s1 * 32) - P.s0 * 32);
+                P.pos0 = h_sptr[l][P.s0];
+                const size_t len = l + 1 < L ? h_sptr[l][P.s1] - P.pos0 : 0;
+                P.len = (int)len;
+                P.o_val = put(P.pos0, len, 8);
+                P.o_col = put(P.pos0, len, 4);
+                P.o_acol = put(P.pos0, len, 4);
+                P.o_ptr = put(P.s0, P.s1 - P.s0 + 1, 4);
+                if (l > t) {
+                    const int i0 = std::min(c->lv[l].n, P.s0 * 32);
+                    P.mem0 = h_mptr[l - 1][i0];
+                    P.nmem = h_mptr[l - 1][i0 + rows] - P.mem0;
+                    P.o_mem = put(P.mem0, P.nmem, 4);
+                    P.o_mptr = put(P.s0 * 32, rows + 1, 4);
+                }
+            }
+            TailPart& B = parts[(size_t)r * (L - t) + L - 1 - t];
+            const size_t nc = (size_t)c->lv[L - 1].n, rows = std::max(0, std::min((int)nc, B.s1 * 32) - B.s0 * 32);
+            B.o_rhs = put(0, nc, 8);
+            B.o_inv = inv_in_smem ? put(0, rows * nc, 8) : -1;
+            most = std::max(most, q);
+        }
+        return most;
+    };
+    std::vector<TailPart> parts, next;
+    int t = L - 1;
+    c->tail_smem = layout(t, parts);
+    if (c->tail_smem > (size_t)kTailSmem / 2) {  // a large inverse is read in place
+        inv_in_smem = false;
+        c->tail_smem = layout(t, parts);
+    }
+    while (t > 1 && 32 * per[t - 1] <= kTailRowsMax) {
+        const size_t most = layout(t - 1, next);
+        if (most > (size_t)kTailSmem) break;
+        parts.swap(next);
+        c->tail_smem = most;
+        --t;
+    }
+    if (c->tail_smem > (size_t)kTailSmem) return fvgb_fail(FVGB_ERR_UNSUPPORTED, "multigrid: coarsest level too large");
+    c->tail_from = t;
+    cudaError_t e = upload(c, &c->tail_parts, parts);
+    auto enc = [&](int l, int i) { return i / (32 * per[l]) << 16 | i % (32 * per[l]); };
+    c->tail_idx.resize(L - t);
+    for (int l = t; l < L && e == cudaSuccess; ++l) {
+        auto& E = c->tail_idx[l - t];
+        E.per = per[l];
+        if (l + 1 < L) {
+            std::vector<int> col(h_scol[l]), acol(h_scol[l]), agg(h_agg[l]);
+            for (int& v : acol) v = enc(l + 1, h_agg[l][v]);
+            for (int& v : col) v = enc(l, v);
+            for (int& v : agg) v = enc(l + 1, v);
+            col.resize(col.size() + 8);  // copies run to the end of a 16-byte line
+            acol.resize(acol.size() + 8);
+            e = upload(c, &E.col, col);
+            if (e == cudaSuccess) e = upload(c, &E.acol, acol);
+            if (e == cudaSuccess) e = upload(c, &E.agg, agg);
+        }
+        if (l > t && e == cudaSuccess) {
+            std::vector<int> mem(h_mem[l - 1]), mptr(h_mptr[l - 1]);
+            for (int& v : mem) v = enc(l - 1, v);
+            mem.resize(mem.size() + 8);
+            mptr.resize(mptr.size() + 8);
+            e = upload(c, &E.mem, mem);
+            if (e == cudaSuccess) e = upload(c, &E.mptr, mptr);
+        }
+    }
+    if (e == cudaSuccess) e = upload(c, &c->tail, tail_levels<double>(c));
+    return e == cudaSuccess ? FVGB_OK : cuda_fail(e, "multigrid setup");
+}
+
 fvgb_status symbolic(AmgCache* c, cudaStream_t s) {
     const fvgb_ls* ls = c->ls;
     const fvgb_mesh* mesh = ls->mesh;
@@ -958,6 +1411,7 @@ fvgb_status symbolic(AmgCache* c, cudaStream_t s) {
     c->lv[0].nnz = nnz;
     c->lv[0].slots = mesh->m_len;
     std::vector<int> slot_of = csr_pos;  // the current level's slot of each of its CSR entries
+    std::vector<std::vector<int>> h_sptr(1), h_scol(1), h_agg, h_mptr, h_mem;  // of every level; members: of the next level's rows
     while ((int)c->lv.size() < kMaxLevels && A.n > kCoarseRows) {
         // two rounds of pairwise matching per level (double pairwise): the pairs
         // of the first round are matched again on their Galerkin matrix, so a
@@ -994,6 +1448,22 @@ fvgb_status symbolic(AmgCache* c, cudaStream_t s) {
         if (e == cudaSuccess) e = upload(c, &L.gptr, gptr);
         if (e == cudaSuccess) e = upload(c, &L.gsrc, gsrc);
         if (e != cudaSuccess) return cuda_fail(e, "multigrid setup");
+        {  // whole aggregates to blocks of k_resid_restrict
+            std::vector<int> blk(1, 0);
+            bool fits = true;
+            for (int I = 0, m0 = 0; I < nc; ++I) {
+                fits = fits && mptr[I + 1] - mptr[I] <= kT;
+                if (mptr[I + 1] - m0 > kT || I - blk.back() >= kT) {
+                    blk.push_back(I);
+                    m0 = mptr[I];
+                }
+            }
+            blk.push_back(nc);
+            if (fits) {
+                L.nblk = (int)blk.size() - 1;
+                if ((e = upload(c, &L.blk, blk)) != cudaSuccess) return cuda_fail(e, "multigrid setup");
+            }
+        }
         L.nnz_next = (int)Ac.ci.size();
         Level C;
         C.n = Ac.n;
@@ -1021,13 +1491,20 @@ fvgb_status symbolic(AmgCache* c, cudaStream_t s) {
             if (dpos[i] < 0) return fvgb_fail(FVGB_ERR_INVALID_ARG, "multigrid: a coarse row without a diagonal entry");
         C.slots = std::max(1, sptr[ns]);
         e = upload(c, &L.gdst, gdst);
-        if (e == cudaSuccess) e = upload(c, &C.sptr, sptr);
+        std::vector<int> sptr_pad(sptr);
+        sptr_pad.resize(sptr.size() + 8);  // k_tail copies whole 16-byte lines
+        if (e == cudaSuccess) e = upload(c, &C.sptr, sptr_pad);
         if (e == cudaSuccess) e = upload(c, &C.scol, scol);
         if (e == cudaSuccess) e = upload(c, &C.dpos, dpos);
         if (e == cudaSuccess) e = dev_alloc(c, &C.val, (size_t)std::max(1, sptr[ns]));
         if (e == cudaSuccess) e = cudaMemset(C.val, 0, sizeof(double) * (size_t)std::max(1, sptr[ns]));
         if (e != cudaSuccess) return cuda_fail(e, "multigrid setup");
         c->lv.push_back(C);
+        h_sptr.push_back(std::move(sptr));
+        h_scol.push_back(std::move(scol));
+        h_agg.push_back(std::move(agg));
+        h_mptr.push_back(std::move(mptr));
+        h_mem.push_back(std::move(mem));
         slot_of = std::move(gdst);
         A = std::move(Ac);
     }
@@ -1043,22 +1520,9 @@ fvgb_status symbolic(AmgCache* c, cudaStream_t s) {
         if (e == cudaSuccess && l > 0) e = dev_alloc(c, &L.b, (size_t)L.n);
         if (e != cudaSuccess) return cuda_fail(e, "multigrid vectors");
     }
-    {
-        const int L = (int)c->lv.size();
-        int t = 1;
-        while (t < L - 1 && c->lv[t].n > kTailRows) ++t;
-        c->tail_from = t;
-        std::vector<TailLevelT<double>> tl;
-        for (int l = t; l < L; ++l) {
-            const Level& V = c->lv[l];
-            tl.push_back(TailLevelT<double>{V.n, SellRows{V.sptr, V.scol, V.val}, V.dinv, V.agg, V.mptr, V.mem, V.b,
-                                            V.x, V.xo, V.r});
-        }
-        cudaError_t e = upload(c, &c->tail, tl);
-        if (e != cudaSuccess) return cuda_fail(e, "multigrid setup");
-    }
+    if (fvgb_status ts = tail_setup(c, h_sptr, h_scol, h_agg, h_mptr, h_mem); ts != FVGB_OK) return ts;
     c->nblk = (int)grid_for(n, kT);
-    cudaError_t e = dev_alloc(c, &c->ainv, (size_t)c->nc * c->nc);
+    cudaError_t e = dev_alloc(c, &c->ainv, (size_t)c->nc * c->nc + 4);  // k_tail copies whole 16-byte lines
     if (e == cudaSuccess) e = dev_alloc(c, &c->r, (size_t)n);
     if (e == cudaSuccess) e = dev_alloc(c, &c->p, (size_t)n);
     if (e == cudaSuccess) e = dev_alloc(c, &c->q, (size_t)n);
@@ -1084,7 +1548,20 @@ fvgb_status numeric(AmgCache* c, cudaStream_t s) {
     }
     const Level& B = c->lv.back();
     k_dense<<<B.n, kT, 0, s>>>(B.n, SellRows{B.sptr, B.scol, B.val}, c->ainv);
-    k_gauss_jordan<<<1, 1024, sizeof(double) * B.n, s>>>(B.n, c->ainv);
+    const int C = c->cluster;
+    if (C > 1 && gj_smem(B.n, C) <= kGjMaxSmem) {
+        cudaLaunchConfig_t lc{};
+        cudaLaunchAttribute at = cluster_attr(C);
+        lc.gridDim = dim3((unsigned)C);
+        lc.blockDim = dim3(kGjThreads);
+        lc.dynamicSmemBytes = gj_smem(B.n, C);
+        lc.stream = s;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        FVGB_CUDA_TRY(cudaLaunchKernelEx(&lc, k_gauss_jordan_cluster, (int)B.n, c->ainv));
+    } else {
+        k_gauss_jordan<<<1, 1024, sizeof(double) * B.n, s>>>(B.n, c->ainv);
+    }
     FVGB_LAUNCH_CHECK("multigrid numeric setup");
     c->version = ls->version;
     return FVGB_OK;
@@ -1104,13 +1581,8 @@ fvgb_status to_f32(AmgCache* c, cudaStream_t s) {
             if (e == cudaSuccess) e = dev_alloc(c, &V.rf, (size_t)V.n);
             if (e != cudaSuccess) return cuda_fail(e, "multigrid FP32 copies");
         }
-        cudaError_t e = dev_alloc(c, &c->ainvf, (size_t)c->nc * c->nc);
-        std::vector<TailLevelT<float>> tl;
-        for (int l = c->tail_from; l < (int)c->lv.size(); ++l) {
-            const Level& V = c->lv[l];
-            tl.push_back(TailLevelT<float>{V.n, SellRowsT<float>{V.sptr, V.scol, V.valf}, V.dinvf, V.agg, V.mptr, V.mem,
-                                           V.bf, V.xf, V.xof, V.rf});
-        }
+        cudaError_t e = dev_alloc(c, &c->ainvf, (size_t)c->nc * c->nc + 4);
+        const std::vector<TailLevelT<float>> tl = tail_levels<float>(c);
         if (e == cudaSuccess) e = upload(c, &c->tailf, tl);
         if (e != cudaSuccess) return cuda_fail(e, "multigrid FP32 copies");
         c->f32 = true;
@@ -1141,7 +1613,7 @@ cudaError_t add_kernel(cudaGraph_t g, cudaGraphNode_t* node, cudaGraphNode_t* de
 }
 
 // The V-cycle z = M r as a chain of kernel nodes after *prev: levels
-// 0..t-1 one kernel per step, levels t..L-1 in the single-block tail.  T is
+// 0..t-1 one kernel per step, levels t..L-1 in the one-cluster tail.  T is
 // the V-cycle's type; with T = float, level 0's b and x are FP32 copies the
 // CG kernels write and z comes back as double.
 template <class T>
@@ -1168,10 +1640,11 @@ template <> const TailLevelT<float>* tail_of<float>(const AmgCache* c) { return 
 
 // r_in: level 0's b (double* for T = double; the FP32 copy otherwise).
 // z_out: the result (always double).  first_sweep_done: level 0's x was
-// formed by the kernel that produced r_in.
+// formed by the kernel that produced r_in.  h: inside the CG's loop; the last sweep
+// then forms beta and sets the loop's condition (k_post_rz).
 template <class T>
 cudaError_t add_vcycle(AmgCache* c, cudaGraph_t g, cudaGraphNode_t* prev, const T* r_in, double* z_out,
-                       VcycleArgs<T>& va, bool first_sweep_done = false) {
+                       VcycleArgs<T>& va, bool first_sweep_done = false, cudaGraphConditionalHandle* h = nullptr) {
     const size_t L = c->lv.size();
     const size_t t = (size_t)c->tail_from;
     if (!first_sweep_done && !std::is_same<T, double>::value) return cudaErrorInvalidValue;  // FP64 only
@@ -1205,9 +1678,9 @@ cudaError_t add_vcycle(AmgCache* c, cudaGraph_t g, cudaGraphNode_t* prev, const 
     double* z = z_out;
     cudaError_t e = cudaSuccess;
     cudaGraphNode_t node;
-    auto add = [&](void* fn, unsigned grid, unsigned block) {
+    auto add = [&](void* fn, unsigned grid, unsigned block, unsigned smem = 0) {
         if (e != cudaSuccess) return;
-        e = add_kernel(g, &node, prev, fn, grid, block, va.args.back().data());
+        e = add_kernel(g, &node, prev, fn, grid, block, va.args.back().data(), smem);
         if (e == cudaSuccess) *prev = node;
     };
     for (size_t l = 0; l < t && e == cudaSuccess; ++l) {  // down
@@ -1217,26 +1690,54 @@ cudaError_t add_vcycle(AmgCache* c, cudaGraph_t g, cudaGraphNode_t* prev, const 
                 va.args.push_back({&c->st, &va.ns[0], &F.dinv, &va.bs[0], &F.x});
                 add((void*)k_smooth0, grid_for(F.n, kT), kT);
             }
+        }
+        Level& C = c->lv[l + 1];
+        if (F.blk) {
+            if (l == 0)
+                va.args.push_back({&c->st, &va.ell[0], &F.blk, &va.bs[0], &va.xv[0], &F.mptr, &F.mem, &va.dv[1], &va.bv[1], &va.xv[1]});
+            else
+                va.args.push_back({&c->st, &va.sell[l], &F.blk, &va.bs[l], &va.xv[l], &F.mptr, &F.mem, &va.dv[l + 1],
+                                   &va.bv[l + 1], &va.xv[l + 1]});
+            add(l == 0 ? (void*)k_resid_restrict<EllRowsT<T>, T> : (void*)k_resid_restrict<SellRowsT<T>, T>,
+                (unsigned)F.nblk, kT);
+            continue;
+        }
+        if (l == 0) {
             va.args.push_back({&c->st, &va.ell[0], &va.ns[0], &va.bs[0], &va.xv[0], &va.rv[0]});
             add((void*)k_resid<EllRowsT<T>, T>, grid_for(F.n, kT), kT);
         } else {
             va.args.push_back({&c->st, &va.sell[l], &va.ns[l], &va.bs[l], &va.xv[l], &va.rv[l]});
             add((void*)k_resid<SellRowsT<T>, T>, grid_for(F.n, kT), kT);
         }
-        Level& C = c->lv[l + 1];
         va.args.push_back({&c->st, &va.ns[l + 1], &F.mptr, &F.mem, &va.rv[l], &va.dv[l + 1], &va.bv[l + 1], &va.xv[l + 1]});
         add((void*)k_restrict<T>, grid_for(C.n, kT), kT);
     }
-    va.args.push_back({&c->st, &va.tail, &va.nl_tail, &va.ainv});
-    add((void*)k_tail<T>, 1, 1024);
+    va.args.push_back({&c->st, &va.tail, &c->tail_parts, &va.nl_tail, &va.ainv});
+    add((void*)k_tail<T>, (unsigned)c->cluster, kTailThreads, (unsigned)c->tail_smem);
+    if (e == cudaSuccess) {
+        cudaLaunchAttributeValue av{};
+        av.clusterDim.x = (unsigned)c->cluster;
+        av.clusterDim.y = av.clusterDim.z = 1;
+        e = cudaGraphKernelNodeSetAttribute(*prev, cudaLaunchAttributeClusterDimension, &av);
+    }
     for (size_t l = t; l-- > 0 && e == cudaSuccess;) {  // up
         Level& F = c->lv[l];
         va.xcs[l] = va.outs[l + 1];
-        if (l == 0) {
+        if (l == 0 && h && F.n <= kFusedPostRows) {
+            va.args.push_back({&c->st, &va.ell[0], &va.ns[l], &va.dv[l], &va.bs[l], &va.xv[l], &va.xcs[l], &F.agg, &z, &c->r,
+                               &c->part, h});
+            add((void*)k_post_rz<EllRowsT<T>, T, true>, grid_for(F.n, kT), kT);
+        } else if (l == 0) {
             va.args.push_back({&c->st, &va.ns[l], &va.xv[l], &va.xcs[l], &F.agg, &va.rv[l]});  // y = x + P xc
             add((void*)k_prolong<T>, grid_for(F.n, kT), kT);
-            va.args.push_back({&c->st, &va.ell[0], &va.ns[l], &va.dv[l], &va.bs[l], &va.rv[l], &z});
-            add((void*)k_post<EllRowsT<T>, T, double>, grid_for(F.n, kT), kT);
+            if (h) {
+                va.args.push_back({&c->st, &va.ell[0], &va.ns[l], &va.dv[l], &va.bs[l], &va.rv[l], &va.xcs[l], &F.agg, &z, &c->r,
+                                   &c->part, h});
+                add((void*)k_post_rz<EllRowsT<T>, T, false>, grid_for(F.n, kT), kT);
+            } else {
+                va.args.push_back({&c->st, &va.ell[0], &va.ns[l], &va.dv[l], &va.bs[l], &va.rv[l], &z});
+                add((void*)k_post<EllRowsT<T>, T, double>, grid_for(F.n, kT), kT);
+            }
         } else {
             va.args.push_back({&c->st, &va.sell[l], &va.ns[l], &va.dv[l], &va.bs[l], &va.xv[l], &va.xcs[l], &F.agg,
                                &va.outs[l]});
@@ -1277,7 +1778,6 @@ fvgb_status build_graph(AmgCache* c, bool f32) {
     void* a_cond[] = {&c->st, &h};
     void* a_spmv[] = {&c->st, &A, &n, &c->p, &c->q, &c->part};
     void* a_upd[] = {&c->st, &n, &c->p, &c->q, &c->r, &c->part, &c->lv[0].dinv, &x0, &d0f, &b0f, &x0f};
-    void* a_rz[] = {&c->st, &n, &c->r, &c->z, &c->part};
     void* a_dir[] = {&c->st, &n, &c->z, &c->p};
     void* a_stats[] = {&c->st};
     void* a_bnorm[] = {&c->st, &n, &b, &c->part};
@@ -1312,13 +1812,9 @@ fvgb_status build_graph(AmgCache* c, bool f32) {
     if (e == cudaSuccess) e = add_kernel(body, &bnode, &bprev, (void*)k_update, nb, kT, a_upd);
     bprev = bnode;
     if (e == cudaSuccess)
-        e = f32 ? add_vcycle<float>(c, body, &bprev, b0f, c->z, f1, true)
-                : add_vcycle<double>(c, body, &bprev, c->r, c->z, v1, true);
-    if (e == cudaSuccess) e = add_kernel(body, &bnode, &bprev, (void*)k_rz, nb, kT, a_rz);
-    bprev = bnode;
+        e = f32 ? add_vcycle<float>(c, body, &bprev, b0f, c->z, f1, true, &h)
+                : add_vcycle<double>(c, body, &bprev, c->r, c->z, v1, true, &h);
     if (e == cudaSuccess) e = add_kernel(body, &bnode, &bprev, (void*)k_dir, nb, kT, a_dir);
-    bprev = bnode;
-    if (e == cudaSuccess) e = add_kernel(body, &bnode, &bprev, (void*)k_cond, 1, 1, a_cond);
     if (e == cudaSuccess) e = add_kernel(g, &node, &prev, (void*)k_stats, 1, 1, a_stats);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&out, g, 0);
     cudaGraphDestroy(g);
