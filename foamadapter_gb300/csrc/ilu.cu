@@ -67,7 +67,9 @@ struct Csr {
     const int* dof;  // diagonal offset of every row
 };
 
-__device__ __forceinline__ volatile const int32_t& done_flag(const IluState* st) { return st->done; }
+// Set by an earlier kernel, or by the last block of this one after every block has read
+// it: a plain load, one request per SM (a volatile one goes to L2 from every warp).
+__device__ __forceinline__ int done_flag(const IluState* st) { return st->done; }
 
 // ------------------------------------------------------------ reduction tree
 // Row j of this thread: the solver's tree layout.
@@ -75,20 +77,23 @@ __device__ __forceinline__ int tree_row(int R, int j) {
     return blockIdx.x * (kT * R) + (threadIdx.x >> 5) * (32 * R) + j * 32 + (threadIdx.x & 31);
 }
 
-// Block sum of one value per thread; valid in warp 0.
+// Block sum of one value per thread, in every thread; formed by a warp that differs from
+// block to block (solver.cu, block_tree).
 __device__ __forceinline__ double block_tree(double v, double* sm) {
+    __shared__ double out;
     sm[threadIdx.x] = v;
     __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x < 32) {
-        s = sm[threadIdx.x];
+    if ((threadIdx.x >> 5) == (blockIdx.x & 7u)) {
+        const int lane = threadIdx.x & 31;
+        double s = sm[lane];
 #pragma unroll
-        for (int k = 1; k < kT / 32; ++k) s = s + sm[threadIdx.x + 32 * k];
+        for (int k = 1; k < kT / 32; ++k) s = s + sm[lane + 32 * k];
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, off);
+        if (lane == 0) out = s;
     }
     __syncthreads();
-    return s;
+    return out;
 }
 
 __device__ __forceinline__ double final_tree(const double* part, int nb, double* sm) {

@@ -122,20 +122,46 @@ __device__ __forceinline__ int blk_row(const Blk& k, int j) {
     return j < k.R ? k.row0 + (threadIdx.x >> 5) * (32 * k.R) + j * 32 + (threadIdx.x & 31) : INT_MAX;
 }
 
-// Block sum of one value per thread; result valid in warp 0 (every lane).
+// Block sums: the 256 partials in groups of 32 lanes (lane l: l, l+32, ..., l+224),
+// then a xor butterfly; the result in every thread.  The 12 serial additions run in a
+// warp that differs from block to block (and, of a pair of sums, in two warps): an FP64
+// instruction occupies its scheduler for 64 clocks, the blocks of an SM end together,
+// and warp 0 of every one of 7 blocks sits on the same scheduler (2.7 us per sum).
+__device__ __forceinline__ double warp_tree(const double* sm) {
+    const int lane = threadIdx.x & 31;
+    double s = sm[lane];
+#pragma unroll
+    for (int k = 1; k < kT / 32; ++k) s = s + sm[lane + 32 * k];
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, off);
+    return s;
+}
+
 __device__ __forceinline__ double block_tree(double v, double* sm) {
+    __shared__ double out;
     sm[threadIdx.x] = v;
     __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x < 32) {
-        s = sm[threadIdx.x];
-#pragma unroll
-        for (int k = 1; k < kT / 32; ++k) s = s + sm[threadIdx.x + 32 * k];
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, off);
+    if ((threadIdx.x >> 5) == (blockIdx.x & 7u)) {
+        const double s = warp_tree(sm);
+        if ((threadIdx.x & 31) == 0) out = s;
     }
     __syncthreads();
-    return s;
+    return out;
+}
+
+__device__ __forceinline__ void block_tree2(double a, double b, double* sma, double* smb, double* ta, double* tb) {
+    __shared__ double out[2];
+    sma[threadIdx.x] = a;
+    smb[threadIdx.x] = b;
+    __syncthreads();
+    const unsigned w = ((threadIdx.x >> 5) - blockIdx.x) & 7u;
+    if (w < 2) {
+        const double s = warp_tree(w == 0 ? sma : smb);
+        if ((threadIdx.x & 31) == 0) out[w] = s;
+    }
+    __syncthreads();
+    *ta = out[0];
+    *tb = out[1];
 }
 
 // FP32 block sum (inner solve of the mixed scheme: keeps the FP64 pipe free).
@@ -160,6 +186,16 @@ __device__ __forceinline__ double final_tree(const double* part, int nb, double*
     return block_tree(a, sm);
 }
 
+__device__ __forceinline__ void final_tree2(const double* pa, const double* pb, int nb, double* sma, double* smb,
+                                            double* ta, double* tb) {
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < nb; i += kT) {
+        a = a + __ldcg(&pa[i]);
+        b = b + __ldcg(&pb[i]);
+    }
+    block_tree2(a, b, sma, smb, ta, tb);
+}
+
 // Thread 0 has written this block's partials; true in the block that arrives
 // last among `count` blocks sharing `counter` (which wraps back to 0).  The
 // leading barrier keeps a second call in the same kernel from overwriting the
@@ -176,18 +212,33 @@ __device__ __forceinline__ bool arrive_last(unsigned int* counter, unsigned int 
     return am_last;
 }
 
+// A case's flags (active, inner_active, half) are set by earlier kernels, or by its last
+// block after every block has read them, and read with plain loads: one request per SM.
+// Volatile loads go to L2 from every warp, 8,192 times to one address with 1,024
+// blocks, which took 2.2 us of every kernel.  The counts below change during a kernel.
 __device__ __forceinline__ int ld_volatile(const int32_t* p) { return *(const volatile int32_t*)p; }
+
+// Loads of the FP32 matrix: evict-first, so that what stays in L2 from one kernel to the
+// next is the vectors.  On 128^3 cells the matrix copy is 88 MB and the six vectors of
+// the inner CG 50 MB, against 126 MB of L2 on two dies: a mixed solve 17.3 -> 14.0 ms.
+// (The FP64 solve's vectors, 100 MB beside a 146 MB matrix, do not fit either way: no
+// difference.)
+template <bool STREAM, class V>
+__device__ __forceinline__ V ld_matrix(const V* p) {
+    return STREAM ? __ldcs(p) : __ldg(p);
+}
 
 // Columns of a row's first 8 slots (the row itself past its width), the
 // offset or column array chosen once per row so the index loads are issued
 // together.
+template <bool STREAM = false>
 __device__ __forceinline__ void slot_cols(const MeshView& m, int base, int w, int i, int* col) {
     if (m.m_off) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) col[k] = k < w ? i + (int)__ldg(&m.m_off[base + k * 32]) : i;
+        for (int k = 0; k < 8; ++k) col[k] = k < w ? i + (int)ld_matrix<STREAM>(&m.m_off[base + k * 32]) : i;
     } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) col[k] = k < w ? __ldg(&m.m_col[base + k * 32]) : i;
+        for (int k = 0; k < 8; ++k) col[k] = k < w ? ld_matrix<STREAM>(&m.m_col[base + k * 32]) : i;
     }
 }
 
@@ -265,14 +316,14 @@ __device__ __forceinline__ float spmv_row_diff(const MeshView& m, const float* _
     const int base = b0 + lane;
     const int w = (__ldg(&m.m_ptr[slice + 1]) - b0) >> 5;
     int col[8];
-    slot_cols(m, base, w, i, col);
+    slot_cols<true>(m, base, w, i, col);
     float v[8], xv[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         v[k] = 0.0f;
         xv[k] = 0.0f;
         if (k < w) {
-            v[k] = __ldg(&a[base + k * 32]);
+            v[k] = ld_matrix<true>(&a[base + k * 32]);
             xv[k] = __ldg(&x[col[k]]);
         }
     }
@@ -320,13 +371,15 @@ __global__ void __launch_bounds__(kT)
         arz = fma(ri, zi, arz);
         arr = fma(ri, ri, arr);
     }
-    const double ba = block_tree(arz, sma), bb = block_tree(arr, smb);
+    double ba, bb;
+    block_tree2(arz, arr, sma, smb, &ba, &bb);
     if (threadIdx.x == 0) {
         pa[blockIdx.x] = ba;
         pb[blockIdx.x] = bb;
     }
     if (arrive_last(&cs->counter, k.nbc)) {
-        const double rz = final_tree(pa + k.blk0, k.nbc, sma), rr = final_tree(pb + k.blk0, k.nbc, smb);
+        double rz, rr;
+        final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &rz, &rr);
         if (threadIdx.x == 0) {
             const SolverParams& prm = L.bs->prm;
             const double res0 = sqrt(rr);
@@ -357,7 +410,7 @@ __global__ void __launch_bounds__(kT, MINB)
                double* __restrict__ q, double* __restrict__ pa) {
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->active)) return;
+    if (!cs->active) return;
     __shared__ double sma[kT];
     double acc = 0.0;
 #pragma unroll
@@ -390,7 +443,9 @@ __global__ void __launch_bounds__(kT, MINB)
     __shared__ double sma[kT], smb[kT];
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (ld_volatile(&cs->active)) {
+    const bool was_active = cs->active != 0;
+    bool last = false;
+    if (was_active) {
         double* __restrict__ x = L.bs->prm.x;
         const double alpha = cs->alpha;
         double arz = 0.0, arr = 0.0;
@@ -406,13 +461,16 @@ __global__ void __launch_bounds__(kT, MINB)
             arz = fma(ri, zi, arz);
             arr = fma(ri, ri, arr);
         }
-        const double ba = block_tree(arz, sma), bb = block_tree(arr, smb);
+        double ba, bb;
+        block_tree2(arz, arr, sma, smb, &ba, &bb);
         if (threadIdx.x == 0) {
             pa[blockIdx.x] = ba;
             pb[blockIdx.x] = bb;
         }
-        if (arrive_last(&cs->counter, k.nbc)) {
-            const double rzn = final_tree(pa + k.blk0, k.nbc, sma), rr = final_tree(pb + k.blk0, k.nbc, smb);
+        last = arrive_last(&cs->counter, k.nbc);
+        if (last) {
+            double rzn, rr;
+            final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &rzn, &rr);
             if (threadIdx.x == 0) {
                 const double res = sqrt(rr);
                 cs->res = res;
@@ -433,7 +491,10 @@ __global__ void __launch_bounds__(kT, MINB)
             }
         }
     }
-    if (arrive_last(&L.bs->gcounter, gridDim.x) && threadIdx.x == 0 && setc)
+    // a single case's last block is the grid's: no second count of arrivals
+    const bool decides = k.nbc == (int)gridDim.x ? last || (!was_active && blockIdx.x == 0)
+                                                 : arrive_last(&L.bs->gcounter, gridDim.x);
+    if (decides && threadIdx.x == 0 && setc)
         cudaGraphSetConditional(h, ld_volatile(&L.bs->n_active) > 0 ? 1u : 0u);
 }
 
@@ -441,7 +502,7 @@ __global__ void __launch_bounds__(kT)
     k_pcg_dir(Layout L, const double* __restrict__ z, double* __restrict__ p) {
     const Blk k = blk_info(L);
     const CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->active)) return;
+    if (!cs->active) return;
     const double beta = cs->beta;
     double pv[kRowsPerThread], zv[kRowsPerThread];
 #pragma unroll
@@ -592,7 +653,7 @@ __global__ void __launch_bounds__(kT)
              double* __restrict__ p, double* __restrict__ y) {
     const Blk k = blk_info(L);
     const CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->active)) return;
+    if (!cs->active) return;
     const double beta = cs->beta, omega = cs->omega;
 #pragma unroll
     for (int j = 0; j < kRowsPerThread; ++j) {
@@ -609,7 +670,7 @@ __global__ void __launch_bounds__(kT)
                const double* __restrict__ rr, double* __restrict__ v, double* __restrict__ pa) {
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->active)) return;
+    if (!cs->active) return;
     __shared__ double sma[kT];
     double acc = 0.0;
 #pragma unroll
@@ -639,7 +700,7 @@ __global__ void __launch_bounds__(kT)
            double* __restrict__ sv, double* __restrict__ z, double* __restrict__ pa) {
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->active)) return;
+    if (!cs->active) return;
     __shared__ double sma[kT];
     const double alpha = cs->alpha;
     double acc = 0.0;
@@ -675,9 +736,9 @@ __global__ void __launch_bounds__(kT)
                double* __restrict__ pa, double* __restrict__ pb) {
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->active)) return;
+    if (!cs->active) return;
     __shared__ double sma[kT], smb[kT];
-    if (ld_volatile(&cs->half)) {  // converged at the half step: x += alpha y, done
+    if (cs->half) {  // converged at the half step: x += alpha y, done
         double* __restrict__ x = L.bs->prm.x;
         const double alpha = cs->alpha;
 #pragma unroll
@@ -702,13 +763,15 @@ __global__ void __launch_bounds__(kT)
         ats = fma(ti, __ldg(&sv[i]), ats);
         att = fma(ti, ti, att);
     }
-    const double ba = block_tree(ats, sma), bb = block_tree(att, smb);
+    double ba, bb;
+    block_tree2(ats, att, sma, smb, &ba, &bb);
     if (threadIdx.x == 0) {
         pa[blockIdx.x] = ba;
         pb[blockIdx.x] = bb;
     }
     if (!arrive_last(&cs->counter, k.nbc)) return;
-    const double ts = final_tree(pa + k.blk0, k.nbc, sma), tt = final_tree(pb + k.blk0, k.nbc, smb);
+    double ts, tt;
+    final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &ts, &tt);
     if (threadIdx.x == 0) {
         const double omega = ts / tt;
         cs->omega = omega;
@@ -726,7 +789,7 @@ __global__ void __launch_bounds__(kT)
     __shared__ double sma[kT], smb[kT];
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (ld_volatile(&cs->active)) {
+    if (cs->active) {
         double* __restrict__ x = L.bs->prm.x;
         const double alpha = cs->alpha, omega = cs->omega;
         double arho = 0.0, arr = 0.0;
@@ -740,13 +803,15 @@ __global__ void __launch_bounds__(kT)
             arho = fma(__ldg(&rr[i]), ri, arho);
             arr = fma(ri, ri, arr);
         }
-        const double ba = block_tree(arho, sma), bb = block_tree(arr, smb);
+        double ba, bb;
+        block_tree2(arho, arr, sma, smb, &ba, &bb);
         if (threadIdx.x == 0) {
             pa[blockIdx.x] = ba;
             pb[blockIdx.x] = bb;
         }
         if (arrive_last(&cs->counter, k.nbc)) {
-            const double rho = final_tree(pa + k.blk0, k.nbc, sma), rr2 = final_tree(pb + k.blk0, k.nbc, smb);
+            double rho, rr2;
+            final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &rho, &rr2);
             if (threadIdx.x == 0) {
                 const double res = sqrt(rr2);
                 cs->res = res;
@@ -835,13 +900,15 @@ __global__ void __launch_bounds__(kT)
         arho = fma(ri, zi, arho);
         arr = fma(ri, ri, arr);
     }
-    const double ba = block_tree(arho, sma), bb = block_tree(arr, smb);
+    double ba, bb;
+    block_tree2(arho, arr, sma, smb, &ba, &bb);
     if (threadIdx.x == 0) {
         pa[blockIdx.x] = ba;
         pb[blockIdx.x] = bb;
     }
     if (arrive_last(&cs->counter, k.nbc)) {
-        const double rho = final_tree(pa + k.blk0, k.nbc, sma), rr = final_tree(pb + k.blk0, k.nbc, smb);
+        double rho, rr;
+        final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &rho, &rr);
         if (threadIdx.x == 0) {
             const SolverParams& prm = L.bs->prm;
             const double res0 = sqrt(rr);
@@ -874,7 +941,7 @@ __global__ void __launch_bounds__(kT)
              double* __restrict__ p2) {
     const Blk k = blk_info(L);
     const CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->active)) return;
+    if (!cs->active) return;
     const double beta = cs->beta;
 #pragma unroll
     for (int j = 0; j < kRowsPerThread; ++j) {
@@ -891,7 +958,7 @@ __global__ void __launch_bounds__(kT)
               double* __restrict__ pa) {
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->active)) return;
+    if (!cs->active) return;
     __shared__ double sma[kT];
     double acc = 0.0;
 #pragma unroll
@@ -925,7 +992,7 @@ __global__ void __launch_bounds__(kT)
     __shared__ double sma[kT], smb[kT];
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (ld_volatile(&cs->active)) {
+    if (cs->active) {
         double* __restrict__ x = L.bs->prm.x;
         const double alpha = cs->alpha;
         double arho = 0.0, arr = 0.0;
@@ -945,13 +1012,15 @@ __global__ void __launch_bounds__(kT)
             arho = fma(r2i, zi, arho);
             arr = fma(ri, ri, arr);
         }
-        const double ba = block_tree(arho, sma), bb = block_tree(arr, smb);
+        double ba, bb;
+        block_tree2(arho, arr, sma, smb, &ba, &bb);
         if (threadIdx.x == 0) {
             pa[blockIdx.x] = ba;
             pb[blockIdx.x] = bb;
         }
         if (arrive_last(&cs->counter, k.nbc)) {
-            const double rho = final_tree(pa + k.blk0, k.nbc, sma), rr = final_tree(pb + k.blk0, k.nbc, smb);
+            double rho, rr;
+            final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &rho, &rr);
             if (threadIdx.x == 0) {
                 const double res = sqrt(rr);
                 cs->res = res;
@@ -1082,7 +1151,7 @@ __global__ void __launch_bounds__(kT)
     __shared__ float smf[kT];
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (FIRST || ld_volatile(&cs->active)) {
+    if (FIRST || cs->active) {
         const double* __restrict__ x = L.bs->prm.x;
         double sig, isig;
         residual_scale(cs->sres, &sig, &isig);  // from the previous residual (k_ir_prepare's for the first)
@@ -1113,7 +1182,8 @@ __global__ void __launch_bounds__(kT)
             pc[blockIdx.x] = bc;
         }
         if (arrive_last(&cs->counter, k.nbc)) {
-            const double rr = final_tree(pa + k.blk0, k.nbc, sma), rho = final_tree(pb + k.blk0, k.nbc, smb);
+            double rr, rho;
+            final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &rr, &rho);
             const double sr2 = final_tree(pc + k.blk0, k.nbc, smc);
             if (threadIdx.x == 0) {
                 const SolverParams& prm = L.bs->prm;
@@ -1180,7 +1250,7 @@ __global__ void __launch_bounds__(kT)
     k_ir_reliable_dir(Layout L, const float* __restrict__ dinv, const float* __restrict__ rh, float* __restrict__ p) {
     const Blk k = blk_info(L);
     const CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->inner_active)) return;
+    if (!cs->inner_active) return;
     const float fb = cs->frel;
 #pragma unroll
     for (int j = 0; j < kRowsPerThread; ++j) {
@@ -1203,7 +1273,7 @@ __global__ void __launch_bounds__(kT, MINB)
               const float* __restrict__ p, float* __restrict__ q, double* __restrict__ pa) {
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->inner_active)) return;
+    if (!cs->inner_active) return;
     __shared__ double sma[kT];
     __shared__ float smf[kT];
     float acc = 0.0f;
@@ -1244,7 +1314,9 @@ __global__ void __launch_bounds__(kT, MINB)
     __shared__ float smf[kT];
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (ld_volatile(&cs->inner_active)) {
+    const bool was_active = cs->inner_active != 0;
+    bool last = false;
+    if (was_active) {
         const float fa = cs->falpha;
         float acc = 0.0f;
         constexpr int G = 4;  // rows whose loads are issued together (more spill at 32-40 registers)
@@ -1275,7 +1347,8 @@ __global__ void __launch_bounds__(kT, MINB)
         }
         const float ba = block_tree_f(acc, smf);
         if (threadIdx.x == 0) pa[blockIdx.x] = (double)ba;
-        if (arrive_last(&cs->counter, k.nbc)) {
+        last = arrive_last(&cs->counter, k.nbc);
+        if (last) {
             const double rhon = final_tree(pa + k.blk0, k.nbc, sma);
             if (threadIdx.x == 0) {
                 const SolverParams& prm = L.bs->prm;
@@ -1289,7 +1362,10 @@ __global__ void __launch_bounds__(kT, MINB)
             }
         }
     }
-    if (arrive_last(&L.bs->gcounter, gridDim.x) && threadIdx.x == 0 && setc)
+    // a single case's last block is the grid's: no second count of arrivals
+    const bool decides = k.nbc == (int)gridDim.x ? last || (!was_active && blockIdx.x == 0)
+                                                 : arrive_last(&L.bs->gcounter, gridDim.x);
+    if (decides && threadIdx.x == 0 && setc)
         cudaGraphSetConditional(h_inner, ld_volatile(&L.bs->n_inner) > 0 ? 1u : 0u);
 }
 
@@ -1298,7 +1374,7 @@ __global__ void __launch_bounds__(kT)
     k_ir_dir(Layout L, const float* __restrict__ dinv, const float* __restrict__ rh, float* __restrict__ p) {
     const Blk k = blk_info(L);
     const CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->inner_active)) return;
+    if (!cs->inner_active) return;
     const float fb = cs->fbeta;
     float pv[kRowsPerThread], dv[kRowsPerThread], rv[kRowsPerThread];
 #pragma unroll
@@ -1322,7 +1398,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT) k_ir_xupdate(Layout L, const float* __restrict__ y) {
     const Blk k = blk_info(L);
     const CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->active)) return;
+    if (!cs->active) return;
     double* __restrict__ x = L.bs->prm.x;
     const double isig = cs->isig;
 #pragma unroll
@@ -1358,7 +1434,7 @@ __global__ void __launch_bounds__(kT)
     __shared__ float smf[kT];
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (FIRST || ld_volatile(&cs->active)) {
+    if (FIRST || cs->active) {
         const double* __restrict__ x = L.bs->prm.x;
         double sig, isig;
         residual_scale(cs->sres, &sig, &isig);
@@ -1390,7 +1466,8 @@ __global__ void __launch_bounds__(kT)
             pc[blockIdx.x] = bc;
         }
         if (arrive_last(&cs->counter, k.nbc)) {
-            const double rr2 = final_tree(pa + k.blk0, k.nbc, sma), rho = final_tree(pb + k.blk0, k.nbc, smb);
+            double rr2, rho;
+            final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &rr2, &rho);
             const double sr2 = final_tree(pc + k.blk0, k.nbc, smc);
             if (threadIdx.x == 0) {
                 const SolverParams& prm = L.bs->prm;
@@ -1463,7 +1540,7 @@ __global__ void __launch_bounds__(kT)
              float* __restrict__ p, float* __restrict__ yv) {
     const Blk k = blk_info(L);
     const CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->inner_active)) return;
+    if (!cs->inner_active) return;
     const float fb = cs->fbeta, fo = cs->fomega;
 #pragma unroll
     for (int j = 0; j < kRowsPerThread; ++j) {
@@ -1482,7 +1559,7 @@ __global__ void __launch_bounds__(kT)
                double* __restrict__ pa) {
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->inner_active)) return;
+    if (!cs->inner_active) return;
     __shared__ double sma[kT];
     __shared__ float smf[kT];
     float acc = 0.0f;
@@ -1515,7 +1592,7 @@ __global__ void __launch_bounds__(kT)
            float* __restrict__ sv, float* __restrict__ z, double* __restrict__ pa) {
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->inner_active)) return;
+    if (!cs->inner_active) return;
     __shared__ double sma[kT];
     __shared__ float smf[kT];
     const float fa = cs->falpha;
@@ -1546,10 +1623,10 @@ __global__ void __launch_bounds__(kT)
                float* __restrict__ t, float* __restrict__ e, double* __restrict__ pa, double* __restrict__ pb) {
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (!ld_volatile(&cs->inner_active)) return;
+    if (!cs->inner_active) return;
     __shared__ double sma[kT], smb[kT];
     __shared__ float smf[kT], smg[kT];
-    if (ld_volatile(&cs->half)) {
+    if (cs->half) {
         const float fa = cs->falpha;
 #pragma unroll
         for (int j = 0; j < kRowsPerThread; ++j) {
@@ -1581,7 +1658,8 @@ __global__ void __launch_bounds__(kT)
         pb[blockIdx.x] = (double)bb;
     }
     if (!arrive_last(&cs->counter, k.nbc)) return;
-    const double ts = final_tree(pa + k.blk0, k.nbc, sma), tt = final_tree(pb + k.blk0, k.nbc, smb);
+    double ts, tt;
+    final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &ts, &tt);
     if (threadIdx.x == 0) {
         const double omega = ts / tt;
         if (tt == 0.0 || !isfinite(omega) || omega == 0.0) {
@@ -1603,7 +1681,7 @@ __global__ void __launch_bounds__(kT)
     __shared__ float smf[kT], smg[kT];
     const Blk k = blk_info(L);
     CaseState* cs = &L.cases[k.c];
-    if (ld_volatile(&cs->inner_active)) {
+    if (cs->inner_active) {
         const float fa = cs->falpha, fo = cs->fomega;
         float arho = 0.0f, arr = 0.0f;
 #pragma unroll
@@ -1622,7 +1700,8 @@ __global__ void __launch_bounds__(kT)
             pb[blockIdx.x] = (double)bb;
         }
         if (arrive_last(&cs->counter, k.nbc)) {
-            const double rho = final_tree(pa + k.blk0, k.nbc, sma), r2 = final_tree(pb + k.blk0, k.nbc, smb);
+            double rho, r2;
+            final_tree2(pa + k.blk0, pb + k.blk0, k.nbc, sma, smb, &rho, &r2);
             if (threadIdx.x == 0) {
                 const SolverParams& prm = L.bs->prm;
                 cs->inner_it += 1;
