@@ -99,10 +99,23 @@ __device__ __forceinline__ double facc0(bool plus, double x) {
 // stream, so releasing them never synchronises the device as cudaFree does.
 // The serving loop sets the context on its thread; everything else uses
 // cudaMalloc and cudaFree.  An object keeps the mode it was created in.
+//
+// A request takes one piece of the pool at its admission, of the size its budget
+// counts for it, and its objects' ~50 allocations are cut from it.  Each allocation
+// from the pool cost 15 us with its wait, and 60 once some hundreds of releases had
+// cut the pool up: bursts of 16 requests with 27 ms of device work went from 54 ms
+// to 150 ms, and stay at 46 to 62 ms with one piece each.  What a piece has no room
+// for comes from the pool as before.
+struct DevMemArena {
+    char* base = nullptr;
+    size_t size = 0, used = 0;
+    bool holds(const void* p) const { return (const char*)p >= base && (const char*)p < base + size; }
+};
 struct DevMemCtx {
     cudaMemPool_t pool = nullptr;
     cudaStream_t alloc = nullptr;    // private stream of the allocations
     cudaStream_t release = nullptr;  // stream whose work last used what is released
+    DevMemArena* arena = nullptr;    // of the request whose objects are created, used or released
 };
 inline DevMemCtx& devmem_ctx() {
     static thread_local DevMemCtx c;
@@ -113,12 +126,21 @@ inline cudaError_t devmem_alloc(void** p, size_t bytes, bool pooled) {
     if (!pooled) return cudaMalloc(p, bytes);
     const DevMemCtx& c = devmem_ctx();
     if (!c.pool) return cudaErrorInvalidValue;  // a pooled object grows only on the thread that owns the pool
+    if (DevMemArena* a = c.arena) {
+        const size_t need = (bytes + 255) & ~(size_t)255;
+        if (need <= a->size - a->used) {
+            *p = a->base + a->used;
+            a->used += need;
+            return cudaSuccess;
+        }
+    }
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c.pool, c.alloc);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c.alloc);
     return e;
 }
 inline void devmem_free(void* p, bool pooled) {
     if (!p) return;
+    if (pooled && devmem_ctx().arena && devmem_ctx().arena->holds(p)) return;  // goes with the arena
     if (pooled) cudaFreeAsync(p, devmem_ctx().release);
     else cudaFree(p);
 }

@@ -60,6 +60,7 @@ struct Slot {
     double *U = nullptr, *Ub = nullptr;
     fvgb_solver_stats* stats_dev = nullptr;  // [kChunk]
     fvgb_solver_stats* stats_host = nullptr; // pinned [kChunk]
+    DevMemArena arena;                       // one piece of the pool for all of the above
     cudaEvent_t done_ev = nullptr;
     int32_t inflight = 0;                    // steps of the chunk in flight
     int32_t final_status = FVGB_OK;          // set when the request is retiring
@@ -118,6 +119,7 @@ int64_t estimate_bytes(const fvgb_serve_request& r) {
 // free list (cudaFreeHost would synchronise the device).
 void release(fvgb_server* sv, Slot* s) {
     devmem_ctx().release = s->stream;
+    devmem_ctx().arena = &s->arena;
     double* bufs[] = {s->T, s->Told, s->Tb, s->F, s->gamma, s->ref, s->U, s->Ub};
     for (double* b : bufs) devmem_free(b, true);
     devmem_free(s->stats_dev, true);
@@ -131,6 +133,9 @@ void release(fvgb_server* sv, Slot* s) {
     s->stats_dev = nullptr;
     s->ls = nullptr;
     s->mesh = nullptr;
+    devmem_ctx().arena = nullptr;
+    devmem_free(s->arena.base, true);
+    s->arena = DevMemArena{};
     devmem_ctx().release = nullptr;
 }
 
@@ -157,6 +162,14 @@ __global__ void k_fill(double* a, int count, double v) {
 
 fvgb_status setup(fvgb_server* sv, Slot* s) {
     const fvgb_serve_request& r = s->req;
+    devmem_ctx().arena = nullptr;
+    if (devmem_alloc((void**)&s->arena.base, (size_t)s->bytes, true) == cudaSuccess) {
+        s->arena.size = (size_t)s->bytes;
+    } else {  // no one piece that large: piece by piece from the pool
+        s->arena.base = nullptr;
+        cudaGetLastError();
+    }
+    devmem_ctx().arena = &s->arena;
     fvgb_box_spec spec{r.nx, r.ny, r.nz, 1.0, 1.0, 1.0, 0.0, 0, 0};
     int32_t range[2];
     fvgb_status st = fvgb_mesh_create_boxes(&spec, 1, &s->mesh, range, s->stream);
@@ -373,6 +386,7 @@ void run(fvgb_server* sv) {
             s->stream = sv->streams[next_stream++ % sv->streams.size()];
             s->start_s = sv->now();
             fvgb_status st = setup(sv, s);
+            devmem_ctx().arena = nullptr;
             if (st != FVGB_OK) {
                 finish(sv, s, st);
                 continue;
@@ -426,7 +440,9 @@ void run(fvgb_server* sv) {
             }
             const int todo = std::min(kChunk, s->req.steps - s->steps_done);
             int32_t status = FVGB_OK;
+            devmem_ctx().arena = &s->arena;
             for (int k = 0; k < todo && status == FVGB_OK; ++k) status = enqueue_step(s, k);
+            devmem_ctx().arena = nullptr;
             if (status == FVGB_OK &&
                 cudaMemcpyAsync(s->stats_host, s->stats_dev, sizeof(fvgb_solver_stats) * todo,
                                 cudaMemcpyDeviceToHost, s->stream) != cudaSuccess)

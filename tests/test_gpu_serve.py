@@ -209,3 +209,26 @@ def test_rhs_only_steps_equal_full_reassembly(cuda, precision):
         outs.append([o.copy() for _, _, o in subs])
     for a, b in zip(*outs):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("flags", [0, abi.SERVE_REASSEMBLE])
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED_IR])
+def test_requests_on_reused_memory_keep_their_bits(cuda, precision, flags):
+    """Later bursts run on the pieces of memory that earlier requests gave back."""
+    reqs = [(*d, 5, (0.4, -0.3, 0.2), 2e-2) for d in [(2, 2, 2), (31, 2, 2), (33, 7, 5), (8, 8, 8), (20, 19, 17)]]
+    alone = []
+    for r in reqs:
+        sv = make_server()
+        _, rid, out = submit(sv, *r, precision=precision, flags=flags)
+        res = drain(sv, 1)
+        abi.lib().fvgb_server_destroy(sv)
+        alone.append((res[rid].status, out))   # (2, 2, 2) ends above the tolerance in mixed precision
+    sv = make_server(streams=3)
+    for burst in range(3):
+        sent = [(k, submit(sv, *reqs[k], precision=precision, flags=flags))
+                for k in (range(5) if burst % 2 == 0 else range(4, -1, -1))]
+        res = drain(sv, 5)
+        for k, (_, rid, out) in sent:
+            assert res[rid].status == alone[k][0]
+            np.testing.assert_array_equal(out, alone[k][1])
+    abi.lib().fvgb_server_destroy(sv)
