@@ -81,6 +81,34 @@ __device__ __forceinline__ double fmul(const MeshView& m, double a, double b) { 
 __device__ __forceinline__ double facc(const MeshView& m, double s, bool plus, double x) {
     return __fma_rn(x, plus ? m.k_one : m.k_mone, s);
 }
+// a * b with the bits of fmul, on the integer pipes when both factors lie in
+// 2^-511 .. 2^511 (no zero, subnormal, infinity or NaN: then the product is normal or
+// rounds to infinity), by fmul otherwise.  The 53 x 53-bit product is formed with the
+// factors shifted left by 3 and 10, so that its bits from 64 up are the 53 of the
+// result, a rounding bit and perhaps one more, and every bit below is sticky.
+__device__ __forceinline__ double imul(const MeshView& m, double a, double b) {
+    const unsigned alo = (unsigned)__double2loint(a), ahi = (unsigned)__double2hiint(a);
+    const unsigned blo = (unsigned)__double2loint(b), bhi = (unsigned)__double2hiint(b);
+    const unsigned ea = ahi & 0x7ff00000u, eb = bhi & 0x7ff00000u;
+    if (max(ea - (512u << 20), eb - (512u << 20)) > (1022u << 20)) return fmul(m, a, b);
+    const unsigned am = (ahi & 0xfffffu) | 0x100000u, bm = (bhi & 0xfffffu) | 0x100000u;
+    const unsigned ah = __funnelshift_l(alo, am, 3), al = alo << 3;
+    const unsigned bh = __funnelshift_l(blo, bm, 10), bl = blo << 10;
+    const unsigned long long p = (unsigned long long)al * bl;
+    unsigned long long t = (unsigned long long)ah * bl + (p >> 32);  // < 2^57
+    t += (unsigned long long)al * bh;                                // < 2^63 + 2^57
+    const unsigned long long q = (unsigned long long)ah * bh + (t >> 32);  // 2^53 .. 2^55
+    unsigned ql = (unsigned)q, qh = (unsigned)(q >> 32);
+    const unsigned n = qh >> 22;  // one bit more than 53 and the rounding bit
+    const unsigned sticky = (unsigned)t | (unsigned)p | (ql & n);
+    ql = __funnelshift_r(ql, qh, n);
+    qh >>= n;
+    const unsigned long long r =
+        ((((unsigned long long)qh << 32) | ql) + (((ql >> 1) & 1u) | (sticky != 0u))) >> 1;  // half to even
+    // the mantissa's leading bit adds the last 1 to the exponent, a carry one more
+    const unsigned hi = (unsigned)(r >> 32) + (ea + eb - (1024u << 20)) + (n << 20);
+    return __hiloint2double((int)(hi | ((ahi ^ bhi) & 0x80000000u)), (int)(unsigned)r);
+}
 // The first accumulation of a sum from +0, +0 + x (plus) or +0 - x, on the
 // integer pipes: the IEEE result is x or -x exactly, except that a zero result
 // is +0 (a sum of opposite zeros rounds to +0 to nearest).  One FP64

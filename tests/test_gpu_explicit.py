@@ -238,3 +238,48 @@ def test_advection_many_steps_in_one_call(cuda, n, nsteps):
     for _ in range(nsteps):
         T, Tb = o.advect_euler(a.flux.host(), T, Tb, a.dt, np.full(hm.npatch, 2, np.int32), np.zeros(hm.nbf))
     np.testing.assert_array_equal(a.T.host(), T)
+
+
+@pytest.mark.parametrize("dims", [(36, 36, 30), (37, 37, 29), (103, 64, 61)])
+@pytest.mark.parametrize("ncomp", [1, 3])
+@pytest.mark.parametrize("tile", [2, 4, 8])
+def test_passes_by_mesh_size_and_extreme_values(cuda, dims, ncomp, tile):
+    """One pass up to 38,912 cells (here 38,880), a face pass and a cell pass beyond
+    (39,701 and 402,112, no multiple of a block): the oracle's bits with values from the
+    subnormal to the overflowing, zeros of both signs, infinities and NaN among ordinary
+    ones, whose products the face passes form on the integer pipes."""
+    hm = mesh.box(*dims, jitter=0.1, seed=2)
+    dm = DeviceMesh(hm)
+    abi.check(abi.lib().fvgb_mesh_face_tile(dm.handle, tile))
+    o = Oracle(hm)
+    rng = np.random.default_rng(5 + ncomp)
+
+    def wild(n):
+        v = rng.standard_normal(n)
+        k = rng.integers(0, 40, n)
+        v = np.where(k == 0, v * 2.0 ** rng.integers(-1060, -480, n), v)
+        v = np.where(k == 1, v * 2.0 ** rng.integers(480, 1000, n), v)
+        v = np.where(k == 2, 0.0 * v, v)
+        v = np.where(k == 3, np.sign(v), v)
+        special = rng.integers(0, n, 6)
+        v[special] = [np.inf, -np.inf, np.nan, 5e-324, 1.7e308, -2.0 ** -1022]
+        return v
+
+    def same(got, want):
+        got, nan = got.cpu().numpy(), np.isnan(want)
+        assert np.array_equal(np.isnan(got), nan) and np.array_equal(bits(got)[~nan], bits(want)[~nan])
+
+    with np.errstate(all="ignore"):
+        T = neon.VolumeField(dm, wild(hm.n * ncomp), rand_bcs(hm, rng, ncomp), ncomp)
+        Th, Tb = T.host(), T.boundary.cpu().numpy()[:hm.nbf * ncomp].copy()
+        flux, gamma = (neon.SurfaceField(dm, wild(hm.nif + hm.nbf)) for _ in range(2))
+        base = rng.standard_normal(hm.n * 3)
+        for scheme in ("linear", "upwind"):
+            want = o.div(neon._scheme(scheme), ncomp, flux.host(), Th, Tb, 1.0, base[:hm.n * ncomp].copy())
+            same(neon.GaussGreenDiv(dm, scheme).div(neon.dev(base[:hm.n * ncomp]), flux, T, 1.0), want)
+        want = o.laplacian(ncomp, gamma.host(), Th, Tb, 1.0, base[:hm.n * ncomp].copy())
+        same(neon.GaussGreenLaplacian(dm).laplacian(neon.dev(base[:hm.n * ncomp]), gamma, T, 1.0), want)
+        same(neon.SurfaceInterpolation(dm, "linear").interpolate(T).values, o.interp_linear(ncomp, Th, Tb))
+        if ncomp == 1:
+            same(neon.GaussGreenGrad(dm).grad(T, 1.0, neon.dev(base)), o.grad(Th, Tb, 1.0, base.copy()))
+            same(neon.FaceNormalGradient(dm).faceNormalGrad(T).values, o.sngrad(Th, Tb))
