@@ -22,9 +22,10 @@
 //    backward z_i = (y_i - sum_j u_ij z_j) / u_ii, each a single sweep over
 //    the rows in level order, fma chains in column order.
 //
-// Each factorization level is one kernel node of the solve's CUDA graph.  Each
-// triangular solve of an application is one launch: rows in level order,
-// each waiting (bounded) for the rows it depends on (the sweeps below).
+// On hex meshes the factorization is a sweep over the rows like a triangular solve,
+// elsewhere each of its levels is one kernel node of the solve's CUDA graph.  A sweep is
+// one launch: rows in level order, each waiting (bounded) for the rows it depends on
+// (the sweeps below).
 // Every row is computed by the same operations in the same order as the
 // sequential restatement (oracle/fvoracle.c or_ilu_*): the bits are those of
 // the exact sequential factorization and solves.  A 128^3 box has 382 levels
@@ -54,7 +55,7 @@ struct IluState {
     double rho, rho_prev, omega;      // BiCGStab
     int32_t iter, status, done, half;
     unsigned counter;
-    unsigned ticket;      // the next chunk of a triangular sweep (0 between launches)
+    unsigned ticket;      // the next part of a triangular sweep (0 between launches)
     int32_t sweep_abort;  // a sweep's wait ran out: the solve ends with FVGB_ERR_CUDA
     fvgb_solver_stats* stats_out;
     fvgb_solver_stats stats;
@@ -198,19 +199,63 @@ __global__ void __launch_bounds__(kT)
 }
 
 // ------------------------------------------------------ triangular sweeps
-// One launch per triangle.  The rows are taken in level order, a chunk of kT
-// rows at a time, by a block ticket: a row depends only on rows of lower
-// levels, which sit earlier in that order, in chunks that blocks already
-// running took before (or in its own block), so every wait ends.  A row's
-// output holds kPending until the row is computed; the one 64-bit store of
-// the value is the signal (relaxed loads and stores at GPU scope, no flag and
-// no fence).  kPending is a signalling NaN: FP64 arithmetic writes quiet NaNs
-// at most, and every value a sweep writes is an arithmetic result.  The
-// forward sweep sets the backward sweep's output to kPending row by row, the
-// backward sweep the forward sweep's output after reading it; the solve graph
-// fills the latter once at its start.
+// One launch per triangle.  The rows are cut into parts of consecutive rows, one part
+// to a block at a time, taken in the sweep's direction by a ticket: a row depends only
+// on rows of its own part and of parts that running blocks took before, so every wait
+// ends.
+//
+// What bounds a sweep is the chain of levels (197 of them for 77 x 64 x 58 cells, 382
+// for 128^3).  Inside a part the levels follow one another through shared memory:
+// teams of W warps take them in turn, a team fetches its next level's rows while the
+// others have theirs, and hands the turn on by a named barrier.  Between parts a value
+// goes through global memory: a row's output holds kPending until the row is computed,
+// and the one 64-bit store of the value is the signal (relaxed at GPU scope, no flag and
+// no fence).  kHaloWarps warps of the block bring the values that the part needs from
+// others into shared memory, in the order in which its rows need them.
+//
+// BiCGStab on 77 x 64 x 58 cells: 6.1 -> 3.2 ms, on 20^3 1.42 -> 0.72, on 128^3 16.1 ->
+// 13.4; before, every value went through L2 (1.6 us a level), and every level of the
+// factorization was a kernel of dependent loads (2.2 of the 6.1 ms, now 0.4).  A level
+// takes 0.4 us inside a part: the barrier 250 clocks, three dependent multiply-adds 200
+// of GB300's FP64; a step to another part 1.3 us.  Rows that poll shared memory without
+// a turn were slower: the polls of the waiting warps take the issue slots and the banks.
+//
+// kPending is a signalling NaN: FP64 arithmetic writes quiet NaNs at most, and every
+// value a sweep writes is an arithmetic result.  The forward sweep sets the backward
+// sweep's output to kPending row by row, the backward sweep the forward sweep's output
+// after reading it; the solve graph fills the latter once at its start.
 constexpr unsigned long long kPending = 0x7ff00000deadbeefull;
-constexpr int kSweepBlocksPerSM = 1;  // 128^3 ILU-CG: 144 ms at 1, 157 at 2
+constexpr int kRowWarps = 16, kHaloWarps = 8;
+constexpr int kSweepThreads = 32 * (kRowWarps + kHaloWarps);
+constexpr int kMaxTeams = 8;   // named barriers 1 .. kMaxTeams
+constexpr int kDeps = 4;       // values a row waits for together; the others one by one
+// Rows of a part: few parts make few trips through L2, and a level of more than 128 rows
+// leaves two teams, which fetch too late.  BiCGStab on 77 x 64 x 58 cells: 3.20 ms with
+// parts of 8,192 rows, 4.06 with 4,096 (levels of up to 128 and 64 rows), 4.05 with
+// 9,600 (up to 140); on 20^3, 0.72 ms with 1,024 and 1.00 in one part (300).
+constexpr int kPart = 8192, kMinPart = 1024, kLevelRows = 128;
+constexpr int kMaxSweepSmem = (3 * kPart + 1) * (int)sizeof(double);
+
+// A triangle's sweep.  Part p has the rows from p * rpp on; its levels are lev[p] to
+// lev[p + 1] - 1, level q its rows rows[32 chunk[q]] to rows[32 chunk[q + 1] - 1] (-1:
+// none), np of them in all.  Of row number t the values it depends on (k < K) are at
+// slot[k np + t]: a place in the part's shared memory (its own rows, then what the halo
+// warps bring), -1 none, below -1 the row -2 - slot read from global memory.
+// val[k np + t]: the factor's entries, filled in every solve; from val[K np + t] on the
+// pivots and their reciprocals (backward) or the matrix's a_ki and a_ii (forward: until
+// the factorization, which reads the matrix's a_ik at val[k np + t], is done).
+struct Sweep {
+    int n, np, rpp, nparts, K, hcap, W;
+    const int* rows;
+    const int* lev;
+    const int* chunk;
+    int* place;        // [n] a row's place in its part's shared memory: its rank in level order
+    const int* off;    // [levels] 32 chunk minus the place of the level's first row
+    int* slot;
+    double* val;
+    int* halo;   // [nparts][hcap] rows of other parts
+    int* nhalo;  // [nparts]
+};
 
 __device__ __forceinline__ bool pending(double v) { return (unsigned long long)__double_as_longlong(v) == kPending; }
 
@@ -258,70 +303,125 @@ __global__ void __launch_bounds__(kT) k_il_pending(int n, double* y) {
     if (i < n) y[i] = __longlong_as_double((long long)kPending);
 }
 
-// out = (s - sum over entries e in [e0, e1) of lu_e v_{col_e}) [/ piv], the
-// sum in entry order over values of this sweep.  The first kDeps values are
-// polled together, and a row stores its value from inside the polling loop as
-// soon as its own values are there: a lane that had left its wait would
-// otherwise hold its store at the warp's reconvergence point until the slowest
-// lane of the warp (a row one level up, or one whose values come from a
-// farther SM) arrived, and every level would wait for the slowest warp lane.
-// Entries past the first kDeps (none on hex meshes) are waited for one by
-// one.  Gives up, raising the abort flag, after about a second (or 2^26
-// polls), or when another wait of the sweep did.
-constexpr int kDeps = 4;
-template <bool DIV>
-__device__ __forceinline__ void sweep_store(IluState* st, const Csr& A, const double* __restrict__ lu, int e0,
-                                            int e1, const double* v, double s, double piv, double* out) {
-    int cj[kDeps];
-    double l[kDeps], x[kDeps];
-#pragma unroll
-    for (int k = 0; k < kDeps; ++k) {
-        x[k] = 0.0;  // not pending
-        if (e0 + k < e1) {
-            cj[k] = __ldg(&A.col[e0 + k]);
-            l[k] = __ldg(&lu[e0 + k]);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < kDeps; ++k)
-        if (e0 + k < e1) x[k] = ld_relaxed(&v[cj[k]]);
-    unsigned long long t0 = 0;
-    for (unsigned it = 0; it < (1u << 26); ++it) {
-        bool ready = true;
-#pragma unroll
-        for (int k = 0; k < kDeps; ++k) ready = ready && !pending(x[k]);
-        if (ready) {
-#pragma unroll
-            for (int k = 0; k < kDeps; ++k)
-                if (e0 + k < e1) s = fma(-l[k], x[k], s);
-            for (int e = e0 + kDeps; e < e1; ++e) {
-                double xe;
-                if (!await_row(&v[__ldg(&A.col[e])], xe, st)) return;
-                s = fma(-__ldg(&lu[e]), xe, s);
-            }
-            st_relaxed(out, DIV ? s / piv : s);
-            return;
-        }
-        if (it == 0) t0 = now_ns();
-        if (it > 2) __nanosleep(it < 16 ? 32 : 256);
-#pragma unroll
-        for (int k = 0; k < kDeps; ++k)
-            if (pending(x[k])) x[k] = ld_relaxed(&v[cj[k]]);
-        if ((it & 31) == 31) {
-            if (*(volatile const int32_t*)&st->sweep_abort) return;
-            if (now_ns() - t0 > 1000000000ull) break;
-        }
-    }
-    atomicExch(&st->sweep_abort, 1);
+// A value of the block's shared memory that another warp reads or writes; a: 32-bit address
+__device__ __forceinline__ double ld_shared(unsigned a) {
+    double v;
+    asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_shared(unsigned a, double v) {
+    asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
-// Chunk of this block (the same in all its threads), or >= nchunks when none is left.
-__device__ __forceinline__ unsigned next_chunk(IluState* st) {
-    __shared__ unsigned chunk;
+// Every row's place in its part's shared memory.  A position's level is the last one
+// that starts at or before it.
+__global__ void __launch_bounds__(kT) k_il_place(Sweep S) {
+    const int t = blockIdx.x * kT + threadIdx.x;
+    const int i = t < S.np ? __ldg(&S.rows[t]) : -1;
+    if (i < 0) return;
+    int a = 0, b = __ldg(&S.lev[S.nparts]);  // chunk[a] <= t / 32 < chunk[b]
+    while (b - a > 1) {
+        const int h = (a + b) / 2;
+        if (__ldg(&S.chunk[h]) <= t / 32) a = h;
+        else b = h;
+    }
+    S.place[i] = t - __ldg(&S.off[a]);
+}
+
+// Where the values that a part's rows depend on are found: one block per part.
+template <bool BWD>
+__global__ void __launch_bounds__(kT) k_il_plan(Csr A, Sweep S) {
+    __shared__ int wsum[kT / 32], base;
+    const int r0 = blockIdx.x * S.rpp, r1 = min(S.n, r0 + S.rpp);
+    const int t1 = 32 * __ldg(&S.chunk[__ldg(&S.lev[blockIdx.x + 1])]);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) base = 0;
     __syncthreads();
-    if (threadIdx.x == 0) chunk = atomicAdd(&st->ticket, 1u);
+    for (int q = 32 * __ldg(&S.chunk[__ldg(&S.lev[blockIdx.x])]); q < t1; q += kT) {
+        const int t = q + threadIdx.x;
+        const int i = t < t1 ? __ldg(&S.rows[t]) : -1;
+        int e0 = 0, e1 = 0, cnt = 0;
+        if (i >= 0) {
+            const int d = __ldg(&A.ro[i]) + __ldg(&A.dof[i]);
+            e0 = BWD ? d + 1 : __ldg(&A.ro[i]);
+            e1 = min(BWD ? __ldg(&A.ro[i + 1]) : d, e0 + S.K);
+            for (int e = e0; e < e1; ++e) {
+                const int c = __ldg(&A.col[e]);
+                cnt += c < r0 || c >= r1;
+            }
+        }
+        int x = cnt;  // inclusive scan
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[w] = x;
+        __syncthreads();
+        int at = base + x - cnt;
+        for (int k = 0; k < w; ++k) at += wsum[k];
+        if (t < t1) {
+            for (int k = 0; k < S.K; ++k) {
+                int sl = -1;
+                if (e0 + k < e1) {
+                    const int c = __ldg(&A.col[e0 + k]);
+                    if (c >= r0 && c < r1) {
+                        sl = __ldg(&S.place[c]);
+                    } else if (at < S.hcap) {
+                        S.halo[(size_t)blockIdx.x * S.hcap + at] = c;
+                        sl = S.rpp + at++;
+                    } else {
+                        sl = -2 - c;
+                    }
+                }
+                S.slot[(size_t)k * S.np + t] = sl;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int k = 0; k < kT / 32; ++k) base += wsum[k];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) S.nhalo[blockIdx.x] = min(base, S.hcap);
+}
+
+enum SweepKind { kFwd = 0, kBwd = 1, kFactor = 2 };
+
+struct Factor {  // of the pivots alone: entry e of the lower triangle updates its row's by a[g[p[e]]]
+    const double* a;
+    double* lu;
+    const int *p, *g;
+};
+
+// A factor's entries (kFwd, kBwd) or the matrix's (kFactor) in the order of a sweep.
+// piv: the pivots row by row when the factorization was a sweep, else null.
+template <int KIND>
+__global__ void __launch_bounds__(kT) k_il_pack(Csr A, Sweep S, Factor F, const double* __restrict__ piv) {
+    const int t = blockIdx.x * kT + threadIdx.x;
+    const int i = t < S.np ? __ldg(&S.rows[t]) : -1;
+    if (i < 0) return;
+    const int b = __ldg(&A.ro[i]), d = b + __ldg(&A.dof[i]);
+    const int e0 = KIND == kBwd ? d + 1 : b, e1 = min(e0 + S.K, KIND == kBwd ? __ldg(&A.ro[i + 1]) : d);
+    for (int e = e0; e < e1; ++e) {
+        double* v = S.val + (size_t)(e - e0) * S.np + t;
+        *v = KIND == kFactor ? __ldg(&F.a[e]) : F.lu[e];
+        if (KIND == kFactor) v[(size_t)S.K * S.np] = __ldg(&F.a[__ldg(&F.g[__ldg(&F.p[e])])]);
+    }
+    if (KIND == kBwd) {
+        const double u = piv ? piv[i] : F.lu[d];
+        S.val[(size_t)S.K * S.np + t] = u;
+        S.val[(size_t)(S.K + 1) * S.np + t] = 1.0 / u;
+    }
+    if (KIND == kFactor) S.val[(size_t)(2 * S.K) * S.np + t] = __ldg(&F.a[d]);
+}
+
+// Part of this block (the same in all its threads), or >= nparts when none is left.
+__device__ __forceinline__ int next_part(IluState* st) {
+    __shared__ unsigned part;
     __syncthreads();
-    return chunk;
+    if (threadIdx.x == 0) part = atomicAdd(&st->ticket, 1u);
+    __syncthreads();
+    return (int)part;
 }
 
 // The last block resets the ticket and ends an aborted solve.
@@ -335,38 +435,230 @@ __device__ __forceinline__ void end_sweep(IluState* st) {
     }
 }
 
-// y_i = r_i - sum_k l_ik y_k, rows in the lower triangle's level order; the
-// backward sweep's output z set to kPending on the way
-__global__ void __launch_bounds__(kT)
-    k_il_fwd(IluState* st, Csr A, const int* __restrict__ rows, unsigned nchunks, const double* __restrict__ lu,
-             const double* __restrict__ r, double* y, double* z) {
-    if (done_flag(st)) return;
-    for (unsigned c = next_chunk(st); c < nchunks; c = next_chunk(st)) {
-        const int t = (int)c * kT + threadIdx.x;
-        if (t >= A.n) continue;
-        const int i = __ldg(&rows[t]);
-        z[i] = __longlong_as_double((long long)kPending);
-        const int b = __ldg(&A.ro[i]), d = b + __ldg(&A.dof[i]);
-        double s = __ldg(&r[i]);
-        sweep_store<false>(st, A, lu, b, d, y, s, 1.0, &y[i]);
+// What a row needs besides the values it depends on, fetched before its turn.
+// kFwd, kBwd: v the entries of the factor; kFactor: v = a_ik, w = a_ki, s = a_ii.
+template <int K>
+struct RowIn {
+    int i, slot[K];
+    double v[K], w[K], s, piv, rcp;
+};
+
+template <int KIND, int K>
+__device__ __forceinline__ void fetch_row(const Sweep& S, const double* src, int t, int i, RowIn<K>& q) {
+    q.i = i;
+#pragma unroll
+    for (int k = 0; k < K; ++k) q.slot[k] = __ldg(&S.slot[(size_t)k * S.np + t]);
+    q.s = q.piv = q.rcp = 1.0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        q.v[k] = q.slot[k] == -1 ? 0.0 : S.val[(size_t)k * S.np + t];
+        if (KIND == kFactor) q.w[k] = q.slot[k] == -1 ? 0.0 : S.val[(size_t)(K + k) * S.np + t];
     }
-    end_sweep(st);
+    if (i < 0) return;
+    if (KIND == kFactor) {
+        q.s = S.val[(size_t)(2 * K) * S.np + t];
+    } else {
+        q.s = __ldcg(&src[i]);
+        if (KIND == kBwd) {
+            q.piv = S.val[(size_t)K * S.np + t];
+            q.rcp = S.val[(size_t)(K + 1) * S.np + t];
+        }
+    }
 }
 
-// z_i = (y_i - sum_j u_ij z_j) / u_ii, rows in the upper triangle's level
-// order; y_i set back to kPending once read
-__global__ void __launch_bounds__(kT)
-    k_il_bwd(IluState* st, Csr A, const int* __restrict__ rows, unsigned nchunks, const double* __restrict__ lu,
-             double* y, double* z) {
-    if (done_flag(st)) return;
-    for (unsigned c = next_chunk(st); c < nchunks; c = next_chunk(st)) {
-        const int t = (int)c * kT + threadIdx.x;
-        if (t >= A.n) continue;
-        const int i = __ldg(&rows[t]);
-        const int d = __ldg(&A.ro[i]) + __ldg(&A.dof[i]), end = __ldg(&A.ro[i + 1]);
-        double s = __ldcg(&y[i]);
-        y[i] = __longlong_as_double((long long)kPending);
-        sweep_store<true>(st, A, lu, d + 1, end, z, s, __ldg(&lu[d]), &z[i]);
+// a / b with y = 1 / b rounded to nearest (Markstein, IBM J. Res. Dev. 34, 1990): the
+// first correction leaves a quotient within an ulp, the second rounds it correctly, as
+// long as nothing over- or underflows.  Five dependent operations where the division
+// takes about twice as many.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const unsigned ea = (unsigned)__double2hiint(a) & 0x7ff00000u, eb = (unsigned)__double2hiint(b) & 0x7ff00000u;
+    const double q0 = a * y;
+    const double q1 = fma(fma(-q0, b, a), y, q0);
+    const double q2 = fma(fma(-q1, b, a), y, q1);
+    // |a| zero or within 2^-600 .. 2^600, |b| within 2^-300 .. 2^300
+    const bool zero = (unsigned long long)__double_as_longlong(a) << 1 == 0;
+    if ((zero || ea - (423u << 20) <= (1200u << 20)) && eb - (723u << 20) <= (600u << 20)) return zero ? q0 : q2;
+    return a / b;
+}
+
+// Waits for the value that a halo warp brings to the shared address a; after an abort it
+// may not be there (the teams keep taking their turns, so that no barrier is left short).
+__device__ __forceinline__ void await_halo(unsigned a, IluState* st) {
+    unsigned long long t0 = 0;
+    for (unsigned it = 1; pending(ld_shared(a)); ++it) {
+        if ((it & 63) != 0) continue;
+        if (it == 64) t0 = now_ns();
+        if (*(volatile const int32_t*)&st->sweep_abort) break;
+        if (it >= (1u << 26) || now_ns() - t0 > 1000000000ull) {
+            atomicExch(&st->sweep_abort, 1);
+            break;
+        }
+    }
+}
+
+// Rows of one level:
+//   kFwd     v_i = src_i - sum_k l_ik v_k
+//   kBwd     v_i = (src_i - sum_j u_ij v_j) / u_ii
+//   kFactor  l_ik = a_ik / v_k, v_i = a_ii - sum_k l_ik a_ki   (v the pivots)
+// the sums in column order.  TURN: the level's turn is still to come; what other parts
+// give is waited for before.  Values that are not there have v = 0 and the slot that
+// holds +0: fma(-0, +0, s) is s.  Entries past the first K, and values for which shared
+// memory had no room (neither on hex meshes), are waited for one by one in global memory.
+template <int KIND, int K, bool TURN>
+__device__ __forceinline__ double sweep_row(IluState* st, const Csr& A, const Sweep& S, const Factor& F,
+                                            const double* lu, unsigned sm, RowIn<K>& q, const double* v, int turn,
+                                            int count) {
+    bool rare = K == kDeps && q.slot[K - 1] != -1;
+    unsigned at[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int sl = q.slot[k];
+        rare = rare || sl < -1;
+        at[k] = sm + 8u * (unsigned)(sl < 0 ? 3 * S.rpp : sl);
+        if (sl >= S.rpp) await_halo(at[k], st);
+    }
+    rare = __any_sync(0xffffffffu, rare);
+    if (TURN) asm volatile("bar.sync %0, %1;" ::"r"(turn), "r"(count) : "memory");
+    double s = q.s, x[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[k] = ld_shared(at[k]);
+    if (rare) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (q.slot[k] < -1) {
+                x[k] = 0.0;
+                await_row(&v[-2 - q.slot[k]], x[k], st);
+            }
+    }
+    if (KIND == kFactor) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (q.slot[k] != -1) q.v[k] = q.v[k] / x[k];
+            x[k] = q.w[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) s = fma(-q.v[k], x[k], s);
+    if (rare && K == kDeps && q.slot[K - 1] != -1) {
+        const int b = __ldg(&A.ro[q.i]), d = b + __ldg(&A.dof[q.i]);
+        const int e1 = KIND == kBwd ? __ldg(&A.ro[q.i + 1]) : d;
+        for (int e = (KIND == kBwd ? d + 1 : b) + kDeps; e < e1; ++e) {
+            double xe = 1.0;
+            await_row(&v[__ldg(&A.col[e])], xe, st);
+            if (KIND == kFactor) {
+                const double l = __ldg(&F.a[e]) / xe;
+                F.lu[e] = l;
+                s = fma(-l, __ldg(&F.a[__ldg(&F.g[__ldg(&F.p[e])])]), s);
+            } else {
+                s = fma(-__ldg(&lu[e]), xe, s);
+            }
+        }
+    }
+    return KIND == kBwd ? div_by(s, q.piv, q.rcp) : s;
+}
+
+// other_i = pending: the backward sweep's output (kFwd), src once read (kBwd).  A wait
+// gives up, raising the abort flag, after about a second (or 2^26 polls), or when
+// another wait of the sweep did.
+template <int KIND, int K>
+__global__ void __launch_bounds__(kSweepThreads)
+    k_il_sweep(IluState* st, Csr A, Sweep S, Factor F, const double* __restrict__ lu, const double* src, double* v,
+               double* other) {
+    extern __shared__ double smem[];
+    const unsigned sm = (unsigned)__cvta_generic_to_shared(smem);
+    if (KIND != kFactor && done_flag(st)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const double unset = __longlong_as_double((long long)kPending);
+    const int T = min(kMaxTeams, kRowWarps / S.W), count = 64 * S.W;
+    if (threadIdx.x == 0) smem[3 * S.rpp] = 0.0;
+    for (int u = next_part(st); u < S.nparts; u = next_part(st)) {
+        const int part = KIND == kBwd ? S.nparts - 1 - u : u;
+        const int nh = __ldg(&S.nhalo[part]);
+        for (int k = threadIdx.x; k < nh; k += kSweepThreads) smem[S.rpp + k] = unset;
+        __syncthreads();
+        if (w >= kRowWarps) {
+            const int* halo = S.halo + (size_t)part * S.hcap;
+            for (int h = (w - kRowWarps) * 32 + lane; h < nh; h += 32 * kHaloWarps) {
+                const double* p = &v[__ldg(&halo[h])];
+                unsigned long long t0 = 0;
+                for (unsigned it = 0;; ++it) {
+                    const double x = ld_relaxed(p);
+                    if (!pending(x)) {
+                        st_shared(sm + 8u * (unsigned)(S.rpp + h), x);
+                        break;
+                    }
+                    if (it == 0) t0 = now_ns();
+                    if (it > 2) __nanosleep(20);
+                    if ((it & 31) == 31) {
+                        if (*(volatile const int32_t*)&st->sweep_abort) break;
+                        if (it >= (1u << 26) || now_ns() - t0 > 1000000000ull) {
+                            atomicExch(&st->sweep_abort, 1);
+                            break;
+                        }
+                    }
+                }
+            }
+        } else if (w < T * S.W) {
+            const int team = w / S.W, tw = w % S.W;
+            const int l0 = __ldg(&S.lev[part]), l1 = __ldg(&S.lev[part + 1]);
+            // chunks [c, ce) of this warp's level, its rows fetched; [n, ne) of the one after, i the first's rows
+            RowIn<K> q;
+            int c, ce, co, n, ne, no, i = -1;
+            const auto level = [&](int l, int& a, int& b, int& o) {
+                a = b = o = 0;
+                if (l < l1) {
+                    a = __ldg(&S.chunk[l]) + tw;
+                    b = __ldg(&S.chunk[l + 1]);
+                    o = __ldg(&S.off[l]);
+                }
+            };
+            level(l0 + team, c, ce, co);
+            level(l0 + team + T, n, ne, no);
+            if (c < ce) fetch_row<KIND>(S, src, 32 * c + lane, __ldg(&S.rows[32 * c + lane]), q);
+            if (n < ne) i = __ldg(&S.rows[32 * n + lane]);
+            for (int l = l0 + team; l < l1; l += T) {
+                int n2, n2e, n2o;
+                level(l + 2 * T, n2, n2e, n2o);
+                const int turn = 1 + team, next = 1 + (team + 1) % T;
+                if (c < ce) {
+                    double z = l > l0 ? sweep_row<KIND, K, true>(st, A, S, F, lu, sm, q, v, turn, count)
+                                      : sweep_row<KIND, K, false>(st, A, S, F, lu, sm, q, v, turn, count);
+                    for (;;) {
+                        if (q.i >= 0) st_shared(sm + 8u * (unsigned)(32 * c + lane - co), z);
+                        const int cd = c;
+                        c += S.W;
+                        if (c >= ce) {
+                            __syncwarp();
+                            if (l + 1 < l1)
+                                asm volatile("bar.arrive %0, %1;" ::"r"(next), "r"(count) : "memory");
+                        }
+                        if (q.i >= 0) {
+                            st_relaxed(&v[q.i], z);
+                            if (KIND != kFactor) other[q.i] = unset;
+                            if (KIND == kFactor) {
+#pragma unroll
+                                for (int k = 0; k < K; ++k)
+                                    if (q.slot[k] != -1) S.val[(size_t)k * S.np + 32 * cd + lane] = q.v[k];
+                            }
+                        }
+                        if (c >= ce) break;
+                        fetch_row<KIND>(S, src, 32 * c + lane, __ldg(&S.rows[32 * c + lane]), q);
+                        z = sweep_row<KIND, K, false>(st, A, S, F, lu, sm, q, v, 0, 0);
+                    }
+                } else {
+                    if (l > l0) asm volatile("bar.sync %0, %1;" ::"r"(turn), "r"(count) : "memory");
+                    if (l + 1 < l1) asm volatile("bar.arrive %0, %1;" ::"r"(next), "r"(count) : "memory");
+                }
+                c = n;
+                ce = ne;
+                co = no;
+                n = n2;
+                ne = n2e;
+                no = n2o;
+                if (c < ce) fetch_row<KIND>(S, src, 32 * c + lane, i, q);
+                if (n < ne) i = __ldg(&S.rows[32 * n + lane]);
+            }
+        }
     }
     end_sweep(st);
 }
@@ -683,10 +975,13 @@ struct IluCache {
     const fvgb_ls* ls = nullptr;
     int n = 0, nnz = 0, R = 4, nb = 1;
     unsigned sweep_grid = 1;  // resident blocks of a triangular sweep
+    int sweep_smem = 0;
+    bool pivots_only = true;  // the factorization changes the lower triangle and the diagonal alone (hex meshes)
+    Sweep fwd{}, bwd{};
     int *ro = nullptr, *col = nullptr, *dof = nullptr;
     int *op_ptr = nullptr, *op_f = nullptr, *op_g = nullptr;
-    int *fwd_rows = nullptr, *bwd_rows = nullptr;
-    std::vector<int> fwd_ptr, bwd_ptr;  // level offsets into fwd_rows / bwd_rows (host)
+    int* lev_rows = nullptr;   // rows by level of the lower triangle
+    std::vector<int> fwd_ptr;  // level offsets into it (host)
     double *a = nullptr, *lu = nullptr;
     double *r = nullptr, *rr = nullptr, *p = nullptr, *q = nullptr, *v = nullptr, *y = nullptr, *z = nullptr,
            *s = nullptr, *t = nullptr, *w = nullptr, *pa = nullptr, *pb = nullptr;
@@ -696,6 +991,8 @@ struct IluCache {
 };
 
 namespace {
+
+unsigned grid_of(int count) { return count > 0 ? (unsigned)((count + kT - 1) / kT) : 1u; }
 
 template <class T>
 cudaError_t il_alloc(IluCache* c, T** p, size_t count) {
@@ -722,6 +1019,70 @@ void by_level(const std::vector<int>& lev, std::vector<int>& ptr, std::vector<in
     for (int i = 0; i < (int)lev.size(); ++i) rows[(size_t)at[(size_t)lev[(size_t)i]]++] = i;
 }
 
+// Rows of a part: the most, halving from kPart to kMinPart, of which a level has no
+// more than kLevelRows in a part from the middle.
+int part_rows(const std::vector<int>& level) {
+    const int n = (int)level.size();
+    int rpp = kPart;
+    for (std::vector<int> cnt; rpp > kMinPart; rpp /= 2) {
+        const int r0 = (n / 2) / rpp * rpp, r1 = std::min(n, r0 + rpp);
+        const auto mm = std::minmax_element(level.begin() + r0, level.begin() + r1);
+        if (r0 >= r1) break;
+        cnt.assign((size_t)(*mm.second - *mm.first + 1), 0);
+        for (int i = r0; i < r1; ++i) ++cnt[(size_t)(level[(size_t)i] - *mm.first)];
+        if (*std::max_element(cnt.begin(), cnt.end()) <= kLevelRows) break;
+    }
+    return rpp;
+}
+
+// The order of a sweep from the rows' levels: by part, by level, each level filled up to
+// whole warps.
+cudaError_t il_sweep(IluCache* c, Sweep& S, const std::vector<int>& level) {
+    std::vector<int> rows, lev(1, 0), chunk, off, at;
+    rows.reserve((size_t)S.n * 5 / 4);
+    int most = 0;  // chunks of the largest level
+    for (int p = 0; p < S.nparts; ++p) {
+        const int r0 = p * S.rpp, r1 = std::min(S.n, r0 + S.rpp);
+        const auto mm = std::minmax_element(level.begin() + r0, level.begin() + r1);
+        const int lo = *mm.first, nl = *mm.second - lo + 1;
+        at.assign((size_t)nl, 0);
+        for (int i = r0; i < r1; ++i) ++at[(size_t)(level[(size_t)i] - lo)];
+        int end = (int)rows.size(), place = 0;
+        for (int& a : at) {
+            const int cnt = a;
+            a = end;
+            if (cnt == 0) continue;
+            chunk.push_back(end / 32);
+            off.push_back(end - place);
+            place += cnt;
+            end += (cnt + 31) / 32 * 32;
+            most = std::max(most, (cnt + 31) / 32);
+        }
+        rows.resize((size_t)end, -1);
+        for (int i = r0; i < r1; ++i) rows[(size_t)at[(size_t)(level[(size_t)i] - lo)]++] = i;
+        lev.push_back((int)chunk.size());
+    }
+    chunk.push_back((int)(rows.size() / 32));
+    S.np = (int)rows.size();
+    S.W = 1;
+    while (S.W < most && S.W < kRowWarps / 2) S.W *= 2;
+    int *r = nullptr, *lv = nullptr, *ch = nullptr, *of = nullptr;
+    cudaError_t e = il_upload(c, &r, rows);
+    if (e == cudaSuccess) e = il_upload(c, &lv, lev);
+    if (e == cudaSuccess) e = il_upload(c, &ch, chunk);
+    if (e == cudaSuccess) e = il_alloc(c, &S.place, (size_t)S.n);
+    if (e == cudaSuccess) e = il_upload(c, &of, off);
+    S.rows = r;
+    S.off = of;
+    S.lev = lv;
+    S.chunk = ch;
+    if (e == cudaSuccess) e = il_alloc(c, &S.slot, (size_t)S.K * S.np);
+    if (e == cudaSuccess) e = il_alloc(c, &S.val, (size_t)(2 * S.K + 1) * S.np);
+    if (e == cudaSuccess) e = il_alloc(c, &S.halo, (size_t)S.nparts * S.hcap);
+    if (e == cudaSuccess) e = il_alloc(c, &S.nhalo, (size_t)S.nparts);
+    return e;
+}
+
 fvgb_status symbolic(IluCache* c) {
     const fvgb_mesh* m = c->ls->mesh;
     const int n = m->v.n, nnz = m->nnz;
@@ -731,8 +1092,13 @@ fvgb_status symbolic(IluCache* c) {
     const std::vector<int32_t>& col = m->h_col;
     const std::vector<int32_t>& dof = m->h_diag_off;
     std::vector<int> op_ptr((size_t)nnz + 1, 0), op_f, op_g, lev_f((size_t)n, 0), lev_b((size_t)n, 0);
+    op_f.reserve((size_t)(nnz - n) / 2);
+    op_g.reserve((size_t)(nnz - n) / 2);
+    int maxl = 0, maxu = 0;
     for (int i = 0; i < n; ++i) {
         const int d = ro[i] + dof[i], end = ro[i + 1];
+        maxl = std::max(maxl, d - ro[i]);
+        maxu = std::max(maxu, end - d - 1);
         for (int e = ro[i]; e < end; ++e) {
             if (e < d) {
                 const int k = col[e];
@@ -748,36 +1114,46 @@ fvgb_status symbolic(IluCache* c) {
                 }
             }
             op_ptr[(size_t)e + 1] = (int)op_f.size();
+            if (e < d && (op_ptr[(size_t)e + 1] != op_ptr[(size_t)e] + 1 || op_f.back() != d)) c->pivots_only = false;
         }
     }
     for (int i = n - 1; i >= 0; --i)
         for (int e = ro[i] + dof[i] + 1; e < ro[i + 1]; ++e) lev_b[i] = std::max(lev_b[i], lev_b[col[e]] + 1);
-    std::vector<int> fwd_rows, bwd_rows;
-    by_level(lev_f, c->fwd_ptr, fwd_rows);
-    by_level(lev_b, c->bwd_ptr, bwd_rows);
+    std::vector<int> lev_rows;
+    if (!c->pivots_only) by_level(lev_f, c->fwd_ptr, lev_rows);
     c->n = n;
     c->nnz = nnz;
     c->R = n >= (1 << 15) ? 8 : 4;
     c->nb = std::max(1, (n + kT * c->R - 1) / (kT * c->R));
-    {
-        // the sweep's blocks stay resident (a persistent grid taking chunks);
-        // one per SM keeps the rows at the wavefront busy, and more rows in
-        // flight only add polls of rows far behind it
-        int dev = 0, sms = 1, per = 1;
-        FVGB_CUDA_TRY(cudaGetDevice(&dev));
-        FVGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        FVGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_il_fwd, kT, 0));
-        const long chunks = (n + kT - 1) / kT;
-        c->sweep_grid = (unsigned)std::max(1L, std::min(chunks, (long)sms * std::min(per, kSweepBlocksPerSM)));
-    }
+    int dev = 0, sms = 1;
+    FVGB_CUDA_TRY(cudaGetDevice(&dev));
+    FVGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int rpp = std::min((n + 31) / 32 * 32, std::max(32, part_rows(lev_f)));
+    const int nparts = (n + rpp - 1) / rpp;
+    c->sweep_grid = (unsigned)std::max(1, std::min(nparts, sms));
+    const auto setup = [&](Sweep& S, int deps) {
+        S.n = n;
+        S.rpp = rpp;
+        S.nparts = nparts;
+        S.K = deps < kDeps ? kDeps - 1 : kDeps;
+        S.hcap = 2 * rpp;  // a row of a hex mesh needs one value of another part, or two
+    };
+    setup(c->fwd, maxl);
+    setup(c->bwd, maxu);
+    c->sweep_smem = (int)sizeof(double) * (3 * rpp + 1);
+    for (const void* f : {(const void*)k_il_sweep<kFwd, kDeps - 1>, (const void*)k_il_sweep<kFwd, kDeps>,
+                          (const void*)k_il_sweep<kBwd, kDeps - 1>, (const void*)k_il_sweep<kBwd, kDeps>,
+                          (const void*)k_il_sweep<kFactor, kDeps - 1>, (const void*)k_il_sweep<kFactor, kDeps>})
+        FVGB_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSweepSmem));
     cudaError_t e = il_upload(c, &c->ro, ro);
     if (e == cudaSuccess) e = il_upload(c, &c->col, col);
     if (e == cudaSuccess) e = il_upload(c, &c->dof, dof);
     if (e == cudaSuccess) e = il_upload(c, &c->op_ptr, op_ptr);
-    if (e == cudaSuccess) e = il_upload(c, &c->op_f, op_f);
+    if (e == cudaSuccess && !c->pivots_only) e = il_upload(c, &c->op_f, op_f);
     if (e == cudaSuccess) e = il_upload(c, &c->op_g, op_g);
-    if (e == cudaSuccess) e = il_upload(c, &c->fwd_rows, fwd_rows);
-    if (e == cudaSuccess) e = il_upload(c, &c->bwd_rows, bwd_rows);
+    if (e == cudaSuccess && !c->pivots_only) e = il_upload(c, &c->lev_rows, lev_rows);
+    if (e == cudaSuccess) e = il_sweep(c, c->fwd, lev_f);
+    if (e == cudaSuccess) e = il_sweep(c, c->bwd, lev_b);
     if (e == cudaSuccess) e = il_alloc(c, &c->a, (size_t)nnz);
     if (e == cudaSuccess) e = il_alloc(c, &c->lu, (size_t)nnz);
     double** vecs[] = {&c->r, &c->rr, &c->p, &c->q, &c->v, &c->y, &c->z, &c->s, &c->t, &c->w};
@@ -788,6 +1164,13 @@ fvgb_status symbolic(IluCache* c) {
     if (e == cudaSuccess) e = il_alloc(c, &c->st, 1);
     if (e == cudaSuccess) e = cudaMemset(c->st, 0, sizeof(IluState));
     if (e != cudaSuccess) return cuda_fail(e, "ILU setup");
+    const Csr A{n, c->ro, c->col, c->dof};
+    if (n > 0) {
+        for (const Sweep& S : {c->fwd, c->bwd}) k_il_place<<<grid_of(S.np), kT>>>(S);
+        k_il_plan<false><<<nparts, kT>>>(A, c->fwd);
+        k_il_plan<true><<<nparts, kT>>>(A, c->bwd);
+        FVGB_LAUNCH_CHECK("ILU plan");
+    }
     FVGB_CUDA_TRY(settle_creation());
     return FVGB_OK;
 }
@@ -799,6 +1182,7 @@ struct Chain {
     cudaGraphNode_t prev = nullptr;
     bool has_prev = false;
     cudaError_t e = cudaSuccess;
+    int smem = 0;  // of a sweep, which has a block size of its own
 
     template <class... A>
     void add(void* fn, unsigned grid, A... args) {
@@ -807,7 +1191,8 @@ struct Chain {
         cudaKernelNodeParams kp{};
         kp.func = fn;
         kp.gridDim = dim3(grid);
-        kp.blockDim = dim3(fn == (void*)k_il_cond || fn == (void*)k_il_stats ? 1 : kT);
+        kp.blockDim = dim3(fn == (void*)k_il_cond || fn == (void*)k_il_stats ? 1 : smem ? kSweepThreads : kT);
+        kp.sharedMemBytes = (unsigned)smem;
         kp.kernelParams = params;
         cudaGraphNode_t node;
         e = cudaGraphAddKernelNode(&node, g, has_prev ? &prev : nullptr, has_prev ? 1 : 0, &kp);
@@ -818,15 +1203,20 @@ struct Chain {
     }
 };
 
-unsigned grid_of(int count) { return count > 0 ? (unsigned)((count + kT - 1) / kT) : 1u; }
+template <int KIND>
+void add_sweep(IluCache* c, Chain& ch, const Sweep& S, const double* src, double* v, double* other) {
+    const Csr A{c->n, c->ro, c->col, c->dof};
+    const Factor F{c->a, c->lu, c->op_ptr, c->op_g};
+    ch.smem = c->sweep_smem;
+    ch.add(S.K == kDeps ? (void*)k_il_sweep<KIND, kDeps> : (void*)k_il_sweep<KIND, kDeps - 1>, c->sweep_grid, c->st, A,
+           S, F, (const double*)c->lu, src, v, other);
+    ch.smem = 0;
+}
 
 // z = U^-1 L^-1 src through c->w: a forward and a backward sweep
 void add_apply(IluCache* c, Chain& ch, const double* src, double* dst) {
-    const Csr A{c->n, c->ro, c->col, c->dof};
-    const unsigned nchunks = (unsigned)((c->n + kT - 1) / kT);
-    const double* lu = c->lu;
-    ch.add((void*)k_il_fwd, c->sweep_grid, c->st, A, (const int*)c->fwd_rows, nchunks, lu, src, c->w, dst);
-    ch.add((void*)k_il_bwd, c->sweep_grid, c->st, A, (const int*)c->bwd_rows, nchunks, lu, c->w, dst);
+    add_sweep<kFwd>(c, ch, c->fwd, src, c->w, dst);
+    add_sweep<kBwd>(c, ch, c->bwd, c->w, dst, c->w);
 }
 
 fvgb_status build_graph(IluCache* c, bool bicgstab) {
@@ -848,11 +1238,20 @@ fvgb_status build_graph(IluCache* c, bool bicgstab) {
     ch.add((void*)k_il_pending, ng, n, c->w);  // the forward sweeps' output, pending
     ch.add((void*)k_il_gather, grid_of(c->nnz), c->nnz, (const int*)ls->mesh->csr_pos, (const double*)ls->values,
            c->a, c->lu);
-    for (size_t l = 0; l + 1 < c->fwd_ptr.size(); ++l) {
-        const int cnt = c->fwd_ptr[l + 1] - c->fwd_ptr[l];
-        ch.add((void*)k_il_factor, grid_of(cnt), A, (const int*)(c->fwd_rows + c->fwd_ptr[l]), cnt,
-               (const int*)c->op_ptr, (const int*)c->op_f, (const int*)c->op_g, c->lu);
+    const Factor F{c->a, c->lu, c->op_ptr, c->op_g};
+    if (c->pivots_only) {
+        ch.add((void*)k_il_pending, ng, n, c->t);
+        ch.add((void*)k_il_pack<kFactor>, grid_of(c->fwd.np), A, c->fwd, F, (const double*)nullptr);
+        add_sweep<kFactor>(c, ch, c->fwd, c->a, c->t, c->t);
+    } else {
+        for (size_t l = 0; l + 1 < c->fwd_ptr.size(); ++l) {
+            const int cnt = c->fwd_ptr[l + 1] - c->fwd_ptr[l];
+            ch.add((void*)k_il_factor, grid_of(cnt), A, (const int*)(c->lev_rows + c->fwd_ptr[l]), cnt,
+                   (const int*)c->op_ptr, (const int*)c->op_f, (const int*)c->op_g, c->lu);
+        }
     }
+    if (!c->pivots_only) ch.add((void*)k_il_pack<kFwd>, grid_of(c->fwd.np), A, c->fwd, F, (const double*)nullptr);
+    ch.add((void*)k_il_pack<kBwd>, grid_of(c->bwd.np), A, c->bwd, F, (const double*)(c->pivots_only ? c->t : nullptr));
     if (!bicgstab) {
         ch.add((void*)k_ic_init, nb, st, A, R, a, b, c->r, c->pa);
         add_apply(c, ch, c->r, c->z);

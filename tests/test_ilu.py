@@ -303,3 +303,43 @@ def test_ilu_on_reference_meshes_vs_oracle(cuda, case):
         xo = T.host().copy()
         so = o.solve(v, r, xo, rel_tol=1e-12, max_iter=500, method=om, preconditioner=2)
         same(st, so, x, xo)
+
+
+def shuffled(hm, seed):
+    """The mesh with its cells in random order: few and wide levels, rows of up to six
+    earlier neighbours, nearly all of them in other parts of a sweep."""
+    perm = np.random.default_rng(seed).permutation(hm.n).astype(np.int32)  # new number of each cell
+    own, nei = perm[hm.own], perm[hm.nei]
+    flip = own > nei
+    own, nei = np.where(flip, nei, own), np.where(flip, own, nei)
+    order = np.lexsort((nei, own))
+    sign = np.where(flip, -1.0, 1.0)[order]
+    vec = lambda a: np.ascontiguousarray(a.reshape(-1, 3)[order])  # noqa: E731
+    inv = np.argsort(perm)
+    return dataclasses.replace(hm, own=own[order].astype(np.int32), nei=nei[order].astype(np.int32),
+                               Sf=vec(hm.Sf) * sign[:, None], Cf=vec(hm.Cf), magSf=hm.magSf[order],
+                               w=np.where(flip, 1.0 - hm.w, hm.w)[order], delta=hm.delta[order],
+                               V=hm.V[inv].copy(), C=np.ascontiguousarray(hm.C.reshape(-1, 3)[inv]),
+                               bcells=perm[hm.bcells].astype(np.int32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", [
+    lambda: mesh.box(2, 2, 2),                          # one level per warp and less
+    lambda: mesh.box(16, 8, 8, jitter=0.1, seed=1),     # 1,024 rows: one part
+    lambda: mesh.box(41, 5, 5, jitter=0.1, seed=1),     # 1,025
+    lambda: mesh.box(20, 20, 20, jitter=0.1, seed=1),   # levels of 300 rows: parts of 1,024
+    lambda: mesh.box(128, 65, 1, jitter=0.1, seed=1),   # 8,320 rows, two parts
+    lambda: mesh.box(64, 60, 5, jitter=0.1, seed=1),    # 19,200
+    lambda: mesh.box(1500, 3, 2, jitter=0.1, seed=1),   # more levels than a part's rows have warps
+    lambda: diag_mesh(131, 90),                         # fill updates: factored level by level
+    lambda: shuffled(mesh.box(24, 22, 20, jitter=0.1, seed=1), 4),  # direct reads, rows of more than four
+], ids=["2x2x2", "1024", "1025", "cube", "two_parts", "slab", "thin", "fill", "shuffled"])
+def test_ilu_sweeps_by_parts_and_levels(cuda, make):
+    hm = make()
+    for kind, method, om in (("heat", abi.SOLVER_CG, 0), ("convection", abi.SOLVER_BICGSTAB, 1)):
+        T, o, ls, v, r = gpu_system(hm, kind)
+        x, xo = T.internal.clone(), T.host().copy()
+        st = ls.solve(x, rel_tol=1e-9, max_iter=2000, method=method, preconditioner=abi.PRECOND_ILU)
+        so = o.solve(v, r, xo, rel_tol=1e-9, max_iter=2000, method=om, preconditioner=2)
+        same(st, so, x, xo)
