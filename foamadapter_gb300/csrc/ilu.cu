@@ -211,10 +211,11 @@ __global__ void __launch_bounds__(kT)
 // goes through global memory: a row's output holds kPending until the row is computed,
 // and the one 64-bit store of the value is the signal (relaxed at GPU scope, no flag and
 // no fence).  kHaloWarps warps of the block bring the values that the part needs from
-// others into shared memory, in the order in which its rows need them.
+// others into shared memory, in the order in which its rows need them; on large systems
+// (kDirectRows) the row warps read them themselves.
 //
-// BiCGStab on 77 x 64 x 58 cells: 6.1 -> 3.2 ms, on 20^3 1.42 -> 0.72, on 128^3 16.1 ->
-// 13.4; before, every value went through L2 (1.6 us a level), and every level of the
+// BiCGStab on 77 x 64 x 58 cells: 6.1 -> 3.1 ms, on 20^3 1.42 -> 0.70, on 128^3 16.1 ->
+// 12.0; before, every value went through L2 (1.6 us a level), and every level of the
 // factorization was a kernel of dependent loads (2.2 of the 6.1 ms, now 0.4).  A level
 // takes 0.4 us inside a part: the barrier 250 clocks, three dependent multiply-adds 200
 // of GB300's FP64; a step to another part 1.3 us.  Rows that poll shared memory without
@@ -234,6 +235,12 @@ constexpr int kDeps = 4;       // values a row waits for together; the others on
 // parts of 8,192 rows, 4.06 with 4,096 (levels of up to 128 and 64 rows), 4.05 with
 // 9,600 (up to 140); on 20^3, 0.72 ms with 1,024 and 1.00 in one part (300).
 constexpr int kPart = 8192, kMinPart = 1024, kLevelRows = 128;
+// From this size on the row warps read the rows of other parts themselves, before their
+// turn, and two blocks share an SM: with a halo in shared memory one part of 8,192 rows
+// fills it, and 128^3 has 256 parts.  ILU-CG on 128^3 cells 156 ms with halo warps and 121
+// without (145 with every step through L2), 96^3 86.7 and 72.0, 64^3 22.3 and 18.8;
+// BiCGStab on 48^3 2.16 and 2.24 ms, on 80 x 80 x 9 1.84 and 2.11.
+constexpr int kDirectRows = 1 << 18;
 constexpr int kMaxSweepSmem = (3 * kPart + 1) * (int)sizeof(double);
 
 // A triangle's sweep.  Part p has the rows from p * rpp on; its levels are lev[p] to
@@ -504,25 +511,34 @@ __device__ __forceinline__ void await_halo(unsigned a, IluState* st) {
 // give is waited for before.  Values that are not there have v = 0 and the slot that
 // holds +0: fma(-0, +0, s) is s.  Entries past the first K, and values for which shared
 // memory had no room (neither on hex meshes), are waited for one by one in global memory.
-template <int KIND, int K, bool TURN>
+template <int KIND, int K, bool DIRECT, bool TURN>
 __device__ __forceinline__ double sweep_row(IluState* st, const Csr& A, const Sweep& S, const Factor& F,
                                             const double* lu, unsigned sm, RowIn<K>& q, const double* v, int turn,
                                             int count) {
     bool rare = K == kDeps && q.slot[K - 1] != -1;
     unsigned at[K];
+    double x[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         const int sl = q.slot[k];
-        rare = rare || sl < -1;
-        at[k] = sm + 8u * (unsigned)(sl < 0 ? 3 * S.rpp : sl);
-        if (sl >= S.rpp) await_halo(at[k], st);
+        at[k] = sm + 8u * (unsigned)(sl < 0 ? S.rpp + S.hcap : sl);
+        if (DIRECT) {
+            x[k] = 0.0;
+            if (sl < -1) await_row(&v[-2 - sl], x[k], st);
+        } else {
+            rare = rare || sl < -1;
+            if (sl >= S.rpp) await_halo(at[k], st);
+        }
     }
     rare = __any_sync(0xffffffffu, rare);
     if (TURN) asm volatile("bar.sync %0, %1;" ::"r"(turn), "r"(count) : "memory");
-    double s = q.s, x[K];
+    double s = q.s;
 #pragma unroll
-    for (int k = 0; k < K; ++k) x[k] = ld_shared(at[k]);
-    if (rare) {
+    for (int k = 0; k < K; ++k) {
+        const double y = ld_shared(at[k]);
+        x[k] = DIRECT && q.slot[k] < -1 ? x[k] : y;
+    }
+    if (!DIRECT && rare) {
 #pragma unroll
         for (int k = 0; k < K; ++k)
             if (q.slot[k] < -1) {
@@ -557,10 +573,11 @@ __device__ __forceinline__ double sweep_row(IluState* st, const Csr& A, const Sw
     return KIND == kBwd ? div_by(s, q.piv, q.rcp) : s;
 }
 
+// DIRECT: no halo (hcap 0), the row warps read the rows of other parts themselves.
 // other_i = pending: the backward sweep's output (kFwd), src once read (kBwd).  A wait
 // gives up, raising the abort flag, after about a second (or 2^26 polls), or when
 // another wait of the sweep did.
-template <int KIND, int K>
+template <int KIND, int K, bool DIRECT>
 __global__ void __launch_bounds__(kSweepThreads)
     k_il_sweep(IluState* st, Csr A, Sweep S, Factor F, const double* __restrict__ lu, const double* src, double* v,
                double* other) {
@@ -570,7 +587,7 @@ __global__ void __launch_bounds__(kSweepThreads)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const double unset = __longlong_as_double((long long)kPending);
     const int T = min(kMaxTeams, kRowWarps / S.W), count = 64 * S.W;
-    if (threadIdx.x == 0) smem[3 * S.rpp] = 0.0;
+    if (threadIdx.x == 0) smem[S.rpp + S.hcap] = 0.0;
     for (int u = next_part(st); u < S.nparts; u = next_part(st)) {
         const int part = KIND == kBwd ? S.nparts - 1 - u : u;
         const int nh = __ldg(&S.nhalo[part]);
@@ -621,8 +638,8 @@ __global__ void __launch_bounds__(kSweepThreads)
                 level(l + 2 * T, n2, n2e, n2o);
                 const int turn = 1 + team, next = 1 + (team + 1) % T;
                 if (c < ce) {
-                    double z = l > l0 ? sweep_row<KIND, K, true>(st, A, S, F, lu, sm, q, v, turn, count)
-                                      : sweep_row<KIND, K, false>(st, A, S, F, lu, sm, q, v, turn, count);
+                    double z = l > l0 ? sweep_row<KIND, K, DIRECT, true>(st, A, S, F, lu, sm, q, v, turn, count)
+                                      : sweep_row<KIND, K, DIRECT, false>(st, A, S, F, lu, sm, q, v, turn, count);
                     for (;;) {
                         if (q.i >= 0) st_shared(sm + 8u * (unsigned)(32 * c + lane - co), z);
                         const int cd = c;
@@ -643,7 +660,7 @@ __global__ void __launch_bounds__(kSweepThreads)
                         }
                         if (c >= ce) break;
                         fetch_row<KIND>(S, src, 32 * c + lane, __ldg(&S.rows[32 * c + lane]), q);
-                        z = sweep_row<KIND, K, false>(st, A, S, F, lu, sm, q, v, 0, 0);
+                        z = sweep_row<KIND, K, DIRECT, false>(st, A, S, F, lu, sm, q, v, 0, 0);
                     }
                 } else {
                     if (l > l0) asm volatile("bar.sync %0, %1;" ::"r"(turn), "r"(count) : "memory");
@@ -997,6 +1014,13 @@ namespace {
 
 unsigned grid_of(int count) { return count > 0 ? (unsigned)((count + kT - 1) / kT) : 1u; }
 
+template <int KIND>
+const void* sweep_fn(const Sweep& S) {
+    if (S.hcap == 0)
+        return S.K == kDeps ? (const void*)k_il_sweep<KIND, kDeps, true> : (const void*)k_il_sweep<KIND, kDeps - 1, true>;
+    return S.K == kDeps ? (const void*)k_il_sweep<KIND, kDeps, false> : (const void*)k_il_sweep<KIND, kDeps - 1, false>;
+}
+
 template <class T>
 cudaError_t il_alloc(IluCache* c, T** p, size_t count) {
     cudaError_t e = cudaMalloc((void**)p, sizeof(T) * (count ? count : 1));
@@ -1133,20 +1157,18 @@ fvgb_status symbolic(IluCache* c) {
     FVGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int rpp = std::min((n + 31) / 32 * 32, std::max(32, part_rows(lev_f)));
     const int nparts = (n + rpp - 1) / rpp;
-    c->sweep_grid = (unsigned)std::max(1, std::min(nparts, sms));
+    c->sweep_grid = (unsigned)std::max(1, std::min(nparts, n >= kDirectRows ? 2 * sms : sms));
     const auto setup = [&](Sweep& S, int deps) {
         S.n = n;
         S.rpp = rpp;
         S.nparts = nparts;
         S.K = deps < kDeps ? kDeps - 1 : kDeps;
-        S.hcap = 2 * rpp;  // a row of a hex mesh needs one value of another part, or two
+        S.hcap = n >= kDirectRows ? 0 : 2 * rpp;  // a row of a hex mesh needs one value of another part, or two
     };
     setup(c->fwd, maxl);
     setup(c->bwd, maxu);
-    c->sweep_smem = (int)sizeof(double) * (3 * rpp + 1);
-    for (const void* f : {(const void*)k_il_sweep<kFwd, kDeps - 1>, (const void*)k_il_sweep<kFwd, kDeps>,
-                          (const void*)k_il_sweep<kBwd, kDeps - 1>, (const void*)k_il_sweep<kBwd, kDeps>,
-                          (const void*)k_il_sweep<kFactor, kDeps - 1>, (const void*)k_il_sweep<kFactor, kDeps>})
+    c->sweep_smem = (int)sizeof(double) * (rpp + c->fwd.hcap + 1);
+    for (const void* f : {sweep_fn<kFwd>(c->fwd), sweep_fn<kBwd>(c->bwd), sweep_fn<kFactor>(c->fwd)})
         FVGB_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSweepSmem));
     cudaError_t e = il_upload(c, &c->ro, ro);
     if (e == cudaSuccess) e = il_upload(c, &c->col, col);
@@ -1211,8 +1233,7 @@ void add_sweep(IluCache* c, Chain& ch, const Sweep& S, const double* src, double
     const Csr A{c->n, c->ro, c->col, c->dof};
     const Factor F{c->a, c->lu, c->op_ptr, c->op_g};
     ch.smem = c->sweep_smem;
-    ch.add(S.K == kDeps ? (void*)k_il_sweep<KIND, kDeps> : (void*)k_il_sweep<KIND, kDeps - 1>, c->sweep_grid, c->st, A,
-           S, F, (const double*)c->lu, src, v, other);
+    ch.add((void*)sweep_fn<KIND>(S), c->sweep_grid, c->st, A, S, F, (const double*)c->lu, src, v, other);
     ch.smem = 0;
 }
 

@@ -24,9 +24,12 @@
 // condition (any case still active), so there is no host round trip per
 // iteration.  Every loop is bounded by an iteration cap.
 //
+// Small and medium single cases run in one kernel instead (resident.cuh): one cluster
+// up to 4,096 rows, one block per SM with the matrix in shared memory while it fits.
+//
 // Reductions are deterministic.  Block b of case c owns rows
 // row0_b + (t/32)*32R + j*32 + t%32 (thread t, j < R = rows_per_thread(case rows)); a
-// thread sums its rows sequentially, warp 0 sums the 256 partials (lane l:
+// thread sums its rows sequentially, one warp sums the 256 partials (lane l:
 // l, l+32, ..., l+224) and a xor butterfly finishes; the last block of the case
 // to arrive sums the case's block partials in index order with the same tree.
 // The CPU oracle reproduces this tree, so the FP64 iterates match it bit for

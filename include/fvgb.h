@@ -208,9 +208,11 @@ fvgb_status fvgb_advect_euler_step(const fvgb_mesh* mesh, const double* flux,
                                    fvgb_stream stream);
 /* nsteps of fvgb_advect_euler_step in place on (T, T_b), the time loop of
  * test_advection.cpp:116-170 in one call; work/work_b (same sizes) are the other
- * half of the ping-pong.  Meshes of at most 65536 cells take one launch of a
- * one-pass step kernel per step (no face buffer), larger ones the two-pass step
- * of fvgb_advect_euler_step; both give the bits of nsteps single calls. */
+ * half of the ping-pong.  From 4 steps on, meshes of at most 1,024 cells per SM whose
+ * cells have at most 8 faces take one launch for all steps, the cells in registers.
+ * Otherwise, meshes of at most 65536 cells take one launch of a one-pass step kernel
+ * per step (no face buffer), larger ones the two-pass step of fvgb_advect_euler_step;
+ * all give the bits of nsteps single calls. */
 fvgb_status fvgb_advect_euler_steps(const fvgb_mesh* mesh, const double* flux, double* T, double* T_b,
                                     double dt, const fvgb_bc* bc, int32_t nsteps, double* work,
                                     double* work_b, fvgb_stream stream);
@@ -311,8 +313,10 @@ typedef struct fvgb_solver_cfg {
     double inner_rel_tol;      /* MIXED_IR: residual reduction asked of each inner solve */
     int32_t inner_max_iter;    /* MIXED_IR: inner iteration cap per refinement step    */
     int32_t max_outer;         /* MIXED_IR: refinement step cap                        */
-    int32_t kernel_mode;       /* 0 automatic, 1 graph of kernels, 2 one persistent
-                                  cooperative kernel (FP64 single case), 3 host-driven
+    int32_t kernel_mode;       /* 0 automatic, 1 graph of kernels, 2 one kernel for the
+                                  whole solve (single case; one cluster, one block per
+                                  SM with the matrix in shared memory, or a persistent
+                                  grid, by size), 3 host-driven
                                   loop (FP64; blocks the caller); same results          */
     int32_t flags;             /* FVGB_SOLVE_NO_TUNE: default kernel variants, no timing
                                   at the first solve (the timing synchronises the device);

@@ -343,3 +343,15 @@ def test_ilu_sweeps_by_parts_and_levels(cuda, make):
         st = ls.solve(x, rel_tol=1e-9, max_iter=2000, method=method, preconditioner=abi.PRECOND_ILU)
         so = o.solve(v, r, xo, rel_tol=1e-9, max_iter=2000, method=om, preconditioner=2)
         same(st, so, x, xo)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(64, 64, 63), (64, 64, 64)])
+def test_ilu_sweeps_with_and_without_halo_warps(cuda, dims):
+    """Below and at the size from which the rows of other parts are read directly."""
+    hm = mesh.box(*dims, jitter=0.1, seed=2)
+    T, o, ls, v, r = gpu_system(hm, "convection")
+    x, xo = T.internal.clone(), T.host().copy()
+    st = ls.solve(x, rel_tol=1e-9, max_iter=200, method=abi.SOLVER_BICGSTAB, preconditioner=abi.PRECOND_ILU)
+    so = o.solve(v, r, xo, rel_tol=1e-9, max_iter=200, method=1, preconditioner=2)
+    same(st, so, x, xo)
