@@ -3289,16 +3289,25 @@ bool resident_fits(SolverCache* c, bool mixed, cudaStream_t s) {
         if (calloc_dev(c, &d, 4) != cudaSuccess || calloc_dev(c, &mail, 1) != cudaSuccess ||
             settle_creation() != cudaSuccess)
             return false;
+        // on the solve's stream: a device-built mesh may still be in the making there
         const MeshView m = c->ls->mesh->v;
-        if (rows_per_thread(c->n) == 8) k_res_need<8><<<c->nb, kT>>>(m, d);
-        else k_res_need<4><<<c->nb, kT>>>(m, d);
-        if (cudaMemcpy(c->res_need, d, sizeof(c->res_need), cudaMemcpyDeviceToHost) != cudaSuccess) return false;
+        if (rows_per_thread(c->n) == 8) k_res_need<8><<<c->nb, kT, 0, s>>>(m, d);
+        else k_res_need<4><<<c->nb, kT, 0, s>>>(m, d);
+        if (cudaMemcpyAsync(c->res_need, d, sizeof(c->res_need), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess)
+            return false;
         c->mail = mail;
     }
     if (c->res_need[mixed ? 1 : 0] > (unsigned)kResSmem) return false;
     cudaError_t e = cudaSuccess;
-    if (mixed && !c->zll32) e = calloc_dev(c, &c->zll32, (size_t)c->n);
-    if (!mixed && !c->zll) e = calloc_dev(c, &c->zll, (size_t)c->n);
+    if (mixed && !c->zll32) {
+        e = calloc_dev(c, &c->zll32, (size_t)c->n);
+        if (e == cudaSuccess) e = settle_creation();
+    }
+    if (!mixed && !c->zll) {
+        e = calloc_dev(c, &c->zll, (size_t)c->n);
+        if (e == cudaSuccess) e = settle_creation();
+    }
     return e == cudaSuccess;
 }
 

@@ -232,3 +232,36 @@ def test_requests_on_reused_memory_keep_their_bits(cuda, precision, flags):
             assert res[rid].status == alone[k][0]
             np.testing.assert_array_equal(out, alone[k][1])
     abi.lib().fvgb_server_destroy(sv)
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED_IR])
+def test_one_kernel_solves_of_served_requests(cuda, precision):
+    """kernel_mode 2 on requests whose meshes are still being built on the request's
+    stream when the first solve asks how much shared memory they need: cluster, resident
+    (both trees) and persistent sizes, one after another and all at once, give the bits
+    of the graph solves."""
+    dims = [(16, 16, 15), (116, 45, 23), (20, 19, 17), (70, 70, 63), (39, 140, 53), (80, 80, 60)]
+
+    def burst(mode, together):
+        sv, sent, outs = make_server(streams=4), [], []
+        for d in dims:
+            out = np.zeros(d[0] * d[1] * d[2])
+            req = abi.ServeRequest(nx=d[0], ny=d[1], nz=d[2], steps=3, U=(C.c_double * 3)(0.4, -0.3, 0.2), D=2e-3,
+                                   dt=0.0, precision=precision, kernel_mode=mode, flags=0, T_out=out.ctypes.data,
+                                   T_init=None)
+            rid = C.c_int64()
+            abi.check(abi.lib().fvgb_server_submit(sv, C.byref(req), C.byref(rid)))
+            sent.append((req, rid.value))
+            outs.append(out)
+            if not together:
+                drain(sv, 1)
+        if together:
+            res = drain(sv, len(dims))
+            assert all(res[r].status == abi.OK and res[r].steps_done == 3 for _, r in sent)
+        abi.lib().fvgb_server_destroy(sv)
+        return outs
+
+    want = burst(1, True)
+    for together in (False, True, False):
+        for a, b in zip(burst(2, together), want):
+            np.testing.assert_array_equal(a, b)
