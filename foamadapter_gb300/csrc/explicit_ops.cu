@@ -876,7 +876,7 @@ __global__ void __launch_bounds__(kThreads)
 // scale = coeff/V_c (mode 0), 1/V_c (mode 1: coeff 1) or coeff (mode 2: volume integrated).
 // Blocks of 128 threads, 16 an SM for one component and 8 for three (64 registers):
 // with blocks of 256 the registers left room for 48 and 24 warps (128^3 cells: 39 and
-// 96 us, now 27 and 72).  ADD false: out_c = +0 + that, for a buffer that would be zeroed.
+// 96 us, now 35 and 85).  ADD false: out_c = +0 + that, for a buffer that would be zeroed.
 template <int NC, bool ADD>
 __global__ void __launch_bounds__(kGatherThreads, NC == 1 ? 16 : NC == 3 ? 8 : 1)
     k_gather_fx(MeshView m, const double* __restrict__ fx, double coeff, int unit, double* __restrict__ out) {
