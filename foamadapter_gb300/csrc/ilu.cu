@@ -236,10 +236,12 @@ constexpr int kDeps = 4;       // values a row waits for together; the others on
 // 9,600 (up to 140); on 20^3, 0.72 ms with 1,024 and 1.00 in one part (300).
 constexpr int kPart = 8192, kMinPart = 1024, kLevelRows = 128;
 // From this size on the row warps read the rows of other parts themselves, before their
-// turn, and two blocks share an SM: with a halo in shared memory one part of 8,192 rows
-// fills it, and 128^3 has 256 parts.  ILU-CG on 128^3 cells 156 ms with halo warps and 121
-// without (145 with every step through L2), 96^3 86.7 and 72.0, 64^3 22.3 and 18.8;
-// BiCGStab on 48^3 2.16 and 2.24 ms, on 80 x 80 x 9 1.84 and 2.11.
+// turn: their reads are further ahead of need than the halo warps' when levels are wide.
+// ILU-CG on 128^3 cells 156 ms with halo warps and 121 without (145 with every step
+// through L2), 96^3 86.7 and 72.0, 64^3 22.3 and 18.8; BiCGStab on 48^3 2.16 and 2.24 ms,
+// on 80 x 80 x 9 1.84 and 2.11.  The grid is then twice the SMs, of which one block each
+// is resident (123.5 -> 120.0 ms on 128^3, which has 256 parts); without the idle halo
+// warps two were, and it took 140.
 constexpr int kDirectRows = 1 << 18;
 constexpr int kMaxSweepSmem = (3 * kPart + 1) * (int)sizeof(double);
 
