@@ -993,8 +993,19 @@ __global__ void __launch_bounds__(2 * kClRows, 1)
     __shared__ ClShared sh;
     const int n = m.n, T = threadIdx.x, lane = T & 31, wid = T >> 5, nw = (int)blockDim.x >> 5;
     const int rows = (int)blockDim.x, lg = rows == kClRows ? 7 : 8;  // one unit per block, or two
-    const int rank = (int)blockIdx.x, ncta = (int)gridDim.x;
+    // The cluster's size is a power of two, `ncta` of its blocks hold rows.  The others
+    // take no part: a word is written again two epochs on, when every block that sends
+    // partials has read it, and a block without rows sends none, so nothing would make
+    // the others wait for it.
+    const int rank = (int)blockIdx.x, ncta = (units * kClRows + rows - 1) / rows;
     const int row0 = rank * rows, i = row0 + T, nvb = (units + 7) / 8;
+    if (rank >= ncta) {
+        cluster_arrive();
+        cluster_wait();
+        cluster_arrive();
+        cluster_wait();
+        return;
+    }
     const SolverParams prm = L.bs->prm;
     double* x = prm.x;
     for (int k = T; k < (int)(offsetof(ClShared, a) / sizeof(LLWord)); k += rows) ((LLWord*)&sh)[k] = LLWord{0ull, 0ull};

@@ -8,6 +8,8 @@ kernel).  Numberings: the box's own, and a random one in which almost every
 matrix slot reaches into another block (it fits the shared memory with 4 rows
 per thread and does not with 8).
 """
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -114,3 +116,31 @@ def test_resident_solves_on_two_streams(cuda):
         torch.cuda.synchronize()
         for x, w in zip(xs, want):
             np.testing.assert_array_equal(x.cpu().numpy(), w)
+
+
+@pytest.mark.parametrize("n", [257, 520, 1025, 1600, 2049, 3100])
+def test_cluster_blocks_without_rows(cuda, n):
+    """128-row units that do not fill a power-of-two cluster (3, 5, 9, 13 units, 17 and 25 two
+    to a block): thousands of iterations beside other work on the device keep the graph's
+    bits and end at once (a block that waits for a word already written over holds the
+    solve for the seconds that bound a wait)."""
+    hm, T, ls = system((n, 1, 1))
+    kw = dict(rel_tol=1e-300, max_iter=4000, allow=(abi.ERR_NOT_CONVERGED, abi.ERR_BREAKDOWN))
+    x0 = T.internal.clone()
+    want = ls.solve(x0, kernel_mode=1, **kw)
+    other = torch.cuda.Stream()
+    load = torch.randn(1 << 22, device="cuda")
+    for busy in (False, True, True):
+        x = T.internal.clone()
+        ls.solve(x.clone(), kernel_mode=2, **kw)
+        torch.cuda.synchronize()
+        if busy:
+            with torch.cuda.stream(other):
+                for _ in range(200):
+                    load.mul_(1.0001)
+        start = time.perf_counter()
+        st = ls.solve(x, kernel_mode=2, **kw)
+        assert time.perf_counter() - start < 1.0
+        assert (st.num_iter, st.final_res_norm, st.status) == (want.num_iter, want.final_res_norm, want.status)
+        assert torch.equal(x, x0)
+        torch.cuda.synchronize()
