@@ -491,9 +491,13 @@ inline AdvectPlan advect_plan(const fvgb_mesh* m, int nsteps) {
         {(const void*)k_advect_steps<1024, 4>, (const void*)k_advect_steps<1024, 6>,
          (const void*)k_advect_steps<1024, 8>}};
     const void* fn = fns[r][E];
-    const int width = 4 + 2 * E;
-    p.smem = (size_t)bs * (8 * (2 + 2 * width) + 4 * width);
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess) {
+    const int width = 4 + 2 * E, largest = 256 << r;
+    const size_t per_thread = 8 * (2 + 2 * width) + 4 * width;
+    p.smem = bs * per_thread;
+    // the limit belongs to the kernel, not to this call: always its largest block's,
+    // so that calls on other threads never lower it under a launch
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(largest * per_thread)) !=
+        cudaSuccess) {
         cudaGetLastError();
         return p;
     }

@@ -7,6 +7,7 @@ and beyond its largest mesh.  Flows in one direction only, random fluxes, every
 boundary condition and a random cell numbering (neighbours in every block).
 """
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -64,3 +65,58 @@ def test_random_flux_and_boundaries(cuda, dims, shuffled):
     T0 = rng.standard_normal(hm.n)
     T0[::13] = 0.0
     run(hm, flux, T0, bcs, 25, 1e-2)
+
+
+def test_calls_on_two_threads(cuda):
+    """Two meshes whose blocks (384 and 512 threads) are launched from the same kernel,
+    each advanced on a thread and stream of its own."""
+    L = abi.lib()
+
+    def case(dims):
+        hm = mesh.box(*dims)
+        dm = DeviceMesh(hm)
+        rng = np.random.default_rng(4)
+        F = neon.SurfaceField(dm, rng.standard_normal(hm.nif + hm.nbf) * 1e-3)
+        T = neon.VolumeField(dm, rng.standard_normal(hm.n), [("zeroGradient", 0.0)] * hm.npatch)
+        return dm, F, T, T.internal.clone(), T.boundary.clone(), torch.empty_like(T.internal), torch.empty_like(T.boundary)
+
+    def call(c, stream):
+        dm, F, T, _, _, w, wb = c
+        bc = T.bc_struct()
+        return lambda: L.fvgb_advect_euler_steps(dm.handle, abi.ptr(F.values), abi.ptr(T.internal), abi.ptr(T.boundary),
+                                                 1e-2, C.byref(bc), 4, abi.ptr(w), abi.ptr(wb), stream.cuda_stream)
+
+    def restore(c):
+        c[2].internal.copy_(c[3])
+        c[2].boundary.copy_(c[4])
+        torch.cuda.synchronize()
+
+    cases = [case(d) for d in ((40, 36, 33), (60, 40, 30), (40, 36, 33), (60, 40, 30))]
+    streams = [torch.cuda.Stream() for _ in cases]
+    calls = [call(c, s) for c, s in zip(cases, streams)]
+    want = []
+    for c, f in zip(cases, calls):
+        assert f() == abi.OK
+        torch.cuda.synchronize()
+        want.append(c[2].internal.clone())
+        restore(c)
+    bad = []
+
+    def loop(f):
+        for _ in range(5000):
+            if f() != abi.OK:
+                bad.append(abi.lib().fvgb_last_error())
+                return
+
+    threads = [threading.Thread(target=loop, args=(f,)) for f in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not bad
+    for c, f, w in zip(cases, calls, want):
+        restore(c)
+        assert f() == abi.OK
+        torch.cuda.synchronize()
+        assert torch.equal(c[2].internal, w)
