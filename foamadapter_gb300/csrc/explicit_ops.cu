@@ -1343,8 +1343,8 @@ extern "C" fvgb_status fvgb_advect_euler_steps(const fvgb_mesh* m, const double*
             e = cudaLaunchCooperativeKernel(plan.fn, dim3(grid_for(v.n, plan.threads)), dim3(plan.threads), args,
                                             plan.smem, s);
         cudaFreeAsync(ex, s);
-        if (e != cudaSuccess) return cuda_fail(e, "fvgb_advect_euler_steps");
-        return FVGB_OK;
+        if (e == cudaSuccess) return FVGB_OK;
+        cudaGetLastError();  // not launched (fewer SMs than the device's): a launch per step needs no co-residency
     }
     // the fixed-gradient boundary quotients ref/delta do not change between
     // steps: formed once for the whole call

@@ -3412,6 +3412,9 @@ fvgb_status launch(SolverCache* c, double* x, const fvgb_solver_cfg* cfg, fvgb_s
         const double* b = c->ls->rhs;
         int nvb = c->nb;
         const bool mixed = cfg->precision == FVGB_PREC_MIXED_IR;
+        // A kernel that the device refuses (a partition of its SMs, say) leaves the solve to
+        // the next one, the graph at last.
+        cudaError_t e = cudaErrorNotSupported;  // until one is launched
         const ClusterPlan cl = mixed ? ClusterPlan{} : cluster_plan(c);
         if (cl.ctas) {
             cudaLaunchConfig_t lc{};
@@ -3425,44 +3428,48 @@ fvgb_status launch(SolverCache* c, double* x, const fvgb_solver_cfg* cfg, fvgb_s
             lc.stream = s;
             lc.attrs = &at;
             lc.numAttrs = 1;
-            FVGB_CUDA_TRY(cudaLaunchKernelEx(&lc, k_pcg_cluster, L, m, val, b, cl.units));
+            e = cudaLaunchKernelEx(&lc, k_pcg_cluster, L, m, val, b, cl.units);
+        }
+        const int pg = persistent_grid(c, mixed);
+        const int grid = nvb < pg ? nvb : pg;
+        const bool r8 = rows_per_thread(c->n) == 8;
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            FVGB_CUDA_TRY(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), s));
+            if (resident_fits(c, mixed, s)) {
+                FVGB_CUDA_TRY(cudaMemsetAsync(c->mail, 0, sizeof(ResMail), s));
+                const unsigned int* need = c->res_need + (mixed ? 1 : 0);
+                const size_t smem = need[2] <= (unsigned)kResSmem ? need[2] : need[0];
+                if (mixed) {
+                    FVGB_CUDA_TRY(cudaMemsetAsync(c->zll32, 0, sizeof(*c->zll32) * (size_t)c->n, s));
+                    void* args[] = {&L, &m, &val, &b, &c->ah, &c->ev, &c->dinvf, &c->zll32, &c->mail, &c->bar};
+                    const void* fn = r8 ? (const void*)k_ir_resident<8> : (const void*)k_ir_resident<4>;
+                    e = cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s);
+                } else {
+                    FVGB_CUDA_TRY(cudaMemsetAsync(c->zll, 0, sizeof(LLWord) * (size_t)c->n, s));
+                    void* args[] = {&L, &m, &val, &b, &c->zll, &c->mail, &c->bar};
+                    const void* fn = r8 ? (const void*)k_pcg_resident<8> : (const void*)k_pcg_resident<4>;
+                    e = cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s);
+                }
+            }
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            // k_ir_persistent(L, m, val, b, a32, ev, dinv, r0, rh, y, pbuf0, pbuf1, z, q, pa, pb, pc, gb, nvb)
+            void* args_mixed[] = {&L,     &m,    &val,   &b,     &c->ah, &c->ev, &c->dinvf, &c->r0, &c->rh, &c->y,
+                                  &c->pf, &c->pf2, &c->zf, &c->qf, &c->pa, &c->pb, &c->pc,   &c->bar, &nvb};
+            void* args_fp64[] = {&L, &m, &val, &b, &c->dinv, &c->r, &c->p, &c->q, &c->z, &c->pa, &c->pb, &c->bar, &nvb};
+            const void* fn_mixed = r8 ? (const void*)k_ir_persistent<8> : (const void*)k_ir_persistent<4>;
+            const void* fn_fp64 = r8 ? (const void*)k_pcg_persistent<8> : (const void*)k_pcg_persistent<4>;
+            e = cudaLaunchCooperativeKernel(mixed ? fn_mixed : fn_fp64, dim3(grid), dim3(kPT),
+                                            mixed ? args_mixed : args_fp64, 0, s);
+        }
+        if (e == cudaSuccess) {
             k_finish<<<grid_for(c->ncases, 128), 128, 0, s>>>(c->L);
             FVGB_LAUNCH_CHECK("fvgb_solve: finish");
             return FVGB_OK;
         }
-        const int pg = persistent_grid(c, mixed);
-        const int grid = nvb < pg ? nvb : pg;
-        FVGB_CUDA_TRY(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), s));
-        const bool r8 = rows_per_thread(c->n) == 8;
-        if (resident_fits(c, mixed, s)) {
-            FVGB_CUDA_TRY(cudaMemsetAsync(c->mail, 0, sizeof(ResMail), s));
-            const unsigned int* need = c->res_need + (mixed ? 1 : 0);
-            const size_t smem = need[2] <= (unsigned)kResSmem ? need[2] : need[0];
-            if (mixed) {
-                FVGB_CUDA_TRY(cudaMemsetAsync(c->zll32, 0, sizeof(*c->zll32) * (size_t)c->n, s));
-                void* args[] = {&L, &m, &val, &b, &c->ah, &c->ev, &c->dinvf, &c->zll32, &c->mail, &c->bar};
-                const void* fn = r8 ? (const void*)k_ir_resident<8> : (const void*)k_ir_resident<4>;
-                FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s));
-            } else {
-                FVGB_CUDA_TRY(cudaMemsetAsync(c->zll, 0, sizeof(LLWord) * (size_t)c->n, s));
-                void* args[] = {&L, &m, &val, &b, &c->zll, &c->mail, &c->bar};
-                const void* fn = r8 ? (const void*)k_pcg_resident<8> : (const void*)k_pcg_resident<4>;
-                FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s));
-            }
-        } else if (mixed) {
-            // k_ir_persistent(L, m, val, b, a32, ev, dinv, r0, rh, y, pbuf0, pbuf1, z, q, pa, pb, pc, gb, nvb)
-            void* args[] = {&L,     &m,    &val,   &b,     &c->ah, &c->ev, &c->dinvf, &c->r0, &c->rh, &c->y,
-                            &c->pf, &c->pf2, &c->zf, &c->qf, &c->pa, &c->pb, &c->pc,   &c->bar, &nvb};
-            const void* fn = r8 ? (const void*)k_ir_persistent<8> : (const void*)k_ir_persistent<4>;
-            FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPT), args, 0, s));
-        } else {
-            void* args[] = {&L, &m, &val, &b, &c->dinv, &c->r, &c->p, &c->q, &c->z, &c->pa, &c->pb, &c->bar, &nvb};
-            const void* fn = r8 ? (const void*)k_pcg_persistent<8> : (const void*)k_pcg_persistent<4>;
-            FVGB_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPT), args, 0, s));
-        }
-        k_finish<<<grid_for(c->ncases, 128), 128, 0, s>>>(c->L);
-        FVGB_LAUNCH_CHECK("fvgb_solve: finish");
-        return FVGB_OK;
+        cudaGetLastError();
     }
     FVGB_CUDA_TRY(cudaGraphLaunch(cfg->precision == FVGB_PREC_FP64 ? c->g64 : c->gmix, s));
     return FVGB_OK;
