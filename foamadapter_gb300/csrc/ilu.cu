@@ -245,21 +245,25 @@ constexpr int kPart = 8192, kMinPart = 1024, kLevelRows = 128;
 constexpr int kDirectRows = 1 << 18;
 constexpr int kMaxSweepSmem = (3 * kPart + 1) * (int)sizeof(double);
 
-// A triangle's sweep.  Part p has the rows from p * rpp on; its levels are lev[p] to
-// lev[p + 1] - 1, level q its rows rows[32 chunk[q]] to rows[32 chunk[q + 1] - 1] (-1:
-// none), np of them in all.  Of row number t the values it depends on (k < K) are at
-// slot[k np + t]: a place in the part's shared memory (its own rows, then what the halo
-// warps bring), -1 none, below -1 the row -2 - slot read from global memory.
-// val[k np + t]: the factor's entries, filled in every solve; from val[K np + t] on the
-// pivots and their reciprocals (backward) or the matrix's a_ki and a_ii (forward: until
-// the factorization, which reads the matrix's a_ik at val[k np + t], is done).
+// A triangle's sweep.  Its rows stand at positions 0 .. n - 1, row rows[t] at position t,
+// in the order of the parts, in a part by level: part p has the positions first[p] to
+// first[p + 1] - 1 and the levels lev[p] to lev[p + 1] - 1, level q the positions
+// start[q] to start[q + 1] - 1.  (Levels filled up to whole warps, for aligned loads, took
+// 32 times the memory where a level has one row.)  A row's place in its part's shared
+// memory is its position less the part's first.  Of the row at position t the values it
+// depends on (k < K) are at slot[k n + t]: a place in the part's shared memory (its own
+// rows, then what the halo warps bring), -1 none, below -1 the row -2 - slot read from
+// global memory.  val[k n + t]: the factor's entries, filled in every solve; from
+// val[K n + t] on the pivots and their reciprocals (backward) or the matrix's a_ki and
+// a_ii (forward, where the factorization is a sweep: until it is done, and it reads the
+// matrix's a_ik at val[k n + t]).
 struct Sweep {
-    int n, np, rpp, nparts, K, hcap, W;
+    int n, rpp, nparts, K, hcap, W;
     const int* rows;
+    const int* first;
     const int* lev;
-    const int* chunk;
-    int* place;        // [n] a row's place in its part's shared memory: its rank in level order
-    const int* off;    // [levels] 32 chunk minus the place of the level's first row
+    const int* start;
+    int* pos;    // [n] a row's position
     int* slot;
     double* val;
     int* halo;   // [nparts][hcap] rows of other parts
@@ -322,41 +326,30 @@ __device__ __forceinline__ void st_shared(unsigned a, double v) {
     asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
-// Every row's place in its part's shared memory.  A position's level is the last one
-// that starts at or before it.
-__global__ void __launch_bounds__(kT) k_il_place(Sweep S) {
+__global__ void __launch_bounds__(kT) k_il_pos(Sweep S) {
     const int t = blockIdx.x * kT + threadIdx.x;
-    const int i = t < S.np ? __ldg(&S.rows[t]) : -1;
-    if (i < 0) return;
-    int a = 0, b = __ldg(&S.lev[S.nparts]);  // chunk[a] <= t / 32 < chunk[b]
-    while (b - a > 1) {
-        const int h = (a + b) / 2;
-        if (__ldg(&S.chunk[h]) <= t / 32) a = h;
-        else b = h;
-    }
-    S.place[i] = t - __ldg(&S.off[a]);
+    if (t < S.n) S.pos[__ldg(&S.rows[t])] = t;
 }
 
 // Where the values that a part's rows depend on are found: one block per part.
 template <bool BWD>
 __global__ void __launch_bounds__(kT) k_il_plan(Csr A, Sweep S) {
     __shared__ int wsum[kT / 32], base;
-    const int r0 = blockIdx.x * S.rpp, r1 = min(S.n, r0 + S.rpp);
-    const int t1 = 32 * __ldg(&S.chunk[__ldg(&S.lev[blockIdx.x + 1])]);
+    const int t0 = __ldg(&S.first[blockIdx.x]), t1 = __ldg(&S.first[blockIdx.x + 1]);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x == 0) base = 0;
     __syncthreads();
-    for (int q = 32 * __ldg(&S.chunk[__ldg(&S.lev[blockIdx.x])]); q < t1; q += kT) {
+    for (int q = t0; q < t1; q += kT) {
         const int t = q + threadIdx.x;
-        const int i = t < t1 ? __ldg(&S.rows[t]) : -1;
         int e0 = 0, e1 = 0, cnt = 0;
-        if (i >= 0) {
+        if (t < t1) {
+            const int i = __ldg(&S.rows[t]);
             const int d = __ldg(&A.ro[i]) + __ldg(&A.dof[i]);
             e0 = BWD ? d + 1 : __ldg(&A.ro[i]);
             e1 = min(BWD ? __ldg(&A.ro[i + 1]) : d, e0 + S.K);
             for (int e = e0; e < e1; ++e) {
-                const int c = __ldg(&A.col[e]);
-                cnt += c < r0 || c >= r1;
+                const int c = __ldg(&S.pos[__ldg(&A.col[e])]);
+                cnt += c < t0 || c >= t1;
             }
         }
         int x = cnt;  // inclusive scan
@@ -373,17 +366,17 @@ __global__ void __launch_bounds__(kT) k_il_plan(Csr A, Sweep S) {
             for (int k = 0; k < S.K; ++k) {
                 int sl = -1;
                 if (e0 + k < e1) {
-                    const int c = __ldg(&A.col[e0 + k]);
-                    if (c >= r0 && c < r1) {
-                        sl = __ldg(&S.place[c]);
+                    const int r = __ldg(&A.col[e0 + k]), c = __ldg(&S.pos[r]);
+                    if (c >= t0 && c < t1) {
+                        sl = c - t0;
                     } else if (at < S.hcap) {
-                        S.halo[(size_t)blockIdx.x * S.hcap + at] = c;
+                        S.halo[(size_t)blockIdx.x * S.hcap + at] = r;
                         sl = S.rpp + at++;
                     } else {
-                        sl = -2 - c;
+                        sl = -2 - r;
                     }
                 }
-                S.slot[(size_t)k * S.np + t] = sl;
+                S.slot[(size_t)k * S.n + t] = sl;
             }
         }
         __syncthreads();
@@ -407,21 +400,21 @@ struct Factor {  // of the pivots alone: entry e of the lower triangle updates i
 template <int KIND>
 __global__ void __launch_bounds__(kT) k_il_pack(Csr A, Sweep S, Factor F, const double* __restrict__ piv) {
     const int t = blockIdx.x * kT + threadIdx.x;
-    const int i = t < S.np ? __ldg(&S.rows[t]) : -1;
-    if (i < 0) return;
+    if (t >= S.n) return;
+    const int i = __ldg(&S.rows[t]);
     const int b = __ldg(&A.ro[i]), d = b + __ldg(&A.dof[i]);
     const int e0 = KIND == kBwd ? d + 1 : b, e1 = min(e0 + S.K, KIND == kBwd ? __ldg(&A.ro[i + 1]) : d);
     for (int e = e0; e < e1; ++e) {
-        double* v = S.val + (size_t)(e - e0) * S.np + t;
+        double* v = S.val + (size_t)(e - e0) * S.n + t;
         *v = KIND == kFactor ? __ldg(&F.a[e]) : F.lu[e];
-        if (KIND == kFactor) v[(size_t)S.K * S.np] = __ldg(&F.a[__ldg(&F.g[__ldg(&F.p[e])])]);
+        if (KIND == kFactor) v[(size_t)S.K * S.n] = __ldg(&F.a[__ldg(&F.g[__ldg(&F.p[e])])]);
     }
     if (KIND == kBwd) {
         const double u = piv ? piv[i] : F.lu[d];
-        S.val[(size_t)S.K * S.np + t] = u;
-        S.val[(size_t)(S.K + 1) * S.np + t] = 1.0 / u;
+        S.val[(size_t)S.K * S.n + t] = u;
+        S.val[(size_t)(S.K + 1) * S.n + t] = 1.0 / u;
     }
-    if (KIND == kFactor) S.val[(size_t)(2 * S.K) * S.np + t] = __ldg(&F.a[d]);
+    if (KIND == kFactor) S.val[(size_t)(2 * S.K) * S.n + t] = __ldg(&F.a[d]);
 }
 
 // Part of this block (the same in all its threads), or >= nparts when none is left.
@@ -456,21 +449,21 @@ template <int KIND, int K>
 __device__ __forceinline__ void fetch_row(const Sweep& S, const double* src, int t, int i, RowIn<K>& q) {
     q.i = i;
 #pragma unroll
-    for (int k = 0; k < K; ++k) q.slot[k] = __ldg(&S.slot[(size_t)k * S.np + t]);
+    for (int k = 0; k < K; ++k) q.slot[k] = i < 0 ? -1 : __ldg(&S.slot[(size_t)k * S.n + t]);
     q.s = q.piv = q.rcp = 1.0;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        q.v[k] = q.slot[k] == -1 ? 0.0 : S.val[(size_t)k * S.np + t];
-        if (KIND == kFactor) q.w[k] = q.slot[k] == -1 ? 0.0 : S.val[(size_t)(K + k) * S.np + t];
+        q.v[k] = q.slot[k] == -1 ? 0.0 : S.val[(size_t)k * S.n + t];
+        if (KIND == kFactor) q.w[k] = q.slot[k] == -1 ? 0.0 : S.val[(size_t)(K + k) * S.n + t];
     }
     if (i < 0) return;
     if (KIND == kFactor) {
-        q.s = S.val[(size_t)(2 * K) * S.np + t];
+        q.s = S.val[(size_t)(2 * K) * S.n + t];
     } else {
         q.s = __ldcg(&src[i]);
         if (KIND == kBwd) {
-            q.piv = S.val[(size_t)K * S.np + t];
-            q.rcp = S.val[(size_t)(K + 1) * S.np + t];
+            q.piv = S.val[(size_t)K * S.n + t];
+            q.rcp = S.val[(size_t)(K + 1) * S.n + t];
         }
     }
 }
@@ -591,12 +584,11 @@ __global__ void __launch_bounds__(kSweepThreads)
     const int T = min(kMaxTeams, kRowWarps / S.W), count = 64 * S.W;
     if (threadIdx.x == 0) smem[S.rpp + S.hcap] = 0.0;
     for (int u = next_part(st); u < S.nparts; u = next_part(st)) {
-        const int part = KIND == kBwd ? S.nparts - 1 - u : u;
-        const int nh = __ldg(&S.nhalo[part]);
+        const int nh = __ldg(&S.nhalo[u]), t0 = __ldg(&S.first[u]);
         for (int k = threadIdx.x; k < nh; k += kSweepThreads) smem[S.rpp + k] = unset;
         __syncthreads();
         if (w >= kRowWarps) {
-            const int* halo = S.halo + (size_t)part * S.hcap;
+            const int* halo = S.halo + (size_t)u * S.hcap;
             for (int h = (w - kRowWarps) * 32 + lane; h < nh; h += 32 * kHaloWarps) {
                 const double* p = &v[__ldg(&halo[h])];
                 unsigned long long t0 = 0;
@@ -619,33 +611,33 @@ __global__ void __launch_bounds__(kSweepThreads)
             }
         } else if (w < T * S.W) {
             const int team = w / S.W, tw = w % S.W;
-            const int l0 = __ldg(&S.lev[part]), l1 = __ldg(&S.lev[part + 1]);
-            // chunks [c, ce) of this warp's level, its rows fetched; [n, ne) of the one after, i the first's rows
+            const int l0 = __ldg(&S.lev[u]), l1 = __ldg(&S.lev[u + 1]);
+            // positions [c, ce) of this warp's level, 32 at a time, the first fetched; [n, ne) of the one after, i the first's rows
             RowIn<K> q;
-            int c, ce, co, n, ne, no, i = -1;
-            const auto level = [&](int l, int& a, int& b, int& o) {
-                a = b = o = 0;
+            int c, ce, n, ne, i = -1;
+            const auto level = [&](int l, int& a, int& b) {
+                a = b = 0;
                 if (l < l1) {
-                    a = __ldg(&S.chunk[l]) + tw;
-                    b = __ldg(&S.chunk[l + 1]);
-                    o = __ldg(&S.off[l]);
+                    a = __ldg(&S.start[l]) + 32 * tw;
+                    b = __ldg(&S.start[l + 1]);
                 }
             };
-            level(l0 + team, c, ce, co);
-            level(l0 + team + T, n, ne, no);
-            if (c < ce) fetch_row<KIND>(S, src, 32 * c + lane, __ldg(&S.rows[32 * c + lane]), q);
-            if (n < ne) i = __ldg(&S.rows[32 * n + lane]);
+            const auto row = [&](int a, int b) { return a + lane < b ? __ldg(&S.rows[a + lane]) : -1; };
+            level(l0 + team, c, ce);
+            level(l0 + team + T, n, ne);
+            if (c < ce) fetch_row<KIND>(S, src, c + lane, row(c, ce), q);
+            if (n < ne) i = row(n, ne);
             for (int l = l0 + team; l < l1; l += T) {
-                int n2, n2e, n2o;
-                level(l + 2 * T, n2, n2e, n2o);
+                int n2, n2e;
+                level(l + 2 * T, n2, n2e);
                 const int turn = 1 + team, next = 1 + (team + 1) % T;
                 if (c < ce) {
                     double z = l > l0 ? sweep_row<KIND, K, DIRECT, true>(st, A, S, F, lu, sm, q, v, turn, count)
                                       : sweep_row<KIND, K, DIRECT, false>(st, A, S, F, lu, sm, q, v, turn, count);
                     for (;;) {
-                        if (q.i >= 0) st_shared(sm + 8u * (unsigned)(32 * c + lane - co), z);
-                        const int cd = c;
-                        c += S.W;
+                        const int t = c + lane;
+                        if (q.i >= 0) st_shared(sm + 8u * (unsigned)(t - t0), z);
+                        c += 32 * S.W;
                         if (c >= ce) {
                             __syncwarp();
                             if (l + 1 < l1)
@@ -657,11 +649,11 @@ __global__ void __launch_bounds__(kSweepThreads)
                             if (KIND == kFactor) {
 #pragma unroll
                                 for (int k = 0; k < K; ++k)
-                                    if (q.slot[k] != -1) S.val[(size_t)k * S.np + 32 * cd + lane] = q.v[k];
+                                    if (q.slot[k] != -1) S.val[(size_t)k * S.n + t] = q.v[k];
                             }
                         }
                         if (c >= ce) break;
-                        fetch_row<KIND>(S, src, 32 * c + lane, __ldg(&S.rows[32 * c + lane]), q);
+                        fetch_row<KIND>(S, src, c + lane, row(c, ce), q);
                         z = sweep_row<KIND, K, DIRECT, false>(st, A, S, F, lu, sm, q, v, 0, 0);
                     }
                 } else {
@@ -670,12 +662,10 @@ __global__ void __launch_bounds__(kSweepThreads)
                 }
                 c = n;
                 ce = ne;
-                co = no;
                 n = n2;
                 ne = n2e;
-                no = n2o;
-                if (c < ce) fetch_row<KIND>(S, src, 32 * c + lane, i, q);
-                if (n < ne) i = __ldg(&S.rows[32 * n + lane]);
+                if (c < ce) fetch_row<KIND>(S, src, c + lane, i, q);
+                if (n < ne) i = row(n, ne);
             }
         }
     }
@@ -1064,49 +1054,46 @@ int part_rows(const std::vector<int>& level) {
     return rpp;
 }
 
-// The order of a sweep from the rows' levels: by part, by level, each level filled up to
-// whole warps.
-cudaError_t il_sweep(IluCache* c, Sweep& S, const std::vector<int>& level) {
-    std::vector<int> rows, lev(1, 0), chunk, off, at;
-    rows.reserve((size_t)S.n * 5 / 4);
-    int most = 0;  // chunks of the largest level
-    for (int p = 0; p < S.nparts; ++p) {
+// The order of a sweep from the rows' levels: the parts as they are taken, in a part by
+// level.  vals: doubles per row of S.val.
+cudaError_t il_sweep(IluCache* c, Sweep& S, const std::vector<int>& level, bool bwd, int vals) {
+    std::vector<int> rows((size_t)S.n), first(1, 0), lev(1, 0), start, at;
+    int most = 0;  // rows of the largest level
+    for (int u = 0; u < S.nparts; ++u) {
+        const int p = bwd ? S.nparts - 1 - u : u;
         const int r0 = p * S.rpp, r1 = std::min(S.n, r0 + S.rpp);
         const auto mm = std::minmax_element(level.begin() + r0, level.begin() + r1);
         const int lo = *mm.first, nl = *mm.second - lo + 1;
         at.assign((size_t)nl, 0);
         for (int i = r0; i < r1; ++i) ++at[(size_t)(level[(size_t)i] - lo)];
-        int end = (int)rows.size(), place = 0;
+        int end = first.back();
         for (int& a : at) {
             const int cnt = a;
             a = end;
             if (cnt == 0) continue;
-            chunk.push_back(end / 32);
-            off.push_back(end - place);
-            place += cnt;
-            end += (cnt + 31) / 32 * 32;
-            most = std::max(most, (cnt + 31) / 32);
+            start.push_back(end);
+            end += cnt;
+            most = std::max(most, cnt);
         }
-        rows.resize((size_t)end, -1);
         for (int i = r0; i < r1; ++i) rows[(size_t)at[(size_t)(level[(size_t)i] - lo)]++] = i;
-        lev.push_back((int)chunk.size());
+        first.push_back(end);
+        lev.push_back((int)start.size());
     }
-    chunk.push_back((int)(rows.size() / 32));
-    S.np = (int)rows.size();
+    start.push_back(S.n);
     S.W = 1;
-    while (S.W < most && S.W < kRowWarps / 2) S.W *= 2;
-    int *r = nullptr, *lv = nullptr, *ch = nullptr, *of = nullptr;
+    while (32 * S.W < most && S.W < kRowWarps / 2) S.W *= 2;
+    int *r = nullptr, *fi = nullptr, *lv = nullptr, *sa = nullptr;
     cudaError_t e = il_upload(c, &r, rows);
+    if (e == cudaSuccess) e = il_upload(c, &fi, first);
     if (e == cudaSuccess) e = il_upload(c, &lv, lev);
-    if (e == cudaSuccess) e = il_upload(c, &ch, chunk);
-    if (e == cudaSuccess) e = il_alloc(c, &S.place, (size_t)S.n);
-    if (e == cudaSuccess) e = il_upload(c, &of, off);
+    if (e == cudaSuccess) e = il_upload(c, &sa, start);
     S.rows = r;
-    S.off = of;
+    S.first = fi;
     S.lev = lv;
-    S.chunk = ch;
-    if (e == cudaSuccess) e = il_alloc(c, &S.slot, (size_t)S.K * S.np);
-    if (e == cudaSuccess) e = il_alloc(c, &S.val, (size_t)(2 * S.K + 1) * S.np);
+    S.start = sa;
+    if (e == cudaSuccess) e = il_alloc(c, &S.pos, (size_t)S.n);
+    if (e == cudaSuccess) e = il_alloc(c, &S.slot, (size_t)S.K * S.n);
+    if (e == cudaSuccess) e = il_alloc(c, &S.val, (size_t)vals * S.n);
     if (e == cudaSuccess) e = il_alloc(c, &S.halo, (size_t)S.nparts * S.hcap);
     if (e == cudaSuccess) e = il_alloc(c, &S.nhalo, (size_t)S.nparts);
     return e;
@@ -1179,8 +1166,8 @@ fvgb_status symbolic(IluCache* c) {
     if (e == cudaSuccess && !c->pivots_only) e = il_upload(c, &c->op_f, op_f);
     if (e == cudaSuccess) e = il_upload(c, &c->op_g, op_g);
     if (e == cudaSuccess && !c->pivots_only) e = il_upload(c, &c->lev_rows, lev_rows);
-    if (e == cudaSuccess) e = il_sweep(c, c->fwd, lev_f);
-    if (e == cudaSuccess) e = il_sweep(c, c->bwd, lev_b);
+    if (e == cudaSuccess) e = il_sweep(c, c->fwd, lev_f, false, c->pivots_only ? 2 * c->fwd.K + 1 : c->fwd.K);
+    if (e == cudaSuccess) e = il_sweep(c, c->bwd, lev_b, true, c->bwd.K + 2);
     if (e == cudaSuccess) e = il_alloc(c, &c->a, (size_t)nnz);
     if (e == cudaSuccess) e = il_alloc(c, &c->lu, (size_t)nnz);
     double** vecs[] = {&c->r, &c->rr, &c->p, &c->q, &c->v, &c->y, &c->z, &c->s, &c->t, &c->w};
@@ -1193,7 +1180,7 @@ fvgb_status symbolic(IluCache* c) {
     if (e != cudaSuccess) return cuda_fail(e, "ILU setup");
     const Csr A{n, c->ro, c->col, c->dof};
     if (n > 0) {
-        for (const Sweep& S : {c->fwd, c->bwd}) k_il_place<<<grid_of(S.np), kT>>>(S);
+        for (const Sweep& S : {c->fwd, c->bwd}) k_il_pos<<<grid_of(n), kT>>>(S);
         k_il_plan<false><<<nparts, kT>>>(A, c->fwd);
         k_il_plan<true><<<nparts, kT>>>(A, c->bwd);
         FVGB_LAUNCH_CHECK("ILU plan");
@@ -1267,7 +1254,7 @@ fvgb_status build_graph(IluCache* c, bool bicgstab) {
     const Factor F{c->a, c->lu, c->op_ptr, c->op_g};
     if (c->pivots_only) {
         ch.add((void*)k_il_pending, ng, n, c->t);
-        ch.add((void*)k_il_pack<kFactor>, grid_of(c->fwd.np), A, c->fwd, F, (const double*)nullptr);
+        ch.add((void*)k_il_pack<kFactor>, grid_of(n), A, c->fwd, F, (const double*)nullptr);
         add_sweep<kFactor>(c, ch, c->fwd, c->a, c->t, c->t);
     } else {
         for (size_t l = 0; l + 1 < c->fwd_ptr.size(); ++l) {
@@ -1276,8 +1263,8 @@ fvgb_status build_graph(IluCache* c, bool bicgstab) {
                    (const int*)c->op_ptr, (const int*)c->op_f, (const int*)c->op_g, c->lu);
         }
     }
-    if (!c->pivots_only) ch.add((void*)k_il_pack<kFwd>, grid_of(c->fwd.np), A, c->fwd, F, (const double*)nullptr);
-    ch.add((void*)k_il_pack<kBwd>, grid_of(c->bwd.np), A, c->bwd, F, (const double*)(c->pivots_only ? c->t : nullptr));
+    if (!c->pivots_only) ch.add((void*)k_il_pack<kFwd>, grid_of(n), A, c->fwd, F, (const double*)nullptr);
+    ch.add((void*)k_il_pack<kBwd>, grid_of(n), A, c->bwd, F, (const double*)(c->pivots_only ? c->t : nullptr));
     if (!bicgstab) {
         ch.add((void*)k_ic_init, nb, st, A, R, a, b, c->r, c->pa);
         add_apply(c, ch, c->r, c->z);

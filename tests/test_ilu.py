@@ -355,3 +355,22 @@ def test_ilu_sweeps_with_and_without_halo_warps(cuda, dims):
     st = ls.solve(x, rel_tol=1e-9, max_iter=200, method=abi.SOLVER_BICGSTAB, preconditioner=abi.PRECOND_ILU)
     so = o.solve(v, r, xo, rel_tol=1e-9, max_iter=200, method=1, preconditioner=2)
     same(st, so, x, xo)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(20000, 45, 1), (300000, 1, 1)])
+def test_ilu_memory_of_thin_levels(cuda, dims):
+    """Device memory of the first solve where a level has one row, in a part or altogether.
+    Per row of a 2-D mesh: pattern 60 bytes (five entries' columns, operation lists and
+    offsets), two copies of the entries 80, ten vectors 80, the two sweeps 140 (seven and
+    five doubles, three slots each, row order and its inverse) and their levels 8, halo
+    lists 16: 384, a chain's less.  512 with 64 MB for the allocator's granularity."""
+    import torch
+
+    hm = mesh.box(*dims, two_d=dims[1] > 1)
+    T, o, ls, v, r = gpu_system(hm, "heat")
+    x = T.internal.clone()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ls.solve(x, rel_tol=1e-9, max_iter=2, method=abi.SOLVER_CG, preconditioner=abi.PRECOND_ILU)
+    assert free - torch.cuda.mem_get_info()[0] <= 512 * hm.n + (64 << 20)
