@@ -37,6 +37,8 @@
 // final tree), so the oracle's restatements give the same bits.
 #include <algorithm>
 #include <cmath>
+#include <queue>
+#include <utility>
 #include <vector>
 
 #include "internal.cuh"
@@ -234,7 +236,7 @@ constexpr int kDeps = 4;       // values a row waits for together; the others on
 // leaves two teams, which fetch too late.  BiCGStab on 77 x 64 x 58 cells: 3.20 ms with
 // parts of 8,192 rows, 4.06 with 4,096 (levels of up to 128 and 64 rows), 4.05 with
 // 9,600 (up to 140); on 20^3, 0.72 ms with 1,024 and 1.00 in one part (300).
-constexpr int kPart = 8192, kMinPart = 1024, kLevelRows = 128;
+constexpr int kPart = 8192, kMinPart = 1024, kLevelRows = 128, kThinRows = 16;
 // From this size on the row warps read the rows of other parts themselves, before their
 // turn: their reads are further ahead of need than the halo warps' when levels are wide.
 // ILU-CG on 128^3 cells 156 ms with halo warps and 121 without (145 with every step
@@ -1054,29 +1056,89 @@ int part_rows(const std::vector<int>& level) {
     return rpp;
 }
 
+// Rows of a group: parts of consecutive rows have levels of few rows when the mesh's lines
+// are long (one row, where a line is longer than a part), and a level takes as long for one
+// row as for 32.  Such parts are cut from groups of consecutive rows instead, doubled from
+// a part's size until a group in the middle has kThinRows rows a level, or is all rows.
+int group_rows(const std::vector<int>& level, int rpp) {
+    const long n = (long)level.size();
+    long group = rpp;
+    for (; group < n; group *= 2) {
+        const long r0 = (n / 2) / group * group, r1 = std::min(n, r0 + group);
+        const auto mm = std::minmax_element(level.begin() + r0, level.begin() + r1);
+        if (r1 - r0 >= (long)kThinRows * (*mm.second - *mm.first + 1)) break;
+    }
+    return (int)std::min(group, n);
+}
+
+// The order in which the parts of a sweep are taken: after every part it depends on, the
+// one with the lowest first level first.  rows: in the order of groups, in a group by
+// level; part p has rpp of them from p rpp on (a group is a multiple, or all rows).
+std::vector<int> part_order(const fvgb_mesh* m, const std::vector<int>& rows, const std::vector<int>& level, int rpp,
+                            int nparts, bool bwd) {
+    const int n = (int)rows.size();
+    std::vector<int> part((size_t)n), need((size_t)nparts, 0), seen((size_t)nparts, -1), order;
+    std::vector<std::vector<int>> then((size_t)nparts);
+    for (int t = 0; t < n; ++t) part[(size_t)rows[(size_t)t]] = t / rpp;
+    for (int t = 0; t < n; ++t) {
+        const int p = t / rpp, i = rows[(size_t)t], d = m->h_row_offs[i] + m->h_diag_off[i];
+        for (int e = bwd ? d + 1 : m->h_row_offs[i]; e < (bwd ? m->h_row_offs[i + 1] : d); ++e) {
+            const int q = part[(size_t)m->h_col[e]];
+            if (q == p || seen[(size_t)q] == p) continue;
+            seen[(size_t)q] = p;
+            then[(size_t)q].push_back(p);
+            ++need[(size_t)p];
+        }
+    }
+    using Entry = std::pair<int, int>;  // first level, part
+    std::priority_queue<Entry, std::vector<Entry>, std::greater<Entry>> ready;
+    const auto put = [&](int p) { ready.emplace(level[(size_t)rows[(size_t)p * rpp]], p); };
+    for (int p = 0; p < nparts; ++p)
+        if (need[(size_t)p] == 0) put(p);
+    while (!ready.empty()) {
+        const int p = ready.top().second;
+        ready.pop();
+        order.push_back(p);
+        for (int q : then[(size_t)p])
+            if (--need[(size_t)q] == 0) put(q);
+    }
+    return order;
+}
+
 // The order of a sweep from the rows' levels: the parts as they are taken, in a part by
 // level.  vals: doubles per row of S.val.
-cudaError_t il_sweep(IluCache* c, Sweep& S, const std::vector<int>& level, bool bwd, int vals) {
-    std::vector<int> rows((size_t)S.n), first(1, 0), lev(1, 0), start, at;
+cudaError_t il_sweep(IluCache* c, Sweep& S, const std::vector<int>& level, int group, bool bwd, int vals) {
+    std::vector<int> rows((size_t)S.n), sorted((size_t)S.n), order, first(1, 0), lev(1, 0), start, at;
     int most = 0;  // rows of the largest level
-    for (int u = 0; u < S.nparts; ++u) {
-        const int p = bwd ? S.nparts - 1 - u : u;
-        const int r0 = p * S.rpp, r1 = std::min(S.n, r0 + S.rpp);
+    for (int r0 = 0; r0 < S.n; r0 += group) {
+        const int r1 = (int)std::min((long)S.n, (long)r0 + group);
         const auto mm = std::minmax_element(level.begin() + r0, level.begin() + r1);
-        const int lo = *mm.first, nl = *mm.second - lo + 1;
-        at.assign((size_t)nl, 0);
-        for (int i = r0; i < r1; ++i) ++at[(size_t)(level[(size_t)i] - lo)];
-        int end = first.back();
-        for (int& a : at) {
-            const int cnt = a;
-            a = end;
-            if (cnt == 0) continue;
-            start.push_back(end);
-            end += cnt;
-            most = std::max(most, cnt);
+        const int lo = *mm.first;
+        at.assign((size_t)(*mm.second - lo + 2), 0);
+        for (int i = r0; i < r1; ++i) ++at[(size_t)(level[(size_t)i] - lo + 1)];
+        at[0] = r0;
+        for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
+        for (int i = r0; i < r1; ++i) sorted[(size_t)at[(size_t)(level[(size_t)i] - lo)]++] = i;
+        if (r1 == S.n) break;
+    }
+    if (group <= S.rpp) {
+        for (int u = 0; u < S.nparts; ++u) order.push_back(bwd ? S.nparts - 1 - u : u);
+    } else {
+        order = part_order(c->ls->mesh, sorted, level, S.rpp, S.nparts, bwd);
+    }
+    for (int p : order) {
+        const int t0 = p * S.rpp, t1 = std::min(S.n, t0 + S.rpp);
+        int prev = -1;
+        for (int t = t0, at = first.back(); t < t1; ++t, ++at) {
+            const int i = sorted[(size_t)t];
+            rows[(size_t)at] = i;
+            if (level[(size_t)i] == prev) continue;
+            prev = level[(size_t)i];
+            if (start.size() > (size_t)lev.back()) most = std::max(most, at - start.back());
+            start.push_back(at);
         }
-        for (int i = r0; i < r1; ++i) rows[(size_t)at[(size_t)(level[(size_t)i] - lo)]++] = i;
-        first.push_back(end);
+        first.push_back(first.back() + t1 - t0);
+        most = std::max(most, first.back() - start.back());
         lev.push_back((int)start.size());
     }
     start.push_back(S.n);
@@ -1145,8 +1207,11 @@ fvgb_status symbolic(IluCache* c) {
     FVGB_CUDA_TRY(cudaGetDevice(&dev));
     FVGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int rpp = std::min((n + 31) / 32 * 32, std::max(32, part_rows(lev_f)));
-    const int nparts = (n + rpp - 1) / rpp;
-    c->sweep_grid = (unsigned)std::max(1, std::min(nparts, n >= kDirectRows ? 2 * sms : sms));
+    const int nparts = (n + rpp - 1) / rpp, group = group_rows(lev_f, rpp);
+    // one group of several parts: they follow one another, and more than the next few would
+    // only wait (with a part of a chain on every SM, half a second)
+    const int blocks = group > rpp && group == n ? 4 : n >= kDirectRows ? 2 * sms : sms;
+    c->sweep_grid = (unsigned)std::max(1, std::min(nparts, blocks));
     const auto setup = [&](Sweep& S, int deps) {
         S.n = n;
         S.rpp = rpp;
@@ -1166,8 +1231,8 @@ fvgb_status symbolic(IluCache* c) {
     if (e == cudaSuccess && !c->pivots_only) e = il_upload(c, &c->op_f, op_f);
     if (e == cudaSuccess) e = il_upload(c, &c->op_g, op_g);
     if (e == cudaSuccess && !c->pivots_only) e = il_upload(c, &c->lev_rows, lev_rows);
-    if (e == cudaSuccess) e = il_sweep(c, c->fwd, lev_f, false, c->pivots_only ? 2 * c->fwd.K + 1 : c->fwd.K);
-    if (e == cudaSuccess) e = il_sweep(c, c->bwd, lev_b, true, c->bwd.K + 2);
+    if (e == cudaSuccess) e = il_sweep(c, c->fwd, lev_f, group, false, c->pivots_only ? 2 * c->fwd.K + 1 : c->fwd.K);
+    if (e == cudaSuccess) e = il_sweep(c, c->bwd, lev_b, group, true, c->bwd.K + 2);
     if (e == cudaSuccess) e = il_alloc(c, &c->a, (size_t)nnz);
     if (e == cudaSuccess) e = il_alloc(c, &c->lu, (size_t)nnz);
     double** vecs[] = {&c->r, &c->rr, &c->p, &c->q, &c->v, &c->y, &c->z, &c->s, &c->t, &c->w};

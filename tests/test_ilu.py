@@ -374,3 +374,26 @@ def test_ilu_memory_of_thin_levels(cuda, dims):
     free = torch.cuda.mem_get_info()[0]
     ls.solve(x, rel_tol=1e-9, max_iter=2, method=abi.SOLVER_CG, preconditioner=abi.PRECOND_ILU)
     assert free - torch.cuda.mem_get_info()[0] <= 512 * hm.n + (64 << 20)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", [
+    lambda: mesh.box(9001, 29, 1, 1.0, 1.0, 1e-4, two_d=True),     # halo warps; three groups of several parts
+    lambda: mesh.box(3001, 11, 9, jitter=0.1, seed=1),             # 3-D, 297,099 rows: read directly
+    lambda: mesh.box(2000, 1200, 1, 1.0, 1.0, 1e-3, two_d=True),   # a group is not yet the mesh, the last is short
+    lambda: mesh.box(20011, 1, 1),                                 # a chain: one group, a part after the other
+    lambda: mesh.box(8192, 4, 1, 1.0, 1.0, 1e-4, two_d=True),      # a line is a part
+    lambda: diag_mesh(9001, 12),                                   # fill updates
+    lambda: mesh.concat([mesh.box(700, 40, 1, two_d=False), mesh.box(9, 8, 7), mesh.box(5000, 3, 3)])[0],
+], ids=["long2d", "long3d", "plane", "chain", "line", "fill", "packed"])
+def test_ilu_sweeps_of_thin_levels(cuda, make):
+    """Meshes whose lines are long: parts cut by level from groups of rows."""
+    hm = make()
+    for kind, method, om in (("heat", abi.SOLVER_CG, 0), ("convection", abi.SOLVER_BICGSTAB, 1)):
+        T, o, ls, v, r = gpu_system(hm, kind)
+        x, xo = T.internal.clone(), T.host().copy()
+        st = ls.solve(x, rel_tol=1e-9, max_iter=12, method=method, preconditioner=abi.PRECOND_ILU)
+        so = o.solve(v, r, xo, rel_tol=1e-9, max_iter=12, method=om, preconditioner=2)
+        assert st.status == so.status and st.num_iter == so.num_iter   # most end at the cap
+        assert (st.init_res_norm, st.final_res_norm) == (so.init_res_norm, so.final_res_norm)
+        np.testing.assert_array_equal(x.cpu().numpy(), xo)
