@@ -437,6 +437,7 @@ extern "C" fvgb_status fvgb_mesh_create_boxes(const fvgb_box_spec* specs, int32_
     fvgb_mesh* m = new fvgb_mesh();
     m->pooled = devmem_pooled_now();
     m->h_patch_offs = poffs;
+    for (const BoxDev& b : boxes) m->h_boxes.push_back(HostBox{b.nx, b.ny, b.nz, b.cell0});
     m->nnz = (int32_t)(N + 2 * NIF);
     m->nslices = nslices;
     m->m_len = (int64_t)N * kMW;

@@ -173,6 +173,10 @@ inline void devmem_free(void* p, bool pooled) {
     else cudaFree(p);
 }
 
+struct HostBox {  // a hex box of a mesh built on the device: cells cell0 .. cell0 + nx ny nz - 1
+    int32_t nx, ny, nz, cell0;
+};
+
 struct fvgb_mesh {
     MeshView v{};
     int32_t nnz = 0;
@@ -183,6 +187,7 @@ struct fvgb_mesh {
     int32_t* csr_pos = nullptr;  // [nnz] slot of CSR entry j
     std::vector<int32_t> h_patch_offs;
     std::vector<int32_t> h_row_offs, h_col, h_diag_off, h_own_off, h_nei_off;
+    std::vector<HostBox> h_boxes;  // in place of the arrays above, for a mesh built on the device
     std::vector<void*> allocs;
     int64_t bytes = 0;
     bool pooled = false;  // device memory from the serving pool (devmem_*)

@@ -102,16 +102,24 @@ __device__ __forceinline__ V res_block_tree(const V* sm) {
     return s;
 }
 
+// Slots and halo entries of the largest block of a system, by which every block lays its
+// part out; zh: with room for the halo's z.
+struct ResSize {
+    int len, nh;
+    bool zh;
+};
+
 // The block's part of the system in shared memory (V: double, or float for the
 // FP32 inner solve).
 template <class V>
 struct ResMatrix {
-    V* sp;                 // [rows + nh] own directions, then the halo's
-    V* sval;               // [len]
-    V* zh;                 // [nh] the halo's z, fetched while a reduction is under way (null: no room)
-    int* hcol;             // [nh] column of every halo entry
-    unsigned short* scol;  // [len] index into sp
-    int nh, pos0;
+    V* sp;                 // [rows + size.nh] own directions, then the halo's
+    V* sval;               // [size.len]
+    V* zh;                 // [size.nh] the halo's z, fetched while a reduction is under way (null: no room)
+    int* hcol;             // [size.nh] column of every halo entry
+    unsigned short* scol;  // [size.len] index into sp
+    int rows, nh, pos0;
+    bool fits;             // else nothing of it may be used
 };
 
 // bytes of that part: value size v, with or without the staged z (with FP32 values
@@ -121,65 +129,77 @@ __host__ __device__ inline size_t res_bytes(int v, int rows, int len, int nh, bo
            2 * (size_t)len;
 }
 
-// Slots and halo entries of the block's rows [row0, row0 + rows) (all threads;
-// counter: shared).
-__device__ __forceinline__ void res_count(const MeshView& m, int row0, int rows, int* counter, int* len, int* nh) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
-    const int ns = (m.n + 31) >> 5, s0 = min(ns, row0 >> 5), s1 = min(ns, s0 + rows / 32);
-    *len = __ldg(&m.m_ptr[s1]) - __ldg(&m.m_ptr[s0]);
-    if (threadIdx.x == 0) *counter = 0;
-    __syncthreads();
-#pragma unroll 1
-    for (int s = s0 + wid; s < s1; s += nw) {
-        const int b0 = __ldg(&m.m_ptr[s]), w = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5, i = s * 32 + lane;
-        int c = 0;
-#pragma unroll 1
-        for (int k = 0; k < w; ++k)
-            c += (unsigned)(slot_col(m, b0 + k * 32 + lane, i) - row0) >= (unsigned)rows;
-        c = __reduce_add_sync(0xffffffffu, c);
-        if (lane == 0 && c) atomicAdd(counter, c);
+// Slots and halo entries of the largest block of `rows` rows, from the pattern on the
+// host: the rows' columns, or the boxes of a mesh built on the device.
+inline ResSize res_size(const fvgb_mesh* m, int rows) {
+    ResSize z{0, 0, false};
+    const int64_t n = m->v.n;
+    if (!m->h_boxes.empty()) {
+        for (int64_t r0 = 0; r0 < n; r0 += rows) {
+            const int64_t r1 = r0 + rows;
+            int64_t nh = 0;
+            for (const HostBox& b : m->h_boxes) {
+                const int64_t cells = (int64_t)b.nx * b.ny * b.nz, a0 = r0 - b.cell0, a1 = r1 - b.cell0;
+                if (a1 <= 0 || a0 >= cells) continue;
+                int64_t s = 1;  // the neighbour's distance
+                for (int64_t d : {b.nx, b.ny, b.nz}) {
+                    // cells below c that have an upper neighbour
+                    const auto below = [&](int64_t c) {
+                        c = std::min(std::max<int64_t>(c, 0), cells);
+                        return c / (s * d) * (s * (d - 1)) + std::min(c % (s * d), s * (d - 1));
+                    };
+                    // pairs (c, c + s) with only c, or only c + s, in the block
+                    nh += below(a1) - below(std::max(a0, a1 - s));
+                    nh += below(std::min(a0, a1 - s)) - below(a0 - s);
+                    s *= d;
+                }
+            }
+            z.len = std::max(z.len, (int)(std::min((int64_t)rows, n - r0) * m->m_width));
+            z.nh = (int)std::max<int64_t>(z.nh, nh);
+        }
+        return z;
     }
-    __syncthreads();
-    *nh = *counter;
-    __syncthreads();
-}
-
-// The largest block's need in bytes: need[0] with FP64 values, need[1] with FP32,
-// need[2] and need[3] the same with the halo's z staged.
-template <int R>
-__global__ void __launch_bounds__(kT) k_res_need(MeshView m, unsigned int* need) {
-    __shared__ int counter;
-    int len, nh;
-    res_count(m, (int)blockIdx.x * (kT * R), kT * R, &counter, &len, &nh);
-    if (threadIdx.x < 4) {
-        const size_t b = kT * R + nh > 65536 ? ~(size_t)0
-                                             : res_bytes(threadIdx.x & 1 ? 4 : 8, kT * R, len, nh, threadIdx.x >= 2);
-        atomicMax(&need[threadIdx.x], b > 0xffffffffull ? 0xffffffffu : (unsigned)b);
+    const std::vector<int32_t>&ro = m->h_row_offs, &col = m->h_col;
+    for (int64_t r0 = 0; r0 < n; r0 += rows) {
+        const int64_t r1 = std::min(n, r0 + rows);
+        int64_t len = 0, nh = 0;
+        for (int64_t s = r0; s < r1; s += 32) {
+            int w = 0;
+            for (int64_t i = s; i < std::min(r1, s + 32); ++i) {
+                const int b = ro[(size_t)i], e = ro[(size_t)i + 1];
+                w = std::max(w, e - b);
+                for (int k = b; k < e && col[(size_t)k] < r0; ++k) ++nh;  // ascending columns
+                for (int k = e; k > b && col[(size_t)k - 1] >= r0 + rows; --k) ++nh;
+            }
+            len += 32 * w;
+            // slots of the lanes past the last row name row 0 (where columns are stored)
+            if (r0 > 0 && s + 32 > n && !m->v.m_off) nh += (s + 32 - n) * w;
+        }
+        z.len = (int)std::max<int64_t>(z.len, len);
+        z.nh = (int)std::max<int64_t>(z.nh, nh);
     }
+    return z;
 }
 
 // Lays the block's part out and fills the columns; the values are the caller's.
 template <class V>
 __device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned char* dyn, int row0, int rows,
-                                                 int* counter) {
+                                                 const ResSize& size, int* counter) {
     const int T = threadIdx.x, lane = T & 31, wid = T >> 5, nw = (int)blockDim.x >> 5;
     const int ns = (m.n + 31) >> 5, s0 = min(ns, row0 >> 5), s1 = min(ns, s0 + rows / 32);
     ResMatrix<V> M;
-    int len;
-    res_count(m, row0, rows, counter, &len, &M.nh);
+    M.rows = rows;
     M.pos0 = __ldg(&m.m_ptr[s0]);
-    unsigned int have;
-    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(have));
-    const bool zh = res_bytes((int)sizeof(V), rows, len, M.nh, true) <= (size_t)have;
     M.sp = (V*)(dyn + (sizeof(V) == 4 ? 8 * rows : 0));
-    M.sval = M.sp + rows + M.nh;
-    M.zh = zh ? M.sval + len : nullptr;
-    M.hcol = (int*)(M.sval + len + (zh ? M.nh : 0));
-    M.scol = (unsigned short*)(M.hcol + M.nh);
+    M.sval = M.sp + rows + size.nh;
+    M.zh = size.zh ? M.sval + size.len : nullptr;
+    M.hcol = (int*)(M.sval + size.len + (size.zh ? size.nh : 0));
+    M.scol = (unsigned short*)(M.hcol + size.nh);
+    M.fits = __ldg(&m.m_ptr[s1]) - M.pos0 <= size.len;
     if (T == 0) *counter = 0;
     __syncthreads();
 #pragma unroll 1
-    for (int s = s0 + wid; s < s1; s += nw) {
+    for (int s = M.fits ? s0 + wid : s1; s < s1; s += nw) {
         const int b0 = __ldg(&m.m_ptr[s]), w = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5, i = s * 32 + lane;
 #pragma unroll 1
         for (int k = 0; k < w; ++k) {
@@ -196,13 +216,15 @@ __device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned cha
             int idx = d;
             if (halo) {
                 const int h = base + __popc(ball & ((1u << lane) - 1));
-                M.hcol[h] = c;
+                if (h < size.nh) M.hcol[h] = c;
                 idx = rows + h;
             }
             M.scol[pos - M.pos0] = (unsigned short)idx;
         }
     }
     __syncthreads();
+    M.nh = *counter;
+    M.fits = M.fits && M.nh <= size.nh;
     return M;
 }
 
@@ -247,7 +269,6 @@ template <class V, class W>
 __device__ __forceinline__ bool res_halo_dir(GridBar* gb, const ResMatrix<V>& M, const W* z, unsigned epoch,
                                              bool restart, V beta) {
     bool good = true;
-    const int nown = (int)(M.sval - M.sp) - M.nh;
 #pragma unroll 1
     for (int h = threadIdx.x; h < M.nh; h += kT) {
         V v;
@@ -262,7 +283,7 @@ __device__ __forceinline__ bool res_halo_dir(GridBar* gb, const ResMatrix<V>& M,
                     break;
                 }
         }
-        V* p = M.sp + nown + h;
+        V* p = M.sp + M.rows + h;
         *p = restart ? v : res_fma(beta, *p, v);
     }
     return good;
@@ -319,6 +340,14 @@ struct ResRows {
     }
 };
 
+// A block whose part is larger than the host counted ends the solve: every block leaves at
+// its next wait.
+__device__ __forceinline__ void res_refuse(const Layout& L, GridBar* gb) {
+    if (threadIdx.x != 0) return;
+    atomicExch(&gb->abort, 1);
+    if (blockIdx.x == 0) L.cases[0].status = FVGB_ERR_CUDA;
+}
+
 struct ResShared {
     double value, res0, res;
     int code, status, iter, bad, counter;
@@ -333,7 +362,7 @@ struct ResShared {
 template <int R>
 __global__ void __launch_bounds__(kT, 1)
     k_pcg_resident(Layout L, MeshView m, const double* __restrict__ val, const double* __restrict__ b, LLWord* z,
-                   ResMail* mail, GridBar* gb) {
+                   ResMail* mail, GridBar* gb, ResSize size) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ double sma[kT], smb[kT];
     __shared__ ResShared sh;
@@ -344,7 +373,8 @@ __global__ void __launch_bounds__(kT, 1)
     const SolverParams prm = L.bs->prm;
     double* x = prm.x;
     if (T == 0) sh.bad = 0;
-    const ResMatrix<double> M = res_load<double>(m, dyn, row0, ROWS, &sh.counter);
+    const ResMatrix<double> M = res_load<double>(m, dyn, row0, ROWS, size, &sh.counter);
+    if (!M.fits) return res_refuse(L, gb);
     // cold code in rolled loops: the kernel's iteration has to stay in the
     // instruction cache (unrolled over the rows it was 97 KB)
 #pragma unroll 1
@@ -532,7 +562,7 @@ struct IrResShared {
 template <int R>
 __global__ void __launch_bounds__(kT, 1)
     k_ir_resident(Layout L, MeshView m, const double* __restrict__ val, const double* __restrict__ b, float* a32,
-                  float* ev, float* dinv, unsigned long long* z, ResMail* mail, GridBar* gb) {
+                  float* ev, float* dinv, unsigned long long* z, ResMail* mail, GridBar* gb, ResSize size) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ double sma[kT], smb[kT];
     __shared__ float smf[kT];
@@ -548,7 +578,8 @@ __global__ void __launch_bounds__(kT, 1)
         sh.flags = 0u;
     }
     double* stage = (double*)dyn;  // [rows] FP64 residuals
-    const ResMatrix<float> M = res_load<float>(m, dyn, row0, ROWS, &sh.counter);
+    const ResMatrix<float> M = res_load<float>(m, dyn, row0, ROWS, size, &sh.counter);
+    if (!M.fits) return res_refuse(L, gb);
     // prepare: dinv, a32, ev (formed, or those of the unchanged matrix), sign flags, |D^-1/2 (b - A x0)|
     unsigned int f = 0u;
     double asr = 0.0;
@@ -1010,7 +1041,7 @@ __global__ void __launch_bounds__(2 * kClRows, 1)
     double* x = prm.x;
     for (int k = T; k < (int)(offsetof(ClShared, a) / sizeof(LLWord)); k += rows) ((LLWord*)&sh)[k] = LLWord{0ull, 0ull};
     if (T == 0) sh.code = sh.bad = 0;
-    const ResMatrix<double> M = res_load<double>(m, dyn, row0, rows, &sh.counter);
+    const ResMatrix<double> M = res_load<double>(m, dyn, row0, rows, ResSize{rows * 8, rows * 8, false}, &sh.counter);
     // this thread's row, its slots (at most 8) in registers
     double xr = 0.0, rv = 0.0, pr = 0.0, di = 0.0, v8[8];
     int c8[8], w = 0, b0 = 0;

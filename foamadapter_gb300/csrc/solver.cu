@@ -45,6 +45,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 
 namespace {
 
@@ -2544,7 +2545,7 @@ struct SolverCache {
     ResMail* mail = nullptr;               // resident solves: partials and answers in flight
     LLWord* zll = nullptr;                 // resident solves: published preconditioned residuals [n]
     unsigned long long* zll32 = nullptr;   // the same of the mixed solve
-    unsigned int res_need[4] = {~0u, ~0u, ~0u, ~0u};  // resident solves: shared memory of the largest block (k_res_need)
+    ResSize res_size{-1, 0, false};        // resident solves: the largest block (-1: not counted yet)
     float *pf2 = nullptr, *zf = nullptr;   // second direction buffer and z of the persistent mixed solve
     double* r0 = nullptr;                   // mixed: first FP64 residual, from the preparation kernel
     uint64_t converted_version = 0;        // fvgb_ls::version the FP32 matrix copy was formed from
@@ -3276,39 +3277,35 @@ ClusterPlan cluster_plan(const SolverCache* c) {
 }
 
 // Whether this system can be solved resident: at most one block per SM and every
-// block's matrix rows in its shared memory.  Asked once per system (one small
-// kernel and a read of its result); allocates what the solve keeps.
-bool resident_fits(SolverCache* c, bool mixed, cudaStream_t s) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+// block's matrix rows in its shared memory (*smem, with the halo's z where there is room).
+// Counted once per system on the host, from the pattern, so that nothing on the stream is
+// waited for; allocates what the solve keeps.
+bool resident_fits(SolverCache* c, bool mixed, cudaStream_t s, ResSize* size, size_t* smem) {
     if (c->nb > resident_blocks()) return false;
-    if (!c->mail || !(mixed ? (void*)c->zll32 : (void*)c->zll))
-        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
-    if (!c->mail) {
-        unsigned int* d = nullptr;
-        ResMail* mail = nullptr;
-        if (calloc_dev(c, &d, 4) != cudaSuccess || calloc_dev(c, &mail, 1) != cudaSuccess ||
-            settle_creation() != cudaSuccess)
+    const int rows = kT * rows_per_thread(c->n);
+    if (c->res_size.len < 0) c->res_size = res_size(c->ls->mesh, rows);
+    *size = c->res_size;
+    if (rows + size->nh > 65536) return false;  // 16-bit columns
+    for (bool zh : {true, false}) {
+        size->zh = zh;
+        *smem = res_bytes(mixed ? 4 : 8, rows, size->len, size->nh, zh);
+        if (*smem <= (size_t)kResSmem) break;
+    }
+    if (*smem > (size_t)kResSmem) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const auto have = [&](auto** p, size_t count) {  // cleared by every solve
+        if (*p) return true;
+        void* q = nullptr;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+            devmem_alloc(&q, sizeof(**p) * count, c->pooled) != cudaSuccess) {
+            cudaGetLastError();
             return false;
-        // on the solve's stream: a device-built mesh may still be in the making there
-        const MeshView m = c->ls->mesh->v;
-        if (rows_per_thread(c->n) == 8) k_res_need<8><<<c->nb, kT, 0, s>>>(m, d);
-        else k_res_need<4><<<c->nb, kT, 0, s>>>(m, d);
-        if (cudaMemcpyAsync(c->res_need, d, sizeof(c->res_need), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
-            return false;
-        c->mail = mail;
-    }
-    if (c->res_need[mixed ? 1 : 0] > (unsigned)kResSmem) return false;
-    cudaError_t e = cudaSuccess;
-    if (mixed && !c->zll32) {
-        e = calloc_dev(c, &c->zll32, (size_t)c->n);
-        if (e == cudaSuccess) e = settle_creation();
-    }
-    if (!mixed && !c->zll) {
-        e = calloc_dev(c, &c->zll, (size_t)c->n);
-        if (e == cudaSuccess) e = settle_creation();
-    }
-    return e == cudaSuccess;
+        }
+        c->allocs.push_back(q);
+        *p = (std::remove_reference_t<decltype(*p)>)q;
+        return true;
+    };
+    return have(&c->mail, 1) && (mixed ? have(&c->zll32, (size_t)c->n) : have(&c->zll, (size_t)c->n));
 }
 
 bool use_persistent(SolverCache* c, const fvgb_solver_cfg* cfg) {
@@ -3436,18 +3433,18 @@ fvgb_status launch(SolverCache* c, double* x, const fvgb_solver_cfg* cfg, fvgb_s
         if (e != cudaSuccess) {
             cudaGetLastError();
             FVGB_CUDA_TRY(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), s));
-            if (resident_fits(c, mixed, s)) {
+            ResSize size;
+            size_t smem = 0;
+            if (resident_fits(c, mixed, s, &size, &smem)) {
                 FVGB_CUDA_TRY(cudaMemsetAsync(c->mail, 0, sizeof(ResMail), s));
-                const unsigned int* need = c->res_need + (mixed ? 1 : 0);
-                const size_t smem = need[2] <= (unsigned)kResSmem ? need[2] : need[0];
                 if (mixed) {
                     FVGB_CUDA_TRY(cudaMemsetAsync(c->zll32, 0, sizeof(*c->zll32) * (size_t)c->n, s));
-                    void* args[] = {&L, &m, &val, &b, &c->ah, &c->ev, &c->dinvf, &c->zll32, &c->mail, &c->bar};
+                    void* args[] = {&L, &m, &val, &b, &c->ah, &c->ev, &c->dinvf, &c->zll32, &c->mail, &c->bar, &size};
                     const void* fn = r8 ? (const void*)k_ir_resident<8> : (const void*)k_ir_resident<4>;
                     e = cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s);
                 } else {
                     FVGB_CUDA_TRY(cudaMemsetAsync(c->zll, 0, sizeof(LLWord) * (size_t)c->n, s));
-                    void* args[] = {&L, &m, &val, &b, &c->zll, &c->mail, &c->bar};
+                    void* args[] = {&L, &m, &val, &b, &c->zll, &c->mail, &c->bar, &size};
                     const void* fn = r8 ? (const void*)k_pcg_resident<8> : (const void*)k_pcg_resident<4>;
                     e = cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s);
                 }

@@ -8,6 +8,7 @@ kernel).  Numberings: the box's own, and a random one in which almost every
 matrix slot reaches into another block (it fits the shared memory with 4 rows
 per thread and does not with 8).
 """
+import ctypes as C
 import time
 
 import numpy as np
@@ -144,3 +145,43 @@ def test_cluster_blocks_without_rows(cuda, n):
         assert (st.num_iter, st.final_res_norm, st.status) == (want.num_iter, want.final_res_norm, want.status)
         assert torch.equal(x, x0)
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED_IR])
+def test_first_resident_solve_waits_for_nothing(cuda, precision):
+    """fvgb_solve_async returns while the stream is still busy with what was queued before,
+    also for the first solve that takes the resident kernel, on a mesh of the host's and
+    on one built on the device."""
+    hm, T, ls = system((47, 41, 17))
+    specs = (abi.BoxSpec * 2)(abi.BoxSpec(33, 31, 20, 1.0, 1.0, 1.0, 0.0, 0, 0), abi.BoxSpec(7, 5, 3, 1.0, 1.0, 1.0, 0.0, 0, 0))
+    ranges, handle, lsd = np.zeros(4, np.int32), C.c_void_p(), C.c_void_p()
+    L = abi.lib()
+    abi.check(L.fvgb_mesh_create_boxes(specs, 2, C.byref(handle), abi.ptr(ranges), None))
+    abi.check(L.fvgb_ls_create(handle, 1, C.byref(lsd)))
+    sizes = (C.c_int64 * 5)()
+    abi.check(L.fvgb_mesh_sizes(handle, sizes))
+    n, nif, nbf = list(sizes)[:3]
+    old = torch.rand(n, dtype=torch.float64, device="cuda")
+    gamma, ref = torch.ones(nif + nbf, dtype=torch.float64, device="cuda"), torch.zeros(nbf, dtype=torch.float64, device="cuda")
+    types = np.full(6, abi.BC_FIXED_GRADIENT, np.int32)
+    bc = abi.BC(abi.ptr(types), abi.ptr(ref))
+    terms = (abi.Term * 2)(abi.Term(abi.TERM_DDT, 0, 1.0, abi.ptr(old), None), abi.Term(abi.TERM_LAPLACIAN, 0, -1.0, None, abi.ptr(gamma)))
+    abi.check(L.fvgb_assemble(lsd, terms, 2, 1e-4, C.byref(bc), abi.ptr(ref), None))
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for handle_ls, x0 in ((ls.handle, T.internal), (lsd, old)):
+        cfg = [abi.SolverCfg(1e-9, 0.0, 50, precision, 0.1, 1000, 50, mode, abi.SOLVE_NO_TUNE) for mode in (1, 2)]
+        x1, x2 = x0.clone(), x0.clone()
+        torch.cuda.synchronize()
+        abi.check(L.fvgb_solve_async(handle_ls, abi.ptr(x1), C.byref(cfg[0]), None, stream.cuda_stream))  # workspaces
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(1 << 30)   # half a second
+        start = time.perf_counter()
+        abi.check(L.fvgb_solve_async(handle_ls, abi.ptr(x2), C.byref(cfg[1]), None, stream.cuda_stream))
+        waited = time.perf_counter() - start
+        assert not stream.query() and waited < 0.2
+        torch.cuda.synchronize()
+        assert torch.equal(x1, x2)
+    L.fvgb_ls_destroy(lsd)
+    L.fvgb_mesh_destroy(handle)
