@@ -131,7 +131,7 @@ __host__ __device__ inline size_t res_bytes(int v, int rows, int len, int nh, bo
 
 // Slots and halo entries of the largest block of `rows` rows, from the pattern on the
 // host: the rows' columns, or the boxes of a mesh built on the device.
-inline ResSize res_size(const fvgb_mesh* m, int rows) {
+inline ResSize res_count(const fvgb_mesh* m, int rows) {
     ResSize z{0, 0, false};
     const int64_t n = m->v.n;
     if (!m->h_boxes.empty()) {
@@ -181,6 +181,12 @@ inline ResSize res_size(const fvgb_mesh* m, int rows) {
     return z;
 }
 
+inline ResSize res_size(const fvgb_mesh* m, int rows) {
+    ResSize z = res_count(m, rows);
+    z.nh = (z.nh + 3) & ~3;  // the values start on a 16-byte boundary
+    return z;
+}
+
 // Lays the block's part out and fills the columns; the values are the caller's.
 template <class V>
 __device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned char* dyn, int row0, int rows,
@@ -198,13 +204,25 @@ __device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned cha
     M.fits = __ldg(&m.m_ptr[s1]) - M.pos0 <= size.len;
     if (T == 0) *counter = 0;
     __syncthreads();
+    // a slice's columns are fetched while the one before is laid out
+    int next[8], w0 = 0, b0 = 0;
+    const auto fetch = [&](int s) {
+        if (s >= s1) return;
+        b0 = __ldg(&m.m_ptr[s]);
+        w0 = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5;
+        slot_cols(m, b0 + lane, w0, s * 32 + lane, next);
+    };
+    int s = M.fits ? s0 + wid : s1;
+    fetch(s);
 #pragma unroll 1
-    for (int s = M.fits ? s0 + wid : s1; s < s1; s += nw) {
-        const int b0 = __ldg(&m.m_ptr[s]), w = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5, i = s * 32 + lane;
-#pragma unroll 1
-        for (int k = 0; k < w; ++k) {
-            const int pos = b0 + k * 32 + lane;
-            const int c = slot_col(m, pos, i), d = c - row0;
+    for (; s < s1; s += nw) {
+        const int w = w0, at = b0 + lane;
+        int col[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) col[k] = next[k];
+        fetch(s + nw);
+        const auto place = [&](int k, int c) {
+            const int d = c - row0;
             const bool halo = (unsigned)d >= (unsigned)rows;
             const unsigned ball = __ballot_sync(0xffffffffu, halo);
             int base = 0;
@@ -219,8 +237,13 @@ __device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned cha
                 if (h < size.nh) M.hcol[h] = c;
                 idx = rows + h;
             }
-            M.scol[pos - M.pos0] = (unsigned short)idx;
-        }
+            M.scol[at + 32 * k - M.pos0] = (unsigned short)idx;
+        };
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k < w) place(k, col[k]);
+#pragma unroll 1
+        for (int k = 8; k < w; ++k) place(k, slot_col(m, at + 32 * k, s * 32 + lane));
     }
     __syncthreads();
     M.nh = *counter;
@@ -228,14 +251,16 @@ __device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned cha
     return M;
 }
 
-// The halo's z of `epoch` into M.zh, by threads T0 <= T < kT; four loads in flight each.
-template <class V, class W>
-__device__ __forceinline__ bool res_halo(GridBar* gb, const ResMatrix<V>& M, const W* z, unsigned epoch, int T0) {
+// put(h, z) of every halo entry h = first, first + step, ..., as its z of `epoch` arrives;
+// four loads in flight.
+template <class V, class W, class F>
+__device__ __forceinline__ bool res_halo_get(GridBar* gb, const ResMatrix<V>& M, const W* z, unsigned epoch, int first,
+                                             int step, F put) {
 #pragma unroll 1
-    for (int h0 = (int)threadIdx.x - T0; h0 < M.nh; h0 += 4 * (kT - T0)) {
+    for (int h0 = first; h0 < M.nh; h0 += 4 * step) {
         bool have[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) have[u] = h0 + u * (kT - T0) >= M.nh;
+        for (int u = 0; u < 4; ++u) have[u] = h0 + u * step >= M.nh;
 #pragma unroll 1
         for (unsigned spins = 0;; ++spins) {
             bool all = true;
@@ -244,12 +269,12 @@ __device__ __forceinline__ bool res_halo(GridBar* gb, const ResMatrix<V>& M, con
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 ok[u] = false;
-                if (!have[u]) ok[u] = ll_load(z + M.hcol[h0 + u * (kT - T0)], epoch, &v[u]);
+                if (!have[u]) ok[u] = ll_load(z + M.hcol[h0 + u * step], epoch, &v[u]);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 if (ok[u]) {
-                    M.zh[h0 + u * (kT - T0)] = v[u];
+                    put(h0 + u * step, v[u]);
                     have[u] = true;
                 }
                 all = all && have[u];
@@ -261,6 +286,12 @@ __device__ __forceinline__ bool res_halo(GridBar* gb, const ResMatrix<V>& M, con
     return true;
 }
 
+// The halo's z of `epoch` into M.zh, by threads T0 <= T < kT.
+template <class V, class W>
+__device__ __forceinline__ bool res_halo(GridBar* gb, const ResMatrix<V>& M, const W* z, unsigned epoch, int T0) {
+    return res_halo_get(gb, M, z, epoch, (int)threadIdx.x - T0, kT - T0, [&](int h, V v) { M.zh[h] = v; });
+}
+
 __device__ __forceinline__ double res_fma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float res_fma(float a, float b, float c) { return fmaf(a, b, c); }
 
@@ -268,25 +299,16 @@ __device__ __forceinline__ float res_fma(float a, float b, float c) { return fma
 template <class V, class W>
 __device__ __forceinline__ bool res_halo_dir(GridBar* gb, const ResMatrix<V>& M, const W* z, unsigned epoch,
                                              bool restart, V beta) {
-    bool good = true;
-#pragma unroll 1
-    for (int h = threadIdx.x; h < M.nh; h += kT) {
-        V v;
-        if (M.zh) {
-            v = M.zh[h];
-        } else {  // no room to stage it
-            unsigned spins = 0;
-#pragma unroll 1
-            while (!ll_load(z + M.hcol[h], epoch, &v))
-                if (ll_give_up(gb, spins++)) {
-                    good = false;
-                    break;
-                }
-        }
+    if (!M.zh) return res_halo_get(gb, M, z, epoch, (int)threadIdx.x, kT, [&](int h, V v) {  // no room to stage it
         V* p = M.sp + M.rows + h;
         *p = restart ? v : res_fma(beta, *p, v);
+    });
+#pragma unroll 1
+    for (int h = threadIdx.x; h < M.nh; h += kT) {
+        V* p = M.sp + M.rows + h;
+        *p = restart ? M.zh[h] : res_fma(beta, *p, M.zh[h]);
     }
-    return good;
+    return true;
 }
 
 // The matrix rows of one thread: slot bases (in the block's arrays) and widths of
@@ -375,31 +397,34 @@ __global__ void __launch_bounds__(kT, 1)
     if (T == 0) sh.bad = 0;
     const ResMatrix<double> M = res_load<double>(m, dyn, row0, ROWS, size, &sh.counter);
     if (!M.fits) return res_refuse(L, gb);
-    // cold code in rolled loops: the kernel's iteration has to stay in the
-    // instruction cache (unrolled over the rows it was 97 KB)
-#pragma unroll 1
-    for (int j = 0; j < R; ++j) {
-        const int l = loc0 + 32 * j, i = row0 + l;
-        M.sp[l] = i < n ? __ldg(&b[i]) - spmv_row_cg(m, val, x, i) : 0.0;
+    {  // the block's slots, 16 bytes at a time
+        const int len = min(size.len, __ldg(&m.m_ptr[min((n + 31) >> 5, (row0 + ROWS) >> 5)]) - M.pos0);
+        const unsigned at = (unsigned)__cvta_generic_to_shared(M.sval);
+        for (int k = 2 * T; k < len; k += 2 * kT)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + 8u * k), "l"(val + M.pos0 + k) : "memory");
     }
     double xr[R], rv[R], pr[R], di[R], zr[R];
     ResRows<R> W(m, row0 + wid * (32 * R), M.pos0);
-#pragma unroll 1
-    for (int k = 0; k < W.kmax; ++k) {
-#pragma unroll
-        for (int j = 0; j < R; ++j)
-            if (k < W.w[j]) M.sval[W.base[j] + 32 * k] = __ldg(&val[M.pos0 + W.base[j] + 32 * k]);
-    }
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-        rv[j] = M.sp[loc0 + 32 * j];
-        xr[j] = pr[j] = di[j] = 0.0;
         const int i = row0 + loc0 + 32 * j;
-        if (i < n) {
-            xr[j] = x[i];
-            di[j] = __ldg(&val[__ldg(&m.diag_pos[i])]);
-        }
+        xr[j] = i < n ? x[i] : 0.0;
+        rv[j] = i < n ? __ldg(&b[i]) : 0.0;
+        di[j] = i < n ? __ldg(&val[__ldg(&m.diag_pos[i])]) : 0.0;
+        M.sp[loc0 + 32 * j] = xr[j];
     }
+#pragma unroll 4
+    for (int h = T; h < M.nh; h += kT) M.sp[ROWS + h] = __ldcg(&x[M.hcol[h]]);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    W.product(M, zr, [](double, double xk) { return xk; }, xr);  // b - A x, the chains of the graph's row sums
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        rv[j] = row0 + loc0 + 32 * j < n ? rv[j] - zr[j] : 0.0;
+        pr[j] = 0.0;
+    }
+    // (cold code stays in rolled loops: unrolled over the rows the kernel was 97 KB, and its
+    // iteration has to stay in the instruction cache)
 #pragma unroll 1
     for (int j = 0; j < R; ++j) {  // 1 / diagonal, one division's code
         double d = 1.0;
@@ -584,10 +609,16 @@ __global__ void __launch_bounds__(kT, 1)
     unsigned int f = 0u;
     double asr = 0.0;
     ResRows<R> W(m, row0 + wid * (32 * R), M.pos0);
+    if (!prm.convert) {  // the block's slots, 16 bytes at a time
+        const int len = min(size.len, __ldg(&m.m_ptr[min((n + 31) >> 5, (row0 + ROWS) >> 5)]) - M.pos0);
+        const unsigned at = (unsigned)__cvta_generic_to_shared(M.sval);
+        for (int k = 4 * T; k < len; k += 4 * kT)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + 4u * k), "l"(a32 + M.pos0 + k) : "memory");
+    }
 #pragma unroll 1
     for (int j = 0; j < R; ++j) {
         const int i = row0 + loc0 + 32 * j, s = i >> 5;
-        if (s * 32 >= n) continue;
+        if (s * 32 >= n || !prm.convert) break;
         const int b0 = __ldg(&m.m_ptr[s]), wj = (__ldg(&m.m_ptr[s + 1]) - b0) >> 5;
         float* sv = M.sval + (b0 - M.pos0);
         if (i >= n) {
@@ -596,35 +627,42 @@ __global__ void __launch_bounds__(kT, 1)
             continue;
         }
         const double d = __ldg(&val[__ldg(&m.diag_pos[i])]);
-        f |= d > 0.0 ? 1u : (d < 0.0 ? 2u : 4u);
-        float dj;
-        if (prm.convert) {
-            dj = (float)(1.0 / d);
-            dinv[i] = dj;
-            const double sg = d < 0.0 ? -1.0 : 1.0;
-            double e = 0.0;
+        dinv[i] = (float)(1.0 / d);
+        const double sg = d < 0.0 ? -1.0 : 1.0;
+        double e = 0.0;
 #pragma unroll 1
-            for (int k = 0; k < wj; ++k) {
-                const int pos = b0 + lane + 32 * k;
-                const int code = __ldg(&m.m_code[pos]);
-                float a = 0.0f;
-                if (code != FVGB_PAD) {
-                    const double av = __ldg(&val[pos]);
-                    e = e + av;
-                    if (code != -1) a = (float)(sg * av);
-                }
-                a32[pos] = a;
-                sv[lane + 32 * k] = a;
+        for (int k0 = 0; k0 < wj; k0 += 8) {
+            const int at = b0 + lane + 32 * k0, left = wj - k0;
+            int code[8];
+            double av[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                code[k] = k < left ? __ldg(&m.m_code[at + 32 * k]) : FVGB_PAD;
+                av[k] = k < left ? __ldg(&val[at + 32 * k]) : 0.0;
             }
-            ev[i] = (float)(sg * e);
-        } else {
-            dj = dinv[i];
-#pragma unroll 1
-            for (int k = 0; k < wj; ++k) sv[lane + 32 * k] = a32[b0 + lane + 32 * k];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                if (k >= left) break;
+                float a = 0.0f;
+                if (code[k] != FVGB_PAD) {
+                    e = e + av[k];
+                    if (code[k] != -1) a = (float)(sg * av[k]);
+                }
+                a32[at + 32 * k] = a;
+                sv[lane + 32 * (k0 + k)] = a;
+            }
         }
+        ev[i] = (float)(sg * e);
+    }
+#pragma unroll 4
+    for (int j = 0; j < R; ++j) {
+        const int i = row0 + loc0 + 32 * j;
+        if (i >= n) continue;
+        const double d = __ldg(&val[__ldg(&m.diag_pos[i])]);
+        f |= d > 0.0 ? 1u : (d < 0.0 ? 2u : 4u);
         const double r = __ldg(&b[i]) - spmv_row_cg(m, val, x, i);
         stage[loc0 + 32 * j] = r;
-        asr = fma(r * (double)fabsf(dj), r, asr);
+        asr = fma(r * (double)fabsf(dinv[i]), r, asr);
     }
     double xr[R];
     float yv[R], rh[R], pr[R], zr[R], di[R], ei[R];
@@ -636,6 +674,7 @@ __global__ void __launch_bounds__(kT, 1)
         ei[j] = i < n ? ev[i] : 0.0f;
         yv[j] = rh[j] = pr[j] = zr[j] = 0.0f;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (f) atomicOr(&sh.flags, f);
     sma[T] = asr;
     unsigned epoch = 1;
@@ -702,7 +741,7 @@ __global__ void __launch_bounds__(kT, 1)
         const double ns = sh.nsig;
         ++epoch;
         if (!first) {
-#pragma unroll 1
+#pragma unroll 4
             for (int j = 0; j < R; ++j) {
                 const int i = row0 + loc0 + 32 * j;
                 if (i < n) stage[loc0 + 32 * j] = __ldg(&b[i]) - spmv_row_cg(m, val, x, i);

@@ -45,7 +45,6 @@
 #include <cmath>
 #include <cstdlib>
 #include <string>
-#include <type_traits>
 
 namespace {
 
@@ -2542,9 +2541,7 @@ struct SolverCache {
     cudaGraphExec_t gbg = nullptr;
     fvgb_solver_stats* h_stats = nullptr;  // pinned [ncases]
     GridBar* bar = nullptr;
-    ResMail* mail = nullptr;               // resident solves: partials and answers in flight
-    LLWord* zll = nullptr;                 // resident solves: published preconditioned residuals [n]
-    unsigned long long* zll32 = nullptr;   // the same of the mixed solve
+    char* exchange[2] = {nullptr, nullptr};  // resident solves, FP64 and mixed: what crosses blocks (ResExchange)
     ResSize res_size{-1, 0, false};        // resident solves: the largest block (-1: not counted yet)
     float *pf2 = nullptr, *zf = nullptr;   // second direction buffer and z of the persistent mixed solve
     double* r0 = nullptr;                   // mixed: first FP64 residual, from the preparation kernel
@@ -3276,6 +3273,18 @@ ClusterPlan cluster_plan(const SolverCache* c) {
     return p;
 }
 
+// What crosses the blocks of a resident solve, cleared by each in one piece: the abort
+// flag, the partials, the published preconditioned residuals.
+struct ResExchange {
+    GridBar* bar;
+    ResMail* mail;
+    void* z;
+};
+size_t exchange_bytes(int n, bool mixed) {
+    return 128 + sizeof(ResMail) + (mixed ? sizeof(unsigned long long) : sizeof(LLWord)) * (size_t)n;
+}
+ResExchange exchange_parts(char* p) { return {(GridBar*)p, (ResMail*)(p + 128), p + 128 + sizeof(ResMail)}; }
+
 // Whether this system can be solved resident: at most one block per SM and every
 // block's matrix rows in its shared memory (*smem, with the halo's z where there is room).
 // Counted once per system on the host, from the pattern, so that nothing on the stream is
@@ -3292,20 +3301,17 @@ bool resident_fits(SolverCache* c, bool mixed, cudaStream_t s, ResSize* size, si
         if (*smem <= (size_t)kResSmem) break;
     }
     if (*smem > (size_t)kResSmem) return false;
+    char*& p = c->exchange[mixed];
+    if (p) return true;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const auto have = [&](auto** p, size_t count) {  // cleared by every solve
-        if (*p) return true;
-        void* q = nullptr;
-        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
-            devmem_alloc(&q, sizeof(**p) * count, c->pooled) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        c->allocs.push_back(q);
-        *p = (std::remove_reference_t<decltype(*p)>)q;
-        return true;
-    };
-    return have(&c->mail, 1) && (mixed ? have(&c->zll32, (size_t)c->n) : have(&c->zll, (size_t)c->n));
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+        devmem_alloc((void**)&p, exchange_bytes(c->n, mixed), c->pooled) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+        return false;
+    }
+    c->allocs.push_back(p);
+    return true;
 }
 
 bool use_persistent(SolverCache* c, const fvgb_solver_cfg* cfg) {
@@ -3432,26 +3438,22 @@ fvgb_status launch(SolverCache* c, double* x, const fvgb_solver_cfg* cfg, fvgb_s
         const bool r8 = rows_per_thread(c->n) == 8;
         if (e != cudaSuccess) {
             cudaGetLastError();
-            FVGB_CUDA_TRY(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), s));
             ResSize size;
             size_t smem = 0;
             if (resident_fits(c, mixed, s, &size, &smem)) {
-                FVGB_CUDA_TRY(cudaMemsetAsync(c->mail, 0, sizeof(ResMail), s));
-                if (mixed) {
-                    FVGB_CUDA_TRY(cudaMemsetAsync(c->zll32, 0, sizeof(*c->zll32) * (size_t)c->n, s));
-                    void* args[] = {&L, &m, &val, &b, &c->ah, &c->ev, &c->dinvf, &c->zll32, &c->mail, &c->bar, &size};
-                    const void* fn = r8 ? (const void*)k_ir_resident<8> : (const void*)k_ir_resident<4>;
-                    e = cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s);
-                } else {
-                    FVGB_CUDA_TRY(cudaMemsetAsync(c->zll, 0, sizeof(LLWord) * (size_t)c->n, s));
-                    void* args[] = {&L, &m, &val, &b, &c->zll, &c->mail, &c->bar, &size};
-                    const void* fn = r8 ? (const void*)k_pcg_resident<8> : (const void*)k_pcg_resident<4>;
-                    e = cudaLaunchCooperativeKernel(fn, dim3(nvb), dim3(kT), args, smem, s);
-                }
+                FVGB_CUDA_TRY(cudaMemsetAsync(c->exchange[mixed], 0, exchange_bytes(c->n, mixed), s));
+                ResExchange ex = exchange_parts(c->exchange[mixed]);
+                void* args_mixed[] = {&L, &m, &val, &b, &c->ah, &c->ev, &c->dinvf, &ex.z, &ex.mail, &ex.bar, &size};
+                void* args_fp64[] = {&L, &m, &val, &b, &ex.z, &ex.mail, &ex.bar, &size};
+                const void* fn_mixed = r8 ? (const void*)k_ir_resident<8> : (const void*)k_ir_resident<4>;
+                const void* fn_fp64 = r8 ? (const void*)k_pcg_resident<8> : (const void*)k_pcg_resident<4>;
+                e = cudaLaunchCooperativeKernel(mixed ? fn_mixed : fn_fp64, dim3(nvb), dim3(kT),
+                                                mixed ? args_mixed : args_fp64, smem, s);
             }
         }
         if (e != cudaSuccess) {
             cudaGetLastError();
+            FVGB_CUDA_TRY(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), s));
             // k_ir_persistent(L, m, val, b, a32, ev, dinv, r0, rh, y, pbuf0, pbuf1, z, q, pa, pb, pc, gb, nvb)
             void* args_mixed[] = {&L,     &m,    &val,   &b,     &c->ah, &c->ev, &c->dinvf, &c->r0, &c->rh, &c->y,
                                   &c->pf, &c->pf2, &c->zf, &c->qf, &c->pa, &c->pb, &c->pc,   &c->bar, &nvb};
