@@ -270,6 +270,10 @@ __global__ void k_gather_csr(int nnz, const int32_t* __restrict__ csr_pos,
 
 }  // namespace
 
+int64_t fvgb_system_bytes(int64_t rows, int64_t slots, int64_t nbf) {
+    return devmem_piece(8 * slots) + devmem_piece(8 * rows) + 2 * devmem_piece(8 * nbf);
+}
+
 extern "C" fvgb_status fvgb_ls_create(const fvgb_mesh* mesh, int32_t ncomp, fvgb_ls** out) {
     fvgb_clear_error();
     FVGB_CHECK_ARG(mesh && out, "fvgb_ls_create: null argument");

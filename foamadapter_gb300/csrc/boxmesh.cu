@@ -377,6 +377,20 @@ void free_mesh_partial(fvgb_mesh* m) {
 
 }  // namespace
 
+// The allocations below for one box.
+int64_t fvgb_box_mesh_bytes(int32_t nx, int32_t ny, int32_t nz) {
+    const int64_t N = ((int64_t)nx * ny * nz + 31) / 32 * 32, slices = N / 32;
+    const int64_t NIF = (int64_t)(nx - 1) * ny * nz + (int64_t)nx * (ny - 1) * nz + (int64_t)nx * ny * (nz - 1);
+    const int64_t NBF = 2 * ((int64_t)ny * nz + (int64_t)nx * nz + (int64_t)nx * ny);
+    const int64_t span = nz > 1 ? (int64_t)nx * ny : (ny > 1 ? (int64_t)nx : 1);
+    const auto P = devmem_piece;
+    return 2 * P(8 * N) + 2 * P(4 * NIF) + P(24 * NIF) + 4 * P(8 * NIF) +           // V, invV, own, nei, Sf, magSf, w, delta, geo
+           2 * P(4 * NBF) + P(24 * NBF) + 3 * P(8 * NBF) +                          // bcells, bpatch, bSf, bmagSf, bdelta, bgeo
+           2 * P(4 * (slices + 1)) + 2 * P(4 * N * kGW) + 2 * P(4 * N * kMW) +      // g_ptr, m_ptr, g_code, g_other, m_col, m_code
+           (span <= 32767 ? P(2 * N * kMW) : 0) + P(4 * N) + 2 * P(4 * NIF) +       // m_off, diag_pos, own_pos, nei_pos
+           P(4 * slices) + P(sizeof(BoxDev)) + P(24 * N);                           // slice_box, boxes, centres
+}
+
 extern "C" fvgb_status fvgb_mesh_create_boxes(const fvgb_box_spec* specs, int32_t nboxes, fvgb_mesh** out,
                                               int32_t* row_ranges, fvgb_stream stream) {
     fvgb_clear_error();

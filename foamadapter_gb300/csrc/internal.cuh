@@ -18,6 +18,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstdint>
 #include <string>
@@ -150,12 +151,19 @@ inline DevMemCtx& devmem_ctx() {
     return c;
 }
 inline bool devmem_pooled_now() { return devmem_ctx().pool != nullptr; }
+// What an allocation of `bytes` takes of an arena.
+inline int64_t devmem_piece(int64_t bytes) { return (std::max<int64_t>(bytes, 1) + 255) / 256 * 256; }
+// Device bytes of one box's mesh, of a scalar system on it and of its CG solver, each
+// counted beside the code that allocates them: the serving loop's requests.
+int64_t fvgb_box_mesh_bytes(int32_t nx, int32_t ny, int32_t nz);
+int64_t fvgb_system_bytes(int64_t rows, int64_t slots, int64_t nbf);
+int64_t fvgb_solver_bytes(int64_t rows, int64_t slots, bool mixed, bool one_kernel);
 inline cudaError_t devmem_alloc(void** p, size_t bytes, bool pooled) {
     if (!pooled) return cudaMalloc(p, bytes);
     const DevMemCtx& c = devmem_ctx();
     if (!c.pool) return cudaErrorInvalidValue;  // a pooled object grows only on the thread that owns the pool
     if (DevMemArena* a = c.arena) {
-        const size_t need = (bytes + 255) & ~(size_t)255;
+        const size_t need = (size_t)devmem_piece((int64_t)bytes);
         if (need <= a->size - a->used) {
             *p = a->base + a->used;
             a->used += need;

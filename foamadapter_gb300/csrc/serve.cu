@@ -2,7 +2,7 @@
 //
 // Requests (a box mesh, a uniform velocity, a diffusivity and a number of
 // implicit steps) arrive at any time through fvgb_server_submit.  A host thread
-// admits waiting requests in arrival order whenever their estimated device
+// admits waiting requests in arrival order whenever their device
 // footprint fits the HBM budget, builds their mesh on the device
 // (fvgb_mesh_create_boxes) and keeps fields, matrix and solver state resident
 // until the request finishes.  Each active request advances on its own CUDA
@@ -100,17 +100,18 @@ struct fvgb_server {
 
 namespace {
 
-// Device bytes a request holds while resident (mesh, system, solver, fields).
-int64_t estimate_bytes(const fvgb_serve_request& r) {
-    const int64_t n = ((int64_t)r.nx * r.ny * r.nz + 31) / 32 * 32;
-    const int64_t nif = (int64_t)(r.nx - 1) * r.ny * r.nz + (int64_t)r.nx * (r.ny - 1) * r.nz +
-                        (int64_t)r.nx * r.ny * (r.nz - 1);
+// Device bytes a request holds while resident (mesh, system, solver, fields): the sum of
+// what is allocated for it.
+int64_t request_bytes(const fvgb_serve_request& r) {
+    const int64_t n = ((int64_t)r.nx * r.ny * r.nz + 31) / 32 * 32, slots = 7 * n;
+    const int64_t nf = (int64_t)(r.nx - 1) * r.ny * r.nz + (int64_t)r.nx * (r.ny - 1) * r.nz +
+                       (int64_t)r.nx * r.ny * (r.nz - 1) + nbf_of(r);
     const int64_t nbf = nbf_of(r);
-    const int64_t mesh = 16 * n + 72 * nif + 64 * nbf + 4 * 6 * 2 * n + 4 * 7 * 2 * n + 2 * 7 * n + 4 * n;
-    const int64_t system = 8 * 7 * n + 8 * n + 16 * nbf;
-    const int64_t solver = r.precision == FVGB_PREC_MIXED_IR ? (8 + 28 + 16) * n : 40 * n;
-    const int64_t fields = 16 * n + 8 * nbf + 16 * (nif + nbf) + 24 * (n + nbf) + 8 * nbf;
-    return mesh + system + solver + fields + (1 << 20);
+    const auto P = devmem_piece;
+    const int64_t fields = (r.flags & FVGB_SERVE_REASSEMBLE ? 2 : 1) * P(8 * n) + 2 * P(8 * nbf) + 2 * P(8 * nf) +
+                           P(24 * n) + P(24 * nbf) + P(sizeof(fvgb_solver_stats) * kChunk);
+    return fvgb_box_mesh_bytes(r.nx, r.ny, r.nz) + fvgb_system_bytes(n, slots, nbf) +
+           fvgb_solver_bytes(n, slots, r.precision == FVGB_PREC_MIXED_IR, r.kernel_mode == 2) + fields;
 }
 
 // Device memory of a request comes from the server's pool (set on the loop's
@@ -495,7 +496,7 @@ extern "C" fvgb_status fvgb_server_submit(fvgb_server* sv, const fvgb_serve_requ
         return fvgb_fail(FVGB_ERR_INVALID_ARG, "fvgb_server_submit: bad request");
     Slot* s = new Slot();
     s->req = *req;
-    s->bytes = estimate_bytes(*req);
+    s->bytes = request_bytes(*req);
     if (s->bytes > sv->cfg.budget_bytes) {
         delete s;
         return fvgb_fail(FVGB_ERR_BUDGET, "fvgb_server_submit: request alone exceeds the HBM budget");

@@ -3314,6 +3314,21 @@ bool resident_fits(SolverCache* c, bool mixed, cudaStream_t s, ResSize* size, si
     return true;
 }
 
+}  // namespace
+
+// cache_create, then alloc_fp64 or alloc_mixed, then what one-kernel solves take
+int64_t fvgb_solver_bytes(int64_t rows, int64_t slots, bool mixed, bool one_kernel) {
+    const auto P = devmem_piece;
+    const int64_t rb = kT * rows_per_thread((int)rows), nb = std::max<int64_t>(1, (rows + rb - 1) / rb);
+    int64_t b = 2 * P(4 * nb) + 2 * P(4) + P(8) + P(sizeof(CaseState)) + P(sizeof(BatchState)) +
+                P(sizeof(fvgb_solver_stats)) + 3 * P(8 * nb);
+    b += mixed ? P(4 * slots) + 8 * P(4 * rows) + P(8 * rows) : 5 * P(8 * rows);
+    if (one_kernel) b += P(sizeof(GridBar)) + (nb <= kResMaxBlocks ? P((int64_t)exchange_bytes((int)rows, mixed)) : 0);
+    return b;
+}
+
+namespace {
+
 bool use_persistent(SolverCache* c, const fvgb_solver_cfg* cfg) {
     if (!c->whole || cfg->kernel_mode == 1 || cfg->kernel_mode == 3) return false;
     if (cfg->kernel_mode != 2 && c->n > (1 << 20)) return false;

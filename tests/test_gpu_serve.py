@@ -265,3 +265,31 @@ def test_one_kernel_solves_of_served_requests(cuda, precision):
     for together in (False, True, False):
         for a, b in zip(burst(2, together), want):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED_IR])
+def test_requests_hold_what_they_are_counted_for(cuda, precision, mode):
+    """The device memory a burst takes from the driver is its requests' device_bytes and the
+    pool's granules (32 MB, and 2 MB a request), at sizes of one-kernel (66 cells an edge)
+    and of graph solves."""
+    def burst(sv, dims, count):
+        bytes_ = 0
+        for _ in range(count):
+            req = abi.ServeRequest(nx=dims[0], ny=dims[1], nz=dims[2], steps=1, U=(C.c_double * 3)(0.4, -0.3, 0.2), D=2e-3,
+                                   dt=0.0, precision=precision, kernel_mode=mode, flags=0, T_out=None, T_init=None)
+            rid = C.c_int64()
+            abi.check(abi.lib().fvgb_server_submit(sv, C.byref(req), C.byref(rid)))
+        for r in drain(sv, count).values():
+            bytes_ += r.device_bytes
+        return bytes_
+
+    for dims, count in (((66, 66, 66), 24), ((110, 111, 109), 6)):
+        sv = make_server(budget=64 << 30)
+        burst(sv, (20, 20, 20), 2)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        counted = burst(sv, dims, count)
+        taken = free - torch.cuda.mem_get_info()[0]
+        abi.lib().fvgb_server_destroy(sv)
+        assert taken <= counted + (32 << 20) + count * (2 << 20)
