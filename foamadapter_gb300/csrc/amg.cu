@@ -27,7 +27,8 @@
 //    (more than 90% of the rows left), or kMaxLevels is reached.
 // Setup, numeric (device, whenever the matrix values changed): the coarse
 // values by those fixed sums, the Jacobi diagonals, and the inverse of the
-// coarsest matrix by Gauss-Jordan elimination in one block (no pivoting: the
+// coarsest matrix by Gauss-Jordan elimination in one cluster, its rows dealt over the
+// blocks, or in one block where they do not fit their shared memory (no pivoting: the
 // matrix is symmetric positive definite).
 // V-cycle z = M r: per level one damped-Jacobi sweep from zero (weight 0.9),
 // the residual, restriction by aggregate sums, the coarser level, then the
@@ -36,9 +37,11 @@
 // symmetric sweep, so M is symmetric positive definite and CG applies.
 // Kernels: the first sweep of level 0 is formed by the CG kernels that produce
 // r (k_init, k_update), a coarse level's by the restriction that produces its
-// right-hand side; the residual is one gather per slot (k_resid); level 0
-// adds the coarse correction (k_prolong) before its second sweep (k_post),
-// coarser levels form it inside the sweep (k_post_fused); the small levels and the
+// right-hand side; residual and restriction are one kernel over whole aggregates
+// (k_resid_restrict), or two where an aggregate exceeds a block (k_resid, k_restrict); level
+// 0 adds the coarse correction before its second sweep (k_prolong, k_post), inside it up to
+// kFusedPostRows rows in the CG, where that sweep also forms beta (k_post_rz); coarser
+// levels form it inside the sweep (k_post_fused); the small levels and the
 // coarsest one's dense solve run in one cluster (k_tail).  Coarse levels are sliced
 // ELL like the system matrix.
 //

@@ -201,8 +201,9 @@ __global__ void __launch_bounds__(kT)
 }
 
 // ------------------------------------------------------ triangular sweeps
-// One launch per triangle.  The rows are cut into parts of consecutive rows, one part
-// to a block at a time, taken in the sweep's direction by a ticket: a row depends only
+// One launch per triangle.  The rows are cut into parts, of consecutive rows or, where those
+// would have levels of a few rows, by level from groups of consecutive rows (group_rows),
+// one part to a block at a time, taken by a ticket in an order in which a row depends only
 // on rows of its own part and of parts that running blocks took before, so every wait
 // ends.
 //
@@ -216,8 +217,8 @@ __global__ void __launch_bounds__(kT)
 // others into shared memory, in the order in which its rows need them; on large systems
 // (kDirectRows) the row warps read them themselves.
 //
-// BiCGStab on 77 x 64 x 58 cells: 6.1 -> 3.1 ms, on 20^3 1.42 -> 0.70, on 128^3 16.1 ->
-// 12.0; before, every value went through L2 (1.6 us a level), and every level of the
+// BiCGStab on 77 x 64 x 58 cells: 6.1 -> 3.0 ms, on 20^3 1.41 -> 0.70, on 128^3 16.0 ->
+// 11.4; before, every value went through L2 (1.6 us a level), and every level of the
 // factorization was a kernel of dependent loads (2.2 of the 6.1 ms, now 0.4).  A level
 // takes 0.4 us inside a part: the barrier 250 clocks, three dependent multiply-adds 200
 // of GB300's FP64; a step to another part 1.3 us.  Rows that poll shared memory without
@@ -233,15 +234,18 @@ constexpr int kSweepThreads = 32 * (kRowWarps + kHaloWarps);
 constexpr int kMaxTeams = 8;   // named barriers 1 .. kMaxTeams
 constexpr int kDeps = 4;       // values a row waits for together; the others one by one
 // Rows of a part: few parts make few trips through L2, and a level of more than 128 rows
-// leaves two teams, which fetch too late.  BiCGStab on 77 x 64 x 58 cells: 3.20 ms with
-// parts of 8,192 rows, 4.06 with 4,096 (levels of up to 128 and 64 rows), 4.05 with
-// 9,600 (up to 140); on 20^3, 0.72 ms with 1,024 and 1.00 in one part (300).
+// leaves two teams, which fetch too late.  BiCGStab on 77 x 64 x 58 cells: 2.98 ms with
+// parts of 8,192 rows, 3.45 with 4,096 (levels of up to 128 and 64 rows); on 20^3, 0.70 ms
+// with 1,024 and 1.00 in one part (levels of up to 300).  A part of consecutive rows with
+// fewer than kThinRows rows a level is too long a chain for its rows: ILU-CG iterations of
+// 9000 x 90 x 9 cells 40.7 ms, with groups from 8 rows a level on 13.8, from 16 on 8.4;
+// 2048^2 6.62, 4.61 and 4.07; 512^2 (15.5 rows) 0.86 either way.
 constexpr int kPart = 8192, kMinPart = 1024, kLevelRows = 128, kThinRows = 16;
 // From this size on the row warps read the rows of other parts themselves, before their
 // turn: their reads are further ahead of need than the halo warps' when levels are wide.
-// ILU-CG on 128^3 cells 156 ms with halo warps and 121 without (145 with every step
-// through L2), 96^3 86.7 and 72.0, 64^3 22.3 and 18.8; BiCGStab on 48^3 2.16 and 2.24 ms,
-// on 80 x 80 x 9 1.84 and 2.11.  The grid is then twice the SMs, of which one block each
+// ILU-CG on 128^3 cells 162 ms with halo warps and 122 without (144 with every step
+// through L2), 96^3 83.8 and 66.9, 64^3 21.5 and 18.3; BiCGStab on 40^3 1.42 and 1.48 ms,
+// on 80 x 80 x 9 1.77 and 1.94.  The grid is then twice the SMs, of which one block each
 // is resident (123.5 -> 120.0 ms on 128^3, which has 256 parts); without the idle halo
 // warps two were, and it took 140.
 constexpr int kDirectRows = 1 << 18;

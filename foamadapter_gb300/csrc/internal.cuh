@@ -133,7 +133,7 @@ __device__ __forceinline__ double facc0(bool plus, double x) {
 // counts for it, and its objects' ~50 allocations are cut from it.  Each allocation
 // from the pool cost 15 us with its wait, and 60 once some hundreds of releases had
 // cut the pool up: bursts of 16 requests with 27 ms of device work went from 54 ms
-// to 150 ms, and stay at 46 to 62 ms with one piece each.  What a piece has no room
+// to 203 ms on one server, and stay at 46 to 49 ms (the first: 53) with one piece each.  What a piece has no room
 // for comes from the pool as before.
 struct DevMemArena {
     char* base = nullptr;

@@ -252,7 +252,8 @@ __device__ __forceinline__ ResMatrix<V> res_load(const MeshView& m, unsigned cha
 }
 
 // put(h, z) of every halo entry h = first, first + step, ..., as its z of `epoch` arrives;
-// four loads in flight.
+// four loads in flight (60^3 cells, whose halo has no room to be staged: 18.8 -> 16.0 us an
+// iteration against one at a time).
 template <class V, class W, class F>
 __device__ __forceinline__ bool res_halo_get(GridBar* gb, const ResMatrix<V>& M, const W* z, unsigned epoch, int first,
                                              int step, F put) {
@@ -377,10 +378,15 @@ struct ResShared {
 
 // FP64 Jacobi-CG of one case on its blocks (one per SM); mail and z are zero at
 // launch.  512 x 512 cavity pressure (262,144 rows, 128 blocks, 3,050 iterations):
-// 13.1 us per iteration against 20.1 for k_pcg_persistent (three grid barriers,
+// 12.5 us per iteration against 20.1 for k_pcg_persistent (three grid barriers,
 // every vector through L2); of its 25,600 clocks 12,500 are DFMA issue, 7,500 the
 // two hops and 4,500 the block and final trees and the scalars' divisions (64
 // clocks per dependent FP64 instruction).  1,600 rows: 7.9 us against 15.2.
+//
+// Before the first iteration (50 us at 60^3 cells, of which 33 are the grid-barrier
+// kernel's too): columns fetched a slice ahead, the matrix copied asynchronously beside
+// them, the first residual from the block's own part.  A load at a time these took 74 us,
+// more than a warm-started solve of seven iterations gains.
 template <int R>
 __global__ void __launch_bounds__(kT, 1)
     k_pcg_resident(Layout L, MeshView m, const double* __restrict__ val, const double* __restrict__ b, LLWord* z,
@@ -583,7 +589,7 @@ struct IrResShared {
 // for the other blocks behind a fence and reads the FP64 matrix through L2.  An
 // inner iteration is two hops (2 x 1.4 us with 128 blocks on both dies), two final
 // trees and divisions in FP64 (2 x 0.7 us) and 1.5 us of FP32 work on shared
-// memory.  512 x 512 cavity step: 128 -> 71 ms against k_ir_persistent.
+// memory.  512 x 512 cavity step: 128 -> 66 ms against k_ir_persistent.
 template <int R>
 __global__ void __launch_bounds__(kT, 1)
     k_ir_resident(Layout L, MeshView m, const double* __restrict__ val, const double* __restrict__ b, float* a32,

@@ -212,7 +212,9 @@ fvgb_status fvgb_advect_euler_step(const fvgb_mesh* mesh, const double* flux,
  * cells have at most 8 faces take one launch for all steps, the cells in registers.
  * Otherwise, meshes of at most 65536 cells take one launch of a one-pass step kernel
  * per step (no face buffer), larger ones the two-pass step of fvgb_advect_euler_step;
- * all give the bits of nsteps single calls. */
+ * all give the bits of nsteps single calls.  Waits between the blocks of the one launch
+ * are bounded; the call returns before they run, so one that ran out leaves NaN in
+ * (T, T_b) instead of a status. */
 fvgb_status fvgb_advect_euler_steps(const fvgb_mesh* mesh, const double* flux, double* T, double* T_b,
                                     double dt, const fvgb_bc* bc, int32_t nsteps, double* work,
                                     double* work_b, fvgb_stream stream);
@@ -346,9 +348,11 @@ typedef struct fvgb_solver_cfg {
                                   the FP64 CG) or FVGB_PRECOND_ILU (Ginkgo Ilu with a
                                   ParIlu factorization, OpenFOAM's DILU,
                                   fvSolution.cpp:56-63: the exact ILU(0) factors,
-                                  formed level by level in every solve, and
-                                  triangular solves of one launch each, rows in
-                                  level order; CG or BiCGStab, FP64,
+                                  formed in every solve (by one sweep over the rows on
+                                  hex meshes, level by level elsewhere), and
+                                  triangular solves of one launch each; 360 to
+                                  430 bytes a row from its first solve on; CG or
+                                  BiCGStab, FP64,
                                   single systems, fvgb_solve / fvgb_solve_async)       */
 } fvgb_solver_cfg;
 enum { FVGB_SOLVE_NO_TUNE = 1, FVGB_SOLVE_RHS_BASELINE = 2 };
